@@ -1,0 +1,107 @@
+// coop.cuh -- barrier and sums of a cooperative grid.
+//
+// Iterations whose kernels are shorter than a launch run as one cooperative
+// kernel whose CTAs (all resident, cudaLaunchCooperativeKernel) meet at a
+// counter in global memory.  Every wait is bounded: a CTA that gives up sets
+// `fail`, on which every other CTA leaves too, and the host reads it.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace topo {
+
+struct GridBar {
+    unsigned *count;  // arrivals of this launch; zero between launches
+    unsigned *left;   // CTAs that have finished; the last one zeroes both
+    unsigned *fail;   // set by a CTA whose wait ran out
+};
+constexpr unsigned GRID_BAR_POLLS = 1u << 23;  // about a second
+
+__device__ __forceinline__ unsigned ld_poll(const unsigned *p) {
+    unsigned v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// every thread of every CTA; `arrivals` counts this CTA's barriers.  False:
+// some CTA gave up, and the caller returns at once.
+__device__ __forceinline__ bool grid_sync(const GridBar &b, unsigned &arrivals) {
+    arrivals++;
+    bool ok = true;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(b.count) : "memory");
+        const unsigned target = arrivals * gridDim.x;
+        unsigned polls = 0;
+        while (ld_poll(b.count) < target) {
+            if (++polls > GRID_BAR_POLLS || ((polls & 1023u) == 0 && ld_poll(b.fail))) {
+                atomicExch(b.fail, 1u);
+                ok = false;
+                break;
+            }
+        }
+        __threadfence();
+    }
+    return __syncthreads_and(ok) != 0;
+}
+
+// the end of the kernel, every thread of every CTA: counters back to zero for
+// the next launch on the same stream
+__device__ __forceinline__ void grid_leave(const GridBar &b) {
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(b.left, 1u) == gridDim.x - 1) {
+            *b.count = 0u;
+            *b.left = 0u;
+            __threadfence();
+        }
+    }
+}
+
+// CTA sums of NV values per thread into out[v * stride], v = 0..NV-1, in the
+// type of the values.  Every thread of the CTA calls it; `sm` is free again
+// after the caller's next barrier.  (A scalar FP64 instruction in every thread
+// of a CTA of 256 takes the SM 128 clocks: sums that may be FP32 stay FP32,
+// and scalar algebra belongs in one thread.)
+template <int NT, int NV, class V>
+__device__ __forceinline__ void cta_sums(const V v[NV], V *sm /* NV * NT / 32 */, V *out, size_t stride) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+    for (int i = 0; i < NV; i++) {
+        V x = v[i];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        if (lane == 0) sm[i * (NT / 32) + wid] = x;
+    }
+    __syncthreads();
+    if (threadIdx.x < NV) {
+        V s = V(0);
+#pragma unroll
+        for (int w = 0; w < NT / 32; w++) s += sm[threadIdx.x * (NT / 32) + w];
+        out[threadIdx.x * stride] = s;
+    }
+}
+// after the barrier: the grid's sums of the nv <= NT / 32 values whose CTA sums
+// stand at part[v * gridDim + b], the same in every thread of every CTA (a
+// fixed order: 32 strided sums, one tree), one warp a value
+template <int NT, class V>
+__device__ __forceinline__ void grid_totals(const V *part, int nv, V *sm /* nv */) {
+    const int lane = threadIdx.x & 31, v = threadIdx.x >> 5;
+    if (v < nv) {
+        const V *p = part + (size_t)v * gridDim.x;
+        V s = V(0);
+        // the loads of eight strides in flight at once: one L2 round trip for 256 CTAs
+        for (unsigned b = lane; b < gridDim.x; b += 256) {
+            V t[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) t[u] = b + 32 * u < gridDim.x ? __ldcg(p + b + 32 * u) : V(0);
+#pragma unroll
+            for (int u = 0; u < 8; u++) s += t[u];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) sm[v] = s;
+    }
+    __syncthreads();
+}
+
+}  // namespace topo

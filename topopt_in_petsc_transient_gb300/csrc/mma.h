@@ -4,9 +4,6 @@
 
 namespace topo {
 struct TopoMMA;
-struct GenSubGx {
-    double v[8];
-};
 int mma_create(TopoMMA **out, int n, int m, const double *a, const double *c, const double *d);
 void mma_destroy(TopoMMA *mm);
 int mma_set_asymptotes(TopoMMA *mm, double init, double dec, double inc);
