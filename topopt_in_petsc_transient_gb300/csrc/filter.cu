@@ -2,18 +2,21 @@
 // (Filter.cc) on one GPU.
 //
 // The Helmholtz filter (-R^2 lap + 1) u = T x on the nodal grid has the same
-// 8x8 element matrix KF for every element (R^2 * Laplacian + mass of the box,
-// PDEFilter.cc:485-578), so its assembled operator is applied node-centrically
-// from the element matrix in constant memory; T (0.125 per element node,
-// :580-588) and T^t are gathers.  The solve is Jacobi-preconditioned CG in FP64
-// with device-resident scalars.
+// 8x8 element matrix for every element (R^2 * Laplacian + mass of the box,
+// PDEFilter.cc:485-578); T (0.125 per element node, :580-588) and T^t are
+// gathers.  The assembled operator is a sum of tensor products of the 1-D
+// stiffness and mass, applied without the matrix; the solve is one cooperative
+// kernel (k_filt_solve).
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
 #include <vector>
 
+#include "coop.cuh"
 #include "filter.h"
 #include "kernels.cuh"
+#include "planes.cuh"
 
 namespace topo {
 
@@ -26,199 +29,409 @@ namespace topo {
         }                                                                    \
     } while (0)
 
-struct FiltScalars {
-    double bb, rr, rz, rz_old, pq, alpha, beta;
-    double tol2;
-    int it, maxit, done, status;
+constexpr int FILT_RHS = 2;        // right-hand sides solved at once
+constexpr int FT_N = 256;          // threads: node columns of a CTA, tx x ty of them
+constexpr int FT_PLANE = 2 * FT_N;  // most values of a staged plane: the columns and one node around
+
+// Operator of the unit-scaled filter K / V (V the element volume).  The 1-D
+// assembled mass and stiffness are h [1 4 1] / 6 and [-1 2 -1] / h inside, and
+// at an end half of the same stencil on the mirrored line (v_-1 = v_1).  So
+//   K / V = d A,  A the constant 27-point stencil
+//   [m m m + sum_a (R / h_a)^2 k_a m_b m_c],  m = [1 4 1] / 6, k = [-1 2 -1],
+// on the mirrored field, d = 1/2 per axis on which the node is at an end.  c[S]:
+// A's weight of a neighbour displaced along the axes in S (bit a: axis a).
+template <class T>
+struct FiltOp {
+    T c[8];
 };
+
+struct FiltStatus {
+    int status, it;
+};
+
+struct FiltArgs {
+    GridDesc g;
+    FiltOp<double> Kd;
+    FiltOp<float> Kf;
+    int nr;                             // right-hand sides
+    const double *xin[FILT_RHS];        // element fields
+    double *xout[FILT_RHS], *xphys;     // results; xphys: clamp and project (one right-hand side)
+    int clamp, projection;
+    double beta, eta;
+    double *u[FILT_RHS][2], *b[FILT_RHS], *r[FILT_RHS];
+    float *r32[FILT_RHS][2], *s32[FILT_RHS][2], *w32[FILT_RHS][2], *p32[FILT_RHS], *d32[FILT_RHS];
+    double tol;
+    int maxit;
+    double *part;                       // [2 slots][FILT_RHS][gridDim] FP64 sums, then [2][FILT_RHS][3][gridDim] FP32 ones
+    GridBar bar;
+    FiltStatus *out;                    // mapped host memory
+    int tx, ty, ntx, nty, cz, ncz;      // patches of tx x ty node columns, runs of cz planes
+};
+
+// A applied to a field in runs of planes along z, a column of nodes per thread.
+// F supplies the field and takes the products:
+//   Raw load(n); T val(Raw, s)        value of a staged node, s = 1 / d
+//   Own own(n); put(n, d, Own, v, y)  node n: boundary factor, operands, own value, product
+// In-plane neighbours come from one staged plane; of the two planes beside it
+// only Q, the in-plane sum with the weights of a neighbour along z, is needed,
+// kept in registers: 15 operations a node instead of 27 multiply-adds.  Bound by
+// the latency of its loads (24 warps an SM), so the staged ones are issued two
+// planes ahead of their use and the node's own one plane ahead.
+template <class T, class F>
+__device__ __forceinline__ void filt_apply(const FiltArgs &A, const FiltOp<T> &K, T *plane /* [2][FT_PLANE] */, F &f) {
+    const GridDesc &g = A.g;
+    const int tid = threadIdx.x, ty = tid / A.tx, tx = tid - ty * A.tx;
+    const int row = A.tx + 2, nst = row * (A.ty + 2);
+    const int items = A.ntx * A.nty * A.ncz;
+    const unsigned nxy = (unsigned)g.nx * g.ny;  // node indices stay below 2^32 (lex3)
+    // node index along an axis of n nodes, mirrored one beyond its ends
+    auto mirror = [](int i, int n) { return min(max(i < 0 ? -i : (i >= n ? 2 * n - 2 - i : i), 0), n - 1); };
+    for (int it = blockIdx.x; it < items; it += gridDim.x) {
+        const int bx = it % A.ntx, by = (it / A.ntx) % A.nty, bz = it / (A.ntx * A.nty);
+        const int i0 = bx * A.tx, j0 = by * A.ty, k0 = bz * A.cz, k1 = min(k0 + A.cz, g.nz);
+        const int i = i0 + tx, j = j0 + ty;
+        const bool in = ty < A.ty && i < g.nx && j < g.ny;
+        const float dxy = ((i == 0 || i == g.nx - 1) ? 0.5f : 1.0f) * ((j == 0 || j == g.ny - 1) ? 0.5f : 1.0f);
+        const unsigned nij = i + (unsigned)g.nx * j;
+        int sn[2];    // staged nodes of this thread within a plane (-1: none) and their 1 / d
+        float ss[2];
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const int v = tid + q * FT_N, r = v / row;
+            const int si = mirror(i0 - 1 + v - r * row, g.nx), sj = mirror(j0 - 1 + r, g.ny);
+            sn[q] = v < nst ? si + g.nx * sj : -1;
+            ss[q] = ((si == 0 || si == g.nx - 1) ? 2.0f : 1.0f) * ((sj == 0 || sj == g.ny - 1) ? 2.0f : 1.0f);
+        }
+        typename F::Raw raw[2][2];  // staged values of planes k and k + 1
+        typename F::Own own[2];     // of the planes k (being staged) and k - 1 (being completed)
+        auto fetch = [&](int k, typename F::Raw v[2]) {
+            const unsigned o = nxy * (unsigned)mirror(k, g.nz);
+#pragma unroll
+            for (int q = 0; q < 2; q++)
+                if (sn[q] >= 0) v[q] = f.load(o + sn[q]);
+        };
+        T vc = T(0), P = T(0), Q = T(0), Ql = T(0);
+        auto step = [&](int k, typename F::Raw v[2], typename F::Own &ok, const typename F::Own &okm1) {
+            T *pl = plane + (k & 1) * FT_PLANE;
+            const float sz = (k <= 0 || k >= g.nz - 1) && k != -1 && k != g.nz ? 2.0f : 1.0f;
+            // beyond an end the mirrored plane 1 or nz - 2 is staged, itself an end plane when nz = 2
+            const float s2 = (k == -1 || k == g.nz) && g.nz == 2 ? 2.0f : sz;
+#pragma unroll
+            for (int q = 0; q < 2; q++)
+                if (sn[q] >= 0) pl[tid + q * FT_N] = f.val(v[q], s2 * ss[q]);
+            if (k + 1 < k1) fetch(k + 2, v);
+            if (in && k >= k0 && k < k1) ok = f.own(nij + nxy * (unsigned)k);
+            __syncthreads();  // one barrier a plane: the other buffer was last read before the previous one
+            if (in) {
+                const T *s = pl + (ty + 1) * row + tx + 1, *su = s + row, *sd = s - row;
+                const T c = s[0], ax = s[-1] + s[1], ay = su[0] + sd[0], axy = (su[-1] + su[1]) + (sd[-1] + sd[1]);
+                const T Qn = K.c[4] * c + K.c[5] * ax + K.c[6] * ay + K.c[7] * axy;
+                if (k > k0)  // plane k - 1 is complete
+                    f.put(nij + nxy * (unsigned)(k - 1), (k == 1 || k == g.nz) ? 0.5f * dxy : dxy, okm1, vc,
+                          P + (Ql + Qn));
+                P = K.c[0] * c + K.c[1] * ax + K.c[2] * ay + K.c[3] * axy;
+                Ql = Q;
+                Q = Qn;
+                vc = c;
+            }
+        };
+        fetch(k0 - 1, raw[0]);
+        fetch(k0, raw[1]);
+        for (int k = k0 - 1; k <= k1; k += 2) {  // by two: the buffers swap by name, no copies that wait for loads
+            step(k, raw[0], own[0], own[1]);
+            if (k + 1 <= k1) step(k + 1, raw[1], own[1], own[0]);
+        }
+        __syncthreads();  // the planes are restaged by the next run
+    }
+}
+
+// start of a correction: r32 = r / rms(r), z = Dinv r32, w = K z, d = 0
+struct FiltStart {
+    const double *r64;
+    ScaleF64 sg;
+    float dinv, *r, *w, *d, sum[3];
+    using Raw = double;
+    using Own = double;
+    __device__ Raw load(unsigned n) const { return r64[n]; }
+    __device__ float val(Raw v, float s) const { return s * dinv * scaled_f32(v, sg); }
+    __device__ Own own(unsigned n) const { return r64[n]; }
+    __device__ void put(unsigned n, float bd, Own v, float z, float y) {
+        const float rv = scaled_f32(v, sg), wv = bd * y;
+        r[n] = rv;
+        w[n] = wv;
+        d[n] = 0.0f;
+        sum[0] += rv * z;
+        sum[1] += wv * z;
+    }
+};
+// one CG iteration (k_filt_solve)
+struct FiltIter {
+    float al, be, dinv;
+    const float *ro, *so, *wo;
+    float *rn, *sn, *wn, *p, *d, sum[3];
+    struct Raw {
+        float r, w, s;
+    };
+    struct Own {
+        float r, w, s, p, d;
+    };
+    // beta = 0 (the first step): s and p may hold anything
+    __device__ float snew(float w, float s) const { return be == 0.0f ? w : w + be * s; }
+    __device__ Raw load(unsigned n) const { return {ro[n], wo[n], so[n]}; }
+    __device__ float val(const Raw &v, float s) const { return s * dinv * (v.r - al * snew(v.w, v.s)); }
+    __device__ Own own(unsigned n) const { return {ro[n], wo[n], so[n], p[n], d[n]}; }
+    __device__ void put(unsigned n, float bd, const Own &o, float z, float y) {
+        const float sv = snew(o.w, o.s), rv = o.r - al * sv, zold = dinv * o.r * (bd == 1.0f ? 1.0f : 1.0f / bd);
+        const float pv = be == 0.0f ? zold : zold + be * o.p, wv = bd * y;
+        sn[n] = sv;
+        rn[n] = rv;
+        p[n] = pv;
+        d[n] = o.d + al * pv;
+        wn[n] = wv;
+        sum[0] += rv * z;
+        sum[1] += wv * z;
+        sum[2] += rv * rv;
+    }
+};
+// end of a correction: u += d / sigma, r = b - K u
+struct FiltResid {
+    const double *uo, *b;
+    const float *d;
+    double is, *un, *r, sum;
+    struct Raw {
+        double u;
+        float d;
+    };
+    using Own = double;
+    __device__ Raw load(unsigned n) const { return {uo[n], d[n]}; }
+    __device__ double val(const Raw &v, float) const { return fma(is, f32_to_f64(v.d), v.u); }
+    __device__ Own own(unsigned n) const { return b[n]; }
+    __device__ void put(unsigned n, float bd, Own bv, double v, double y) {
+        un[n] = v;
+        const double e = bv - (bd == 1.0f ? y : (double)bd * y);
+        r[n] = e;
+        sum += e * e;
+    }
+};
+
+// One or two filter solves: u = K^-1 (T x), then T^t u (and the projection).
+// FP64 iterative refinement: the residual b - K u and u in FP64, each
+// correction by Jacobi CG in FP32 on the residual scaled to unit mean square
+// (GB300 runs FP64 at 1/64 of its FP32 rate).  Convergence is decided on the
+// FP64 residual.  In one cooperative kernel, and CG in the form with one set
+// of sums per iteration (Chronopoulos and Gear): with z = Dinv r, w = A z,
+//   s = w + beta s, r = r - alpha s, p = z + beta p, d = d + alpha p,
+//   gamma = r.z, delta = w.z -> beta, alpha
+// where the new r of the neighbours is formed while staging, so an iteration
+// is one pass and one grid barrier.  Filter and chain rule of three fields take
+// 2.9 ms at 192x96x96 and 0.39 ms at 48x24x24, against 13.7 and 1.49 ms of FP64 CG
+// with three launches an iteration and 64 FP64 multiply-adds a node; the result
+// is 3.1e-11 instead of 4.5e-11 from the exact one at rtol 1e-10.
+__global__ void __launch_bounds__(FT_N, 3) k_filt_solve(const FiltArgs A) {
+    constexpr int NV = 3;
+    // scalars of a right-hand side, formed by one thread of every CTA alike
+    struct Rhs {
+        double bb, rr, rms;
+        float gam, alpha, beta, goal;
+        int done, idle;
+    };
+    __shared__ __align__(16) double pl64[2 * FT_PLANE];
+    __shared__ double sred64[FT_N / 32], stot64[FILT_RHS];
+    __shared__ float sred[FILT_RHS][NV * FT_N / 32], stot[FILT_RHS * NV];
+    __shared__ Rhs R[FILT_RHS];
+    __shared__ int s_status;
+    float *pl32 = reinterpret_cast<float *>(pl64);
+    const GridDesc g = A.g;
+    const long long nn = g.nn(), nel = g.nel();
+    const long long t0 = blockIdx.x * (long long)FT_N + threadIdx.x, ts = (long long)gridDim.x * FT_N;
+    unsigned arrivals = 0;
+    int slot = 0;
+    // CTA sums of right-hand side r; after finish() their grid sums stand in stot[NV r + v]
+    float *pf = reinterpret_cast<float *>(A.part + 2 * (size_t)FILT_RHS * gridDim.x);
+    auto sums = [&](int r, const float *v) {
+        cta_sums<FT_N, NV>(v, sred[r], pf + (size_t)(slot * FILT_RHS + r) * NV * gridDim.x + blockIdx.x, gridDim.x);
+    };
+    auto finish = [&]() {
+        if (!grid_sync(A.bar, arrivals)) return false;
+        grid_totals<FT_N>(pf + (size_t)slot * FILT_RHS * NV * gridDim.x, A.nr * NV, stot);
+        slot ^= 1;
+        return true;
+    };
+    // the same for one FP64 value each
+    auto sum64 = [&](int r, double v) {
+        cta_sums<FT_N, 1>(&v, sred64, A.part + (size_t)(slot * FILT_RHS + r) * gridDim.x + blockIdx.x, gridDim.x);
+        __syncthreads();
+    };
+    auto finish64 = [&]() {
+        if (!grid_sync(A.bar, arrivals)) return false;
+        grid_totals<FT_N>(A.part + (size_t)slot * FILT_RHS * gridDim.x, A.nr, stot64);
+        slot ^= 1;
+        return true;
+    };
+    const float dinv = 1.0f / A.Kf.c[0];
+
+    // right-hand sides b = T x, u = 0, r = b
+    for (int r = 0; r < A.nr; r++) {
+        double bb = 0.0;
+        for (long long n = t0; n < nn; n += ts) {
+            int i, j, k;
+            lex3(n, g.nx, g.ny, i, j, k);
+            double acc = 0.0;
+            for (int c = 0; c < 8; c++) {
+                const int ei = i - (c & 1), ej = j - ((c >> 1) & 1), ek = k - (c >> 2);
+                if (ei < 0 || ej < 0 || ek < 0 || ei >= g.ex || ej >= g.ey || ek >= g.ez) continue;
+                acc += A.xin[r][ei + (long long)g.ex * (ej + (long long)g.ey * ek)];
+            }
+            acc *= 0.125;
+            A.b[r][n] = acc;
+            A.r[r][n] = acc;
+            A.u[r][0][n] = 0.0;
+            bb += acc * acc;
+        }
+        sum64(r, bb);
+    }
+    if (!finish64()) return;
+    if (threadIdx.x == 0) {
+        s_status = TOPO_OK;
+        for (int r = 0; r < FILT_RHS; r++) {
+            R[r].done = 1;
+            if (r >= A.nr) continue;
+            R[r].bb = R[r].rr = stot64[r];
+            R[r].done = stot64[r] == 0.0;
+            if (!isfinite(stot64[r])) s_status = TOPO_ERR_NAN;
+        }
+    }
+    __syncthreads();
+    int its = 0, ub = 0;  // ub: which u is current
+    while (s_status == TOPO_OK && !(R[0].done && R[1].done)) {
+        if (threadIdx.x < FILT_RHS && !R[threadIdx.x].done) R[threadIdx.x].rms = sqrt(R[threadIdx.x].rr / (double)nn);
+        __syncthreads();
+        // r32 = r / rms(r), z, w = K z, correction 0
+        for (int r = 0; r < A.nr; r++) {
+            if (R[r].done) continue;
+            FiltStart f{A.r[r], scale_split(1.0 / R[r].rms), dinv, A.r32[r][0], A.w32[r][0], A.d32[r], {}};
+            filt_apply<float>(A, A.Kf, pl32, f);
+            sums(r, f.sum);
+        }
+        if (!finish()) return;
+        if (threadIdx.x < FILT_RHS) {
+            const int r = threadIdx.x;
+            Rhs &q = R[r];
+            q.idle = q.done;
+            if (!q.done) {
+                q.gam = stot[NV * r];
+                q.beta = 0.0f;
+                q.alpha = q.gam / stot[NV * r + 1];
+                if (!(q.alpha > 0.0f) || !isfinite(q.alpha)) q.idle = 1;
+                // reduction asked of this correction: half of what is left to the
+                // tolerance, at most 1e-6 (what the FP32 recurrence holds)
+                const double left = fmax(1e-6, 0.5 * A.tol * sqrt(q.bb / q.rr));
+                q.goal = (float)(left * left * (double)nn);
+            }
+        }
+        __syncthreads();
+        for (int it = 0; it < 64 && !(R[0].idle && R[1].idle) && its < A.maxit; it++, its++) {
+            const int o = it & 1, w = o ^ 1;  // buffers read and written
+            for (int r = 0; r < A.nr; r++) {
+                if (R[r].idle) continue;
+                FiltIter f{R[r].alpha, R[r].beta, dinv, A.r32[r][o], A.s32[r][o], A.w32[r][o],
+                           A.r32[r][w], A.s32[r][w], A.w32[r][w], A.p32[r], A.d32[r], {}};
+                filt_apply<float>(A, A.Kf, pl32, f);
+                sums(r, f.sum);
+            }
+            if (!finish()) return;
+            if (threadIdx.x < A.nr && !R[threadIdx.x].idle) {
+                Rhs &q = R[threadIdx.x];
+                const float *t = stot + NV * threadIdx.x, be = t[0] / q.gam;
+                q.beta = be;
+                q.alpha = t[0] / (t[1] - be * t[0] / q.alpha);
+                q.gam = t[0];
+                // at the goal, or rounding has used the correction up
+                if (!(t[2] > q.goal) || !(q.alpha > 0.0f) || !isfinite(q.alpha)) q.idle = 1;
+            }
+            __syncthreads();
+        }
+        // u += d / sigma (into the other buffer), r = b - K u, r.r
+        for (int r = 0; r < A.nr; r++) {
+            if (R[r].done) {  // converged earlier: carried along
+                for (long long n = t0; n < nn; n += ts) A.u[r][ub ^ 1][n] = A.u[r][ub][n];
+                continue;
+            }
+            FiltResid f{A.u[r][ub], A.b[r], A.d32[r], R[r].rms, A.u[r][ub ^ 1], A.r[r], 0.0};
+            filt_apply<double>(A, A.Kd, pl64, f);
+            sum64(r, f.sum);
+        }
+        if (!finish64()) return;
+        ub ^= 1;
+        if (threadIdx.x == 0)
+            for (int r = 0; r < A.nr; r++) {
+                Rhs &q = R[r];
+                if (q.done) continue;
+                const double s = stot64[r], was = q.rr;
+                q.rr = s;
+                if (!isfinite(s)) s_status = TOPO_ERR_NAN;
+                // a residual that a correction no longer halves, below 1e-12, is the
+                // rounding of b - K u: tolerances under it are met as far as FP64 goes
+                else if (s <= A.tol * A.tol * q.bb || (s > 0.25 * was && s <= 1e-24 * q.bb)) q.done = 1;
+                else if (its >= A.maxit) s_status = TOPO_ERR_NOT_CONVERGED;
+            }
+        __syncthreads();
+    }
+    const int status = s_status;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        A.out->status = status;
+        A.out->it = its;
+        __threadfence_system();
+    }
+    if (status == TOPO_OK) {
+        // xout = T^t u; optional clamp to [0,1] and smoothed Heaviside projection
+        // (Filter.cc:83-113, Filter.h:80-83)
+        const double th = tanh(A.beta * A.eta), rden = 1.0 / (th + tanh(A.beta * (1.0 - A.eta)));
+        for (int r = 0; r < A.nr; r++) {
+            const double *u = A.u[r][ub];
+            for (long long e = t0; e < nel; e += ts) {
+                int i, j, k;
+                lex3(e, g.ex, g.ey, i, j, k);
+                double acc = 0.0;
+                for (int L = 0; L < 8; L++)
+                    acc += u[(i + (L & 1)) + (long long)g.nx * ((j + ((L >> 1) & 1)) + (long long)g.ny * (k + (L >> 2)))];
+                acc *= 0.125;
+                if (A.clamp) {
+                    if (acc < 0.0) acc = 0.0;
+                    if (acc > 1.0) acc = 1.0;
+                }
+                A.xout[r][e] = acc;
+                if (A.xphys) A.xphys[e] = A.projection ? (th + proj_tanh(A.beta * (acc - A.eta))) * rden : acc;
+            }
+        }
+    }
+    grid_leave(A.bar);
+}
 
 struct TopoPDEFilt {
     GridDesc g;
-    double h[3], R, vol, rtol;
+    double rtol;
     int maxit;
     double KF[64];
-    double *rhs, *u, *r, *p, *q, *dinv;
-    double *e1, *e2;  // element scratch
-    FiltScalars *S;
+    FiltArgs args;   // operator, buffers and layout of the launches
+    unsigned grid;   // CTAs of k_filt_solve: as many as are resident at once, at most one per run
+    double *mnd;
     double *part;
-    unsigned int *counter;
-    unsigned long long *mbits;
+    unsigned int *counter;  // [0] reductions, [1..3] the grid barrier
+    FiltStatus *status;     // mapped host memory
     std::vector<void *> ptrs;
     cudaStream_t stream;
 };
 
-struct KFMat {
-    double v[64];
-};
-
-// y = K_F x (assembled, natural boundary), red: x.y
-__global__ void k_filt_apply(GridDesc g, KFMat KF, const double *__restrict__ x, double *y, Partials<1> part,
-                             const FiltScalars *S, int check_done) {
-    if (check_done && S->done) return;
-    long long nn = g.nn();
-    double v[1] = {0.0};
-    for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < nn; n += (long long)gridDim.x * blockDim.x) {
-        int i, j, k;
-        lex3(n, g.nx, g.ny, i, j, k);
-        double acc = 0.0;
-        for (int c = 0; c < 8; c++) {
-            int ei = i - (c & 1), ej = j - ((c >> 1) & 1), ek = k - (c >> 2);
-            if (ei < 0 || ej < 0 || ek < 0 || ei >= g.ex || ej >= g.ey || ek >= g.ez) continue;
-            // node n is local corner c of element e; KF uses the reference local order
-            for (int L = 0; L < 8; L++) {
-                long long m = (ei + (L & 1)) + (long long)g.nx * ((ej + ((L >> 1) & 1)) + (long long)g.ny * (ek + (L >> 2)));
-                acc += KF.v[c * 8 + L] * x[m];
-            }
-        }
-        y[n] = acc;
-        v[0] += x[n] * acc;
-    }
-    double tot[1];
-    if (grid_reduce<EW, 1>(v, part, tot)) {
-        FiltScalars *Sm = const_cast<FiltScalars *>(S);
-        Sm->pq = tot[0];
-        Sm->alpha = (tot[0] > 0.0) ? Sm->rz / tot[0] : 0.0;
-        if (!(tot[0] > 0.0)) {
-            Sm->done = 1;
-            Sm->status = isfinite(tot[0]) ? TOPO_ERR_BREAKDOWN : TOPO_ERR_NAN;
-        }
-    }
-}
-
-// rhs = vol * T x  (T = 0.125 per element corner)
-__global__ void k_T(GridDesc g, double vol, const double *__restrict__ x, double *rhs) {
-    long long nn = g.nn();
-    for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < nn; n += (long long)gridDim.x * blockDim.x) {
-        int i, j, k;
-        lex3(n, g.nx, g.ny, i, j, k);
-        double acc = 0.0;
-        for (int c = 0; c < 8; c++) {
-            int ei = i - (c & 1), ej = j - ((c >> 1) & 1), ek = k - (c >> 2);
-            if (ei < 0 || ej < 0 || ek < 0 || ei >= g.ex || ej >= g.ey || ek >= g.ez) continue;
-            acc += 0.125 * x[ei + (long long)g.ex * (ej + (long long)g.ey * ek)];
-        }
-        rhs[n] = acc * vol;
-    }
-}
-
-// xout = T^t u; optional clamp to [0,1] and smoothed Heaviside projection
-// (Filter.cc:83-113, Filter.h:80-83)
-__global__ void k_Tt(GridDesc g, const double *__restrict__ u, double *xout, double *xphys, int clamp, int projection,
-                     double beta, double eta) {
-    long long nel = g.nel();
-    double den = tanh(beta * eta) + tanh(beta * (1.0 - eta));
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < nel; e += (long long)gridDim.x * blockDim.x) {
-        int i, j, k;
-        lex3(e, g.ex, g.ey, i, j, k);
-        double acc = 0.0;
-        for (int L = 0; L < 8; L++)
-            acc += 0.125 * u[(i + (L & 1)) + (long long)g.nx * ((j + ((L >> 1) & 1)) + (long long)g.ny * (k + (L >> 2)))];
-        if (clamp) {
-            if (acc < 0.0) acc = 0.0;
-            if (acc > 1.0) acc = 1.0;
-        }
-        xout[e] = acc;
-        if (xphys) xphys[e] = projection ? (tanh(beta * eta) + tanh(beta * (acc - eta))) / den : acc;
-    }
-}
-
 // Filter::Gradients chain rule of the projection (Filter.cc:128-169)
 __global__ void k_chain(long long nel, const double *__restrict__ xt, double *df, int m, double *dg, double beta,
                         double eta) {
-    double den = tanh(beta * eta) + tanh(beta * (1.0 - eta));
+    const double scale = beta / (tanh(beta * eta) + tanh(beta * (1.0 - eta)));
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < nel; e += (long long)gridDim.x * blockDim.x) {
-        double t = tanh(beta * (xt[e] - eta));
-        double d = beta * (1.0 - t * t) / den;
+        const double d = scale * proj_sech2(beta * (xt[e] - eta));
         df[e] *= d;
         for (int j = 0; j < m; j++) dg[(long long)j * nel + e] *= d;
     }
-}
-
-__global__ void k_filt_dinv(GridDesc g, KFMat KF, double *dinv) {
-    long long nn = g.nn();
-    for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < nn; n += (long long)gridDim.x * blockDim.x) {
-        int i, j, k;
-        lex3(n, g.nx, g.ny, i, j, k);
-        double acc = 0.0;
-        for (int c = 0; c < 8; c++) {
-            int ei = i - (c & 1), ej = j - ((c >> 1) & 1), ek = k - (c >> 2);
-            if (ei < 0 || ej < 0 || ek < 0 || ei >= g.ex || ej >= g.ey || ek >= g.ez) continue;
-            acc += KF.v[c * 8 + c];
-        }
-        dinv[n] = 1.0 / acc;
-    }
-}
-
-// r = b (x0 = 0), z = Dinv r, p = z; reductions b.b, r.z
-__global__ void k_fpcg_init(long long n, const double *__restrict__ b, const double *__restrict__ dinv, double *x,
-                            double *r, double *p, FiltScalars *S, Partials<2> part) {
-    double v[2] = {0.0, 0.0};
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        double bi = b[i];
-        x[i] = 0.0;
-        r[i] = bi;
-        double zi = dinv[i] * bi;
-        p[i] = zi;
-        v[0] += bi * bi;
-        v[1] += bi * zi;
-    }
-    double tot[2];
-    if (grid_reduce<EW, 2>(v, part, tot)) {
-        S->bb = tot[0];
-        S->rr = tot[0];
-        S->rz = tot[1];
-        S->it = 0;
-        S->status = 0;
-        S->done = (tot[0] == 0.0);
-    }
-}
-
-// x += a p, r -= a q, z = Dinv r, red r.r, r.z -> beta, convergence
-__global__ void k_fpcg_update(long long n, const double *__restrict__ dinv, double *x, double *r,
-                              const double *__restrict__ p, const double *__restrict__ q, FiltScalars *S,
-                              Partials<2> part) {
-    if (S->done) return;
-    double a = S->alpha;
-    double v[2] = {0.0, 0.0};
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        x[i] += a * p[i];
-        double ri = r[i] - a * q[i];
-        r[i] = ri;
-        v[0] += ri * ri;
-        v[1] += ri * dinv[i] * ri;
-    }
-    double tot[2];
-    if (grid_reduce<EW, 2>(v, part, tot)) {
-        S->rr = tot[0];
-        S->rz_old = S->rz;
-        S->rz = tot[1];
-        S->beta = tot[1] / S->rz_old;
-        S->it += 1;
-        if (!isfinite(tot[0])) {
-            S->status = TOPO_ERR_NAN;
-            S->done = 1;
-        } else if (tot[0] <= S->tol2 * S->bb) {
-            S->done = 1;
-        } else if (S->it >= S->maxit) {
-            S->status = TOPO_ERR_NOT_CONVERGED;
-            S->done = 1;
-        }
-    }
-}
-
-__global__ void k_fpcg_p(long long n, const double *__restrict__ dinv, const double *__restrict__ r, double *p,
-                         const FiltScalars *S) {
-    if (S->done) return;
-    double b = S->beta;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        p[i] = dinv[i] * r[i] + b * p[i];
-}
-
-__global__ void k_fprime(FiltScalars *S, double tol2, int maxit) {
-    S->tol2 = tol2;
-    S->maxit = maxit;
-    S->done = 0;
-    S->status = 0;
 }
 
 // GetMND (Filter.cc:208-227)
@@ -240,16 +453,12 @@ int pdefilt_create(TopoPDEFilt **out, int nx, int ny, int nz, double hx, double 
     }
     TopoPDEFilt *f = new TopoPDEFilt();
     f->g = GridDesc{nx, ny, nz, nx - 1, ny - 1, nz - 1};
-    f->h[0] = hx;
-    f->h[1] = hy;
-    f->h[2] = hz;
-    f->R = rmin / 2.0 / sqrt(3.0);  // PDEFilter.cc:32
-    f->vol = hx * hy * hz;
+    const double R = rmin / 2.0 / sqrt(3.0);  // PDEFilter.cc:32
     f->rtol = rtol;
     f->maxit = maxit;
     // KF = R^2 * Laplacian + mass of the box: mode-basis diagonal, mapped back
     // to the reference local node order (PDEFilter.cc:485-578 gives the same
-    // matrix in closed form)
+    // matrix in closed form); FiltOp holds the same operator for the solve
     {
         const double w[2] = {0.25, 1.0 / 12.0};
         double V = hx * hy * hz, g2[3] = {4.0 / (hx * hx), 4.0 / (hy * hy), 4.0 / (hz * hz)};
@@ -262,10 +471,8 @@ int pdefilt_create(TopoPDEFilt **out, int nx, int ny, int nz, double hx, double 
                     int ms = m & ~(1 << a);
                     lap += g2[a] * V * w[ms & 1] * w[(ms >> 1) & 1] * w[(ms >> 2) & 1];
                 }
-            dm[m] = f->R * f->R * lap + Wm;
+            dm[m] = R * R * lap + Wm;
         }
-        // reference local order node r -> lexicographic L
-        const int lex[8] = {0, 1, 3, 2, 4, 5, 7, 6};
         for (int col = 0; col < 8; col++) {
             double v[8] = {0};
             v[col] = 1.0;
@@ -274,7 +481,17 @@ int pdefilt_create(TopoPDEFilt **out, int nx, int ny, int nz, double hx, double 
             mode_bwd(v);
             for (int L = 0; L < 8; L++) f->KF[L * 8 + col] = v[L];
         }
-        (void)lex;
+    }
+    {
+        const double m[2] = {4.0 / 6.0, 1.0 / 6.0}, k[2] = {2.0, -1.0};  // own node, a neighbour
+        const double rho[3] = {R * R / (hx * hx), R * R / (hy * hy), R * R / (hz * hz)};
+        for (int S = 0; S < 8; S++) {
+            const int b[3] = {S & 1, (S >> 1) & 1, S >> 2};
+            double c = m[b[0]] * m[b[1]] * m[b[2]];
+            for (int a = 0; a < 3; a++) c += rho[a] * k[b[a]] * m[b[(a + 1) % 3]] * m[b[(a + 2) % 3]];
+            f->args.Kd.c[S] = c;
+            f->args.Kf.c[S] = (float)c;
+        }
     }
     cudaError_t e = cudaStreamCreateWithFlags(&f->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) {
@@ -295,31 +512,50 @@ int pdefilt_create(TopoPDEFilt **out, int nx, int ny, int nz, double hx, double 
         return 0;
     };
     int rc = 0;
-    rc |= get((void **)&f->rhs, sizeof(double) * nn);
-    rc |= get((void **)&f->u, sizeof(double) * nn);
-    rc |= get((void **)&f->r, sizeof(double) * nn);
-    rc |= get((void **)&f->p, sizeof(double) * nn);
-    rc |= get((void **)&f->q, sizeof(double) * nn);
-    rc |= get((void **)&f->dinv, sizeof(double) * nn);
-    rc |= get((void **)&f->e1, sizeof(double) * nel);
-    rc |= get((void **)&f->e2, sizeof(double) * nel);
-    rc |= get((void **)&f->S, sizeof(FiltScalars));
+    FiltArgs &A = f->args;
+    A.g = f->g;
+    for (int r = 0; r < FILT_RHS; r++) {
+        for (int k = 0; k < 2; k++) {
+            rc |= get((void **)&A.u[r][k], sizeof(double) * nn);
+            for (float **q : {&A.r32[r][k], &A.s32[r][k], &A.w32[r][k]}) rc |= get((void **)q, sizeof(float) * nn);
+        }
+        for (double **q : {&A.b[r], &A.r[r]}) rc |= get((void **)q, sizeof(double) * nn);
+        for (float **q : {&A.p32[r], &A.d32[r]}) rc |= get((void **)q, sizeof(float) * nn);
+    }
+    rc |= get((void **)&f->mnd, sizeof(double));
     rc |= get((void **)&f->part, sizeof(double) * 2 * 65536);
     rc |= get((void **)&f->counter, sizeof(unsigned int) * 4);
     if (rc) {
         pdefilt_destroy(f);
         return TOPO_ERR_OOM;
     }
-    KFMat K;
-    memcpy(K.v, f->KF, sizeof(K.v));
-    count_launch();
-    k_filt_dinv<<<ew_blocks(nn), EW, 0, f->stream>>>(f->g, K, f->dinv);
-    e = cudaStreamSynchronize(f->stream);
-    if (e != cudaSuccess) {
+    e = cudaHostAlloc((void **)&f->status, sizeof(FiltStatus), cudaHostAllocMapped);
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&A.out, f->status, 0);
+    // resident CTAs, and runs of planes that give each about one: a run reads two planes more than it completes
+    int dev = 0, nsm = 0, per_sm = 0;
+    if (e == cudaSuccess) e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_filt_solve, FT_N, 0);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(f->stream);
+    if (e != cudaSuccess || per_sm < 1) {
         set_error(std::string("PDE filter setup: ") + cudaGetErrorString(e));
         pdefilt_destroy(f);
         return TOPO_ERR_CUDA;
     }
+    const int resident = per_sm * nsm;
+    const Patch pt = plane_patch(nx, ny, FT_N, 1, FT_PLANE);
+    A.tx = pt.tx;
+    A.ty = pt.ty;
+    A.ntx = pt.ntx;
+    A.nty = pt.nty;
+    const int runs = std::max(1, std::min(nz, resident / std::max(1, A.ntx * A.nty)));
+    A.cz = (nz + runs - 1) / runs;
+    A.ncz = (nz + A.cz - 1) / A.cz;
+    f->grid = (unsigned)std::min(resident, A.ntx * A.nty * A.ncz);
+    A.tol = rtol;
+    A.maxit = maxit;
+    A.part = f->part;
+    A.bar = GridBar{f->counter + 1, f->counter + 2, f->counter + 3};
     *out = f;
     return TOPO_OK;
 }
@@ -327,6 +563,7 @@ int pdefilt_create(TopoPDEFilt **out, int nx, int ny, int nz, double hx, double 
 void pdefilt_destroy(TopoPDEFilt *f) {
     if (!f) return;
     for (void *p : f->ptrs) cudaFree(p);
+    if (f->status) cudaFreeHost(f->status);
     if (f->stream) cudaStreamDestroy(f->stream);
     delete f;
 }
@@ -334,58 +571,46 @@ void pdefilt_destroy(TopoPDEFilt *f) {
 long long pdefilt_nel(const TopoPDEFilt *f) { return f->g.nel(); }
 const double *pdefilt_matrix(const TopoPDEFilt *f) { return f->KF; }
 
-// U = K^-1 (vol T x) by Jacobi PCG; the host polls convergence every 8 iterations
-static int helmholtz_solve(TopoPDEFilt *f, const double *x_dev) {
+// results of up to FILT_RHS element fields, in place allowed (every input is
+// read before the first result is written)
+static int filt_solve(TopoPDEFilt *f, int nr, const double *const *xin, double *const *xout, double *xphys, int clamp,
+                      int projection, double beta, double eta) {
     cudaStream_t s = f->stream;
-    long long nn = f->g.nn();
-    Partials<1> p1{f->part, f->counter};
-    Partials<2> p2{f->part, f->counter};
-    KFMat K;
-    memcpy(K.v, f->KF, sizeof(K.v));
+    FiltArgs A = f->args;
+    A.nr = nr;
+    for (int r = 0; r < nr; r++) {
+        A.xin[r] = xin[r];
+        A.xout[r] = xout[r];
+    }
+    A.xphys = xphys;
+    A.clamp = clamp;
+    A.projection = projection;
+    A.beta = beta;
+    A.eta = eta;
+    f->status->status = TOPO_ERR_CUDA;
+    void *args[] = {&A};
     count_launch();
-    k_T<<<ew_blocks(nn), EW, 0, s>>>(f->g, f->vol, x_dev, f->rhs);
-    count_launch();
-    k_fprime<<<1, 1, 0, s>>>(f->S, f->rtol * f->rtol, f->maxit);
-    count_launch();
-    k_fpcg_init<<<red_blocks(nn), EW, 0, s>>>(nn, f->rhs, f->dinv, f->u, f->r, f->p, f->S, p2);
-    FiltScalars h;
-    for (int outer = 0; outer < 1000000; outer++) {
-        for (int it = 0; it < 8; it++) {
-            count_launch();
-            k_filt_apply<<<red_blocks(nn), EW, 0, s>>>(f->g, K, f->p, f->q, p1, f->S, 1);
-            count_launch();
-            k_fpcg_update<<<red_blocks(nn), EW, 0, s>>>(nn, f->dinv, f->u, f->r, f->p, f->q, f->S, p2);
-            count_launch();
-            k_fpcg_p<<<ew_blocks(nn), EW, 0, s>>>(nn, f->dinv, f->r, f->p, f->S);
-        }
-        FCK(cudaMemcpyAsync(&h, f->S, sizeof(h), cudaMemcpyDeviceToHost, s));
+    FCK(cudaLaunchCooperativeKernel((const void *)k_filt_solve, dim3(f->grid), dim3(FT_N), args, 0, s));
+    FCK(cudaStreamSynchronize(s));
+    const int st = *(volatile int *)&f->status->status;
+    if (st == TOPO_OK) return TOPO_OK;
+    if (st == TOPO_ERR_CUDA) {  // the grid barrier gave up
+        FCK(cudaMemsetAsync(f->counter + 1, 0, 3 * sizeof(unsigned), s));
         FCK(cudaStreamSynchronize(s));
-        if (h.done) break;
+        set_error("PDE filter: the solve's grid barrier ran out of time");
+    } else {
+        set_error(std::string("PDE filter solve failed with status ") + std::to_string(st));
     }
-    if (h.status) {
-        set_error(std::string("PDE filter solve failed with status ") + std::to_string(h.status));
-        return h.status;
-    }
-    return TOPO_OK;
+    return st;
 }
 
 int pdefilt_apply_dev(TopoPDEFilt *f, const double *x_dev, double *xout_dev) {
-    int rc = helmholtz_solve(f, x_dev);
-    if (rc) return rc;
-    count_launch();
-    k_Tt<<<ew_blocks(f->g.nel()), EW, 0, f->stream>>>(f->g, f->u, xout_dev, nullptr, 0, 0, 0.0, 0.0);
-    FCK(cudaStreamSynchronize(f->stream));
-    return TOPO_OK;
+    return filt_solve(f, 1, &x_dev, &xout_dev, nullptr, 0, 0, 0.0, 0.0);
 }
 
 int filter_project_dev(TopoPDEFilt *f, const double *x_dev, double *xTilde_dev, double *xPhys_dev, int projection,
                        double beta, double eta) {
-    int rc = helmholtz_solve(f, x_dev);
-    if (rc) return rc;
-    count_launch();
-    k_Tt<<<ew_blocks(f->g.nel()), EW, 0, f->stream>>>(f->g, f->u, xTilde_dev, xPhys_dev, 1, projection, beta, eta);
-    FCK(cudaStreamSynchronize(f->stream));
-    return TOPO_OK;
+    return filt_solve(f, 1, &x_dev, &xTilde_dev, xPhys_dev, 1, projection, beta, eta);
 }
 
 int filter_gradients_dev(TopoPDEFilt *f, const double *xTilde_dev, double *dfdx_dev, int m, double *dgdx_dev,
@@ -395,14 +620,12 @@ int filter_gradients_dev(TopoPDEFilt *f, const double *xTilde_dev, double *dfdx_
         count_launch();
         k_chain<<<ew_blocks(nel), EW, 0, f->stream>>>(nel, xTilde_dev, dfdx_dev, m, dgdx_dev, beta, eta);
     }
-    // PDEFilt::Gradients == FilterProject (PDEFilter.cc:224); in place via scratch
-    FCK(cudaMemcpyAsync(f->e1, dfdx_dev, sizeof(double) * nel, cudaMemcpyDeviceToDevice, f->stream));
-    int rc = pdefilt_apply_dev(f, f->e1, dfdx_dev);
-    if (rc) return rc;
-    for (int j = 0; j < m; j++) {
-        FCK(cudaMemcpyAsync(f->e1, dgdx_dev + (size_t)j * nel, sizeof(double) * nel, cudaMemcpyDeviceToDevice,
-                            f->stream));
-        rc = pdefilt_apply_dev(f, f->e1, dgdx_dev + (size_t)j * nel);
+    // PDEFilt::Gradients == FilterProject (PDEFilter.cc:224), dfdx and the m columns of dgdx
+    for (int j = 0; j <= m; j += FILT_RHS) {
+        double *v[FILT_RHS];
+        int nr = 0;
+        for (; nr < FILT_RHS && j + nr <= m; nr++) v[nr] = j + nr == 0 ? dfdx_dev : dgdx_dev + (size_t)(j + nr - 1) * nel;
+        const int rc = filt_solve(f, nr, v, v, nullptr, 0, 0, 0.0, 0.0);
         if (rc) return rc;
     }
     return TOPO_OK;
@@ -412,8 +635,8 @@ int filter_mnd_dev(TopoPDEFilt *f, const double *x_dev, double *mnd) {
     long long nel = f->g.nel();
     Partials<1> p1{f->part, f->counter};
     count_launch();
-    k_mnd<<<red_blocks(nel), EW, 0, f->stream>>>(nel, x_dev, p1, f->e2);
-    FCK(cudaMemcpyAsync(mnd, f->e2, sizeof(double), cudaMemcpyDeviceToHost, f->stream));
+    k_mnd<<<red_blocks(nel), EW, 0, f->stream>>>(nel, x_dev, p1, f->mnd);
+    FCK(cudaMemcpyAsync(mnd, f->mnd, sizeof(double), cudaMemcpyDeviceToHost, f->stream));
     FCK(cudaStreamSynchronize(f->stream));
     return TOPO_OK;
 }
