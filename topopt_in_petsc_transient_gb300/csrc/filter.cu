@@ -56,8 +56,8 @@ struct FiltArgs {
     int nr;                             // right-hand sides
     const double *xin[FILT_RHS];        // element fields
     double *xout[FILT_RHS], *xphys;     // results; xphys: clamp and project (one right-hand side)
-    int clamp, projection;
-    double beta, eta;
+    int clamp;
+    Projection proj;
     double *u[FILT_RHS][2], *b[FILT_RHS], *r[FILT_RHS];
     float *r32[FILT_RHS][2], *s32[FILT_RHS][2], *w32[FILT_RHS][2], *p32[FILT_RHS], *d32[FILT_RHS];
     double tol;
@@ -386,7 +386,6 @@ __global__ void __launch_bounds__(FT_N, 3) k_filt_solve(const FiltArgs A) {
     if (status == TOPO_OK) {
         // xout = T^t u; optional clamp to [0,1] and smoothed Heaviside projection
         // (Filter.cc:83-113, Filter.h:80-83)
-        const double th = tanh(A.beta * A.eta), rden = 1.0 / (th + tanh(A.beta * (1.0 - A.eta)));
         for (int r = 0; r < A.nr; r++) {
             const double *u = A.u[r][ub];
             for (long long e = t0; e < nel; e += ts) {
@@ -401,7 +400,7 @@ __global__ void __launch_bounds__(FT_N, 3) k_filt_solve(const FiltArgs A) {
                     if (acc > 1.0) acc = 1.0;
                 }
                 A.xout[r][e] = acc;
-                if (A.xphys) A.xphys[e] = A.projection ? (th + proj_tanh(A.beta * (acc - A.eta))) * rden : acc;
+                if (A.xphys) A.xphys[e] = project(A.proj, acc);
             }
         }
     }
@@ -424,11 +423,9 @@ struct TopoPDEFilt {
 };
 
 // Filter::Gradients chain rule of the projection (Filter.cc:128-169)
-__global__ void k_chain(long long nel, const double *__restrict__ xt, double *df, int m, double *dg, double beta,
-                        double eta) {
-    const double scale = beta / (tanh(beta * eta) + tanh(beta * (1.0 - eta)));
+__global__ void k_chain(long long nel, const double *__restrict__ xt, double *df, int m, double *dg, Projection pr) {
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < nel; e += (long long)gridDim.x * blockDim.x) {
-        const double d = scale * proj_sech2(beta * (xt[e] - eta));
+        const double d = project_slope(pr, xt[e]);
         df[e] *= d;
         for (int j = 0; j < m; j++) dg[(long long)j * nel + e] *= d;
     }
@@ -584,9 +581,7 @@ static int filt_solve(TopoPDEFilt *f, int nr, const double *const *xin, double *
     }
     A.xphys = xphys;
     A.clamp = clamp;
-    A.projection = projection;
-    A.beta = beta;
-    A.eta = eta;
+    A.proj = make_projection(projection, beta, eta);
     f->status->status = TOPO_ERR_CUDA;
     void *args[] = {&A};
     count_launch();
@@ -618,7 +613,8 @@ int filter_gradients_dev(TopoPDEFilt *f, const double *xTilde_dev, double *dfdx_
     long long nel = f->g.nel();
     if (projection) {
         count_launch();
-        k_chain<<<ew_blocks(nel), EW, 0, f->stream>>>(nel, xTilde_dev, dfdx_dev, m, dgdx_dev, beta, eta);
+        k_chain<<<ew_blocks(nel), EW, 0, f->stream>>>(nel, xTilde_dev, dfdx_dev, m, dgdx_dev,
+                                                         make_projection(1, beta, eta));
     }
     // PDEFilt::Gradients == FilterProject (PDEFilter.cc:224), dfdx and the m columns of dgdx
     for (int j = 0; j <= m; j += FILT_RHS) {

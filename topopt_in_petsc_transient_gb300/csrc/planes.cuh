@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 
 namespace topo {
 
@@ -34,6 +35,20 @@ inline Patch plane_patch(int nx, int ny, int nt, int halo, int most) {
 // quotient: E = exp(-2 |v|), tanh v = +-(1 - E) / (1 + E), 1 - tanh^2 v =
 // 4 E / (1 + E)^2.  FP64 runs at 2 lanes a clock and SM here, and tanh() takes
 // both of its branches in most warps.
+// its constants, formed once on the host: a thread of a launch with one element
+// a thread would spend more FP64 time on them than on its element
+struct Projection {
+    int on;  // 0: copy
+    double beta, eta, th, rden;  // th = tanh(beta eta), rden = 1 / (th + tanh(beta (1 - eta)))
+};
+inline Projection make_projection(int on, double beta, double eta) {
+    Projection p{on, beta, eta, 0.0, 1.0};
+    if (on) {
+        p.th = std::tanh(beta * eta);
+        p.rden = 1.0 / (p.th + std::tanh(beta * (1.0 - eta)));
+    }
+    return p;
+}
 __device__ __forceinline__ double proj_tanh(double v) {
     const double E = exp(-2.0 * fabs(v));
     return copysign((1.0 - E) / (1.0 + E), v);
@@ -41,6 +56,12 @@ __device__ __forceinline__ double proj_tanh(double v) {
 __device__ __forceinline__ double proj_sech2(double v) {
     const double E = exp(-2.0 * fabs(v)), r = 1.0 / (1.0 + E);
     return 4.0 * E * (r * r);
+}
+__device__ __forceinline__ double project(const Projection &p, double x) {
+    return p.on ? (p.th + proj_tanh(p.beta * (x - p.eta))) * p.rden : x;
+}
+__device__ __forceinline__ double project_slope(const Projection &p, double x) {
+    return p.beta * p.rden * proj_sech2(p.beta * (x - p.eta));
 }
 
 }  // namespace topo
