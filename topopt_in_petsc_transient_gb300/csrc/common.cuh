@@ -261,21 +261,23 @@ struct Partials {
 };
 
 template <int NT, int NV>
-__device__ __forceinline__ void block_reduce(double v[NV], double *smem /* [NV][NT/32] */) {
+__device__ __forceinline__ void block_reduce(double v[NV], double *smem /* [NV][NT/32] */, int nwarps = NT / 32) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (wid < nwarps) {
 #pragma unroll
-    for (int i = 0; i < NV; i++) {
-        double x = v[i];
+        for (int i = 0; i < NV; i++) {
+            double x = v[i];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-        if (lane == 0) smem[i * (NT / 32) + wid] = x;
+            for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+            if (lane == 0) smem[i * (NT / 32) + wid] = x;
+        }
     }
     __syncthreads();
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int i = 0; i < NV; i++) {
             double s = 0.0;
-            for (int w = 0; w < NT / 32; w++) s += smem[i * (NT / 32) + w];
+            for (int w = 0; w < nwarps; w++) s += smem[i * (NT / 32) + w];
             v[i] = s;
         }
     }
@@ -331,7 +333,8 @@ __device__ __forceinline__ bool grid_reduce_blocks(double v[NV], const Partials<
 #pragma unroll
         for (int i = 0; i < NV; i++) s[i] += ((volatile double *)P.part)[(size_t)b * NV + i];
     __syncthreads();
-    block_reduce<NT, NV>(s, sred);
+    // warps without a partial hold zeros: they add nothing and stay off the FP64 pipe
+    block_reduce<NT, NV>(s, sred, nblk < NT ? (int)((nblk + 31) / 32) : NT / 32);
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int i = 0; i < NV; i++) tot[i] = s[i];

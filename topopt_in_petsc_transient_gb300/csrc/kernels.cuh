@@ -23,10 +23,11 @@ __host__ inline unsigned red_blocks(long long n) {
 // Chebyshev coefficients (c1, c2) of steps k = 0..kmax-1 from the device-side
 // spectrum bounds; computed once per design iteration so that no kernel
 // repeats the FP64 divisions per thread
-static __global__ void k_cheb_table(const double *lohi, int kmax, double *coef) {
-    double c1, c2;
+// thread 0: the smoothing interval's table, thread 1: the full spectrum's
+static __global__ void k_cheb_table(const double *lohi, int kmax, double *smooth, double *full) {
+    double *coef = threadIdx.x ? full : smooth, c1, c2;
     for (int k = 0; k < kmax; k++) {
-        cheb_coeffs<double>(lohi, k, c1, c2);
+        cheb_coeffs<double>(lohi + 2 * threadIdx.x, k, c1, c2);
         coef[2 * k] = c1;
         coef[2 * k + 1] = c2;
     }
@@ -333,28 +334,76 @@ static __global__ void k_coarse_assemble(GridDesc g, const uint8_t *__restrict__
     }
 }
 
-// Dense coarsest-level operator (SPD, FP64).  Cholesky factor A = L L' in
-// place in the lower triangle, right-looking, one column per step in two
-// passes: the updated column k is saved (k_chol_save), then scaled into
-// L(:, k) and the trailing lower triangle updated, A(i, j) -= L(i, k) L(j, k)
-// (k_chol_update).  Then W = L^-1 by forward substitution (row i of W scaled
-// by 1 / L(i, i), then subtracted from the rows below) and A^-1 = W' W, so the
-// V-cycle's coarse solve stays one dense matrix-vector product.
-static __global__ void k_chol_save(const double *A, int n, int k, double *col) {
-    for (int t = k + blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
-        col[t] = A[(size_t)t * n + k];
+// Dense coarsest-level operator (SPD, FP64): Cholesky factor A = L L' in place
+// in the lower triangle, right-looking, then W = L^-1 by forward substitution
+// and A^-1 = W' W, so the V-cycle's coarse solve stays one dense matrix-vector
+// product.  In panels of CH columns: every entry takes the same operations in
+// the same order as column by column (a -= (c_i / c_k) c_j for k ascending, c
+// the updated, unscaled column k), with two launches a panel where a column
+// took two: 8 ms of launches for n = 675 become 0.6.
+constexpr int CH = 32;
+// panel k0: rows k0 + 32 b .. of block b, one row a lane, the diagonal block
+// factored by every CTA for itself.  Uc, Qc [n][CH]: unscaled columns and c_i / c_k.
+static __global__ void __launch_bounds__(32) k_chol_panel(double *A, int n, int k0, double *Uc, double *Qc) {
+    const int lane = threadIdx.x, w = min(CH, n - k0);
+    double d[CH], a[CH];
+#pragma unroll
+    for (int j = 0; j < CH; j++) d[j] = lane < w && j <= lane ? A[(size_t)(k0 + lane) * n + k0 + j] : 0.0;
+#pragma unroll
+    for (int k = 0; k < CH; k++) {
+        if (k >= w) break;
+        const double q = d[k] / __shfl_sync(0xffffffffu, d[k], k);
+#pragma unroll
+        for (int j = k + 1; j < CH; j++) d[j] -= q * __shfl_sync(0xffffffffu, d[k], j);
+    }
+    const int row = k0 + CH * blockIdx.x + lane;  // block 0: the diagonal block's own rows
+    if (blockIdx.x == 0) {
+#pragma unroll
+        for (int k = 0; k < CH; k++) {
+            if (k >= w) break;
+            const double p = __shfl_sync(0xffffffffu, d[k], k), r = sqrt(p);
+            if (lane < w && k <= lane) A[(size_t)row * n + k0 + k] = k == lane ? r : d[k] / r;
+        }
+        return;
+    }
+#pragma unroll
+    for (int j = 0; j < CH; j++) a[j] = row < n && j < w ? A[(size_t)row * n + k0 + j] : 0.0;
+#pragma unroll
+    for (int k = 0; k < CH; k++) {
+        if (k >= w) break;
+        const double p = __shfl_sync(0xffffffffu, d[k], k), q = a[k] / p;
+#pragma unroll
+        for (int j = k + 1; j < CH; j++) a[j] -= q * __shfl_sync(0xffffffffu, d[k], j);
+        if (row < n) {
+            Uc[(size_t)row * CH + k] = a[k];
+            Qc[(size_t)row * CH + k] = q;
+            A[(size_t)row * n + k0 + k] = a[k] / sqrt(p);
+        }
+    }
 }
-static __global__ void k_chol_update(double *A, int n, int k, const double *__restrict__ col) {
-    const long long m = n - k;
-    const double p = col[k], d = sqrt(p);
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < m * m; t += (long long)gridDim.x * blockDim.x) {
-        const int i = k + (int)(t / m), j = k + (int)(t % m);
-        if (j > i) continue;
-        double &a = A[(size_t)i * n + j];
-        if (j == k)
-            a = (i == k) ? d : col[i] / d;
-        else
-            a -= (col[i] / p) * col[j];  // L(i, k) L(j, k) = col_i col_j / col_k
+// C(i, j) -= sum over the CH columns k of X(i, k) Y(k, j), k ascending, on 32 x 32
+// tiles at rows r0.. and columns c0..; sx, sy: row strides, ty: Y given as Y(j, k).
+// lower: tiles on and below the diagonal only.
+static __global__ void __launch_bounds__(256) k_chol_update(double *C, int n, int r0, int c0, int c1, const double *X,
+                                                            int sx, const double *Y, int sy, int ty, int lower) {
+    __shared__ double xs[CH][CH + 1], ys[CH][CH + 1];
+    const int i0 = r0 + CH * blockIdx.y, j0 = c0 + CH * blockIdx.x;
+    if (lower && j0 > i0) return;
+    const int tx = threadIdx.x & 31, tw = threadIdx.x >> 5;
+    for (int r = tw; r < CH; r += 8) {
+        xs[r][tx] = i0 + r < n ? X[(size_t)(i0 + r) * sx + tx] : 0.0;
+        if (ty) ys[r][tx] = j0 + r < c1 ? Y[(size_t)(j0 + r) * sy + tx] : 0.0;
+        else ys[tx][r] = j0 + tx < c1 ? Y[(size_t)r * sy + j0 + tx] : 0.0;
+    }
+    __syncthreads();
+    const int j = j0 + tx;
+    for (int r = tw; r < CH; r += 8) {
+        const int i = i0 + r;
+        if (i >= n || j >= c1 || (lower && j > i)) continue;
+        double v = C[(size_t)i * n + j];
+#pragma unroll
+        for (int k = 0; k < CH; k++) v -= xs[r][k] * ys[tx][k];
+        C[(size_t)i * n + j] = v;
     }
 }
 static __global__ void k_chol_identity(double *W, int n) {
@@ -362,27 +411,54 @@ static __global__ void k_chol_identity(double *W, int n) {
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < tot; t += (long long)gridDim.x * blockDim.x)
         W[t] = (t / n == t % n) ? 1.0 : 0.0;
 }
-// forward substitution step i: row i of W (columns <= i) divided by L(i, i)
-static __global__ void k_chol_trsv_scale(const double *L, double *W, int n, int i) {
-    const double d = L[(size_t)i * n + i];
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c <= i; c += gridDim.x * blockDim.x) W[(size_t)i * n + c] /= d;
-}
-// rows r > i of W (columns <= i) minus L(r, i) times row i
-static __global__ void k_chol_trsv_update(const double *L, double *W, int n, int i) {
-    const long long w = i + 1, tot = (long long)(n - i - 1) * w;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < tot; t += (long long)gridDim.x * blockDim.x) {
-        const int r = i + 1 + (int)(t / w), c = (int)(t % w);
-        W[(size_t)r * n + c] -= L[(size_t)r * n + i] * W[(size_t)i * n + c];
+// forward substitution within the rows i0 .. i0 + 31 of W, one column a lane:
+// row i divided by L(i, i), then L(r, i) times it taken from the rows r below
+static __global__ void __launch_bounds__(32) k_chol_trsv(const double *L, double *W, int n, int i0) {
+    __shared__ double Ld[CH][CH + 1];
+    const int lane = threadIdx.x, h = min(CH, n - i0), c = CH * blockIdx.x + lane;
+    for (int r = 0; r < h; r++) Ld[r][lane] = lane < h ? L[(size_t)(i0 + r) * n + i0 + lane] : 0.0;
+    __syncwarp();
+    double w[CH];
+#pragma unroll
+    for (int r = 0; r < CH; r++) w[r] = r < h && c < i0 + h ? W[(size_t)(i0 + r) * n + c] : 0.0;
+#pragma unroll
+    for (int i = 0; i < CH; i++) {
+        if (i >= h) break;
+        w[i] /= Ld[i][i];
+#pragma unroll
+        for (int r = i + 1; r < CH; r++)
+            if (r < h) w[r] -= Ld[r][i] * w[i];
     }
+#pragma unroll
+    for (int r = 0; r < CH; r++)
+        if (r < h && c < i0 + h) W[(size_t)(i0 + r) * n + c] = w[r];
 }
-// A^-1 = W' W with W = L^-1 lower triangular: Ainv(i, j) = sum over r >= max(i, j) of W(r, i) W(r, j)
-static __global__ void k_chol_gram(const double *__restrict__ W, int n, double *Ainv) {
-    const long long tot = (long long)n * n;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < tot; t += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(t / n), j = (int)(t % n);
-        double s = 0.0;
-        for (int r = i > j ? i : j; r < n; r++) s += W[(size_t)r * n + i] * W[(size_t)r * n + j];
-        Ainv[t] = s;
+// A^-1 = W' W with W = L^-1 lower triangular: sum over r >= max(i, j) of W(r, i) W(r, j)
+// (the rows above hold zeros), r ascending; 32 x 32 tiles
+static __global__ void __launch_bounds__(256) k_chol_gram(const double *__restrict__ W, int n, double *Ainv,
+                                                          float *Ainvf) {
+    __shared__ double a[CH][CH + 1], b[CH][CH + 1];
+    const int i0 = CH * blockIdx.y, j0 = CH * blockIdx.x, tx = threadIdx.x & 31, tw = threadIdx.x >> 5;
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int r0 = max(i0, j0); r0 < n; r0 += CH) {
+        __syncthreads();
+        for (int r = tw; r < CH; r += 8) {
+            a[r][tx] = r0 + r < n && i0 + tx < n ? W[(size_t)(r0 + r) * n + i0 + tx] : 0.0;
+            b[r][tx] = r0 + r < n && j0 + tx < n ? W[(size_t)(r0 + r) * n + j0 + tx] : 0.0;
+        }
+        __syncthreads();
+        const int h = min(CH, n - r0);
+        for (int r = 0; r < h; r++)
+#pragma unroll
+            for (int u = 0; u < 4; u++) s[u] += a[r][tw + 8 * u] * b[r][tx];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const int i = i0 + tw + 8 * u, j = j0 + tx;
+        if (i < n && j < n) {
+            Ainv[(size_t)i * n + j] = s[u];
+            Ainvf[(size_t)i * n + j] = (float)s[u];
+        }
     }
 }
 

@@ -734,7 +734,7 @@ int le_alloc(TopoLE *le) {
             CK(cudaMemcpy(le->KEc, KE, sizeof(KE), cudaMemcpyHostToDevice));
             CK(cudaMemcpy(le->MEc, ME, sizeof(ME), cudaMemcpyHostToDevice));
             AG(le->chol_w, (size_t)lnd * lnd);
-            AG(le->chol_col, lnd);
+            AG(le->chol_col, 2 * (size_t)CH * lnd);
         }
     }
     le->L[0].kfd = le->kf;
@@ -821,33 +821,11 @@ static int cheb_kmax(const TopoLE *le) {
 static int setup_operator(TopoLE *le, int o) {
     Operator &op = le->ops[o];
     cudaStream_t s = le->stream;
-    for (int l = 0; l < le->nlev; l++) {
-        Level &lv = le->L[l];
-        const double *kfp = (op.sK != 0.0) ? lv.kfd : nullptr;
-        count_launch();
-        k_dinv<<<ew_blocks(lv.g.nn()), EW, 0, s>>>(lv.g, lv.fixed, kfp, lv.mfd, op.sK, op.sM, lv.dK[0], lv.dK[1],
-                                                   lv.dK[2], lv.dM, op.lv[l].dinvd, op.lv[l].dinvf);
-        count_launch();
-        k_bounds_init<<<1, 1, 0, s>>>(le->bbits);
-        count_launch();
-        k_bounds<<<ew_blocks(lv.g.nel()), EW, 0, s>>>(lv.g.nel(), kfp, lv.mfd, op.sK, op.sM, lv.dK[0], lv.dK[1],
-                                                      lv.dK[2], lv.dM, lv.lamK, 0.125, 3.375, le->bbits);
-        count_launch();
-        k_bounds_final<<<1, 1, 0, s>>>(le->bbits, le->p.cheb_ratio, op.lv[l].lohi);
-        count_launch();
-        k_cheb_table<<<1, 1, 0, s>>>(op.lv[l].lohi, cheb_kmax(le), op.lv[l].cheb);
-        count_launch();
-        k_cheb_table<<<1, 1, 0, s>>>(op.lv[l].lohi + 2, cheb_kmax(le), op.lv[l].chebf);
-    }
-    // Kronecker mass preconditioner: node scaling and the stiffness share
+    // Kronecker mass preconditioner: the stiffness share
     // (sK / sM) max_e(kf_e / mf_e) lambda_max(KE, ME), which bounds the
     // operator against its mass part: u'Au <= (1 + share) sM u'Mu
     {
         Level &l0 = le->L[0];
-        count_launch();
-        k_kron_scale<double><<<ew_blocks(l0.g.nn()), EW, 0, s>>>(l0.g, l0.fixed, l0.mfd, op.sM, op.kscale_d);
-        count_launch();
-        k_kron_scale<float><<<ew_blocks(l0.g.nn()), EW, 0, s>>>(l0.g, l0.fixed, l0.mfd, op.sM, op.kscale_f);
         op.share = 0.0;
         if (op.sK != 0.0) {
             unsigned long long hb = 0ull;
@@ -865,6 +843,37 @@ static int setup_operator(TopoLE *le, int o) {
                                       std::max(kron_yz_smem(l0.g, 2, 8), kron_yz_smem(l0.g, 2, 4, true)));
         op.kron = stage <= KRON_SMEM_MAX && op.sM > 0.0 && op.sK >= 0.0 &&
                   (le->p.mass_precond == 1 || (le->p.mass_precond == 2 && op.share <= le->p.mass_precond_share));
+        if (op.kron) {  // its node scaling, in the precision of the solves
+            count_launch();
+            if (le->p.mixed)
+                k_kron_scale<float><<<ew_blocks(l0.g.nn()), EW, 0, s>>>(l0.g, l0.fixed, l0.mfd, op.sM, op.kscale_f);
+            else
+                k_kron_scale<double><<<ew_blocks(l0.g.nn()), EW, 0, s>>>(l0.g, l0.fixed, l0.mfd, op.sM, op.kscale_d);
+        }
+    }
+    // V-cycle levels; the Kronecker preconditioner takes none, or the finest
+    // one's tables for its smoothing steps
+    const int nlev = !op.kron ? le->nlev : (le->p.mass_precond_smooth > 0 ? 1 : 0);
+    for (int l = 0; l < nlev; l++) {
+        Level &lv = le->L[l];
+        const double *kfp = (op.sK != 0.0) ? lv.kfd : nullptr;
+        count_launch();
+        k_dinv<<<ew_blocks(lv.g.nn()), EW, 0, s>>>(lv.g, lv.fixed, kfp, lv.mfd, op.sK, op.sM, lv.dK[0], lv.dK[1],
+                                                   lv.dK[2], lv.dM, op.lv[l].dinvd, op.lv[l].dinvf);
+        count_launch();
+        k_bounds_init<<<1, 1, 0, s>>>(le->bbits);
+        count_launch();
+        k_bounds<<<ew_blocks(lv.g.nel()), EW, 0, s>>>(lv.g.nel(), kfp, lv.mfd, op.sK, op.sM, lv.dK[0], lv.dK[1],
+                                                      lv.dK[2], lv.dM, lv.lamK, 0.125, 3.375, le->bbits);
+        count_launch();
+        k_bounds_final<<<1, 1, 0, s>>>(le->bbits, le->p.cheb_ratio, op.lv[l].lohi);
+        count_launch();
+        k_cheb_table<<<1, 2, 0, s>>>(op.lv[l].lohi, cheb_kmax(le), op.lv[l].cheb, op.lv[l].chebf);
+    }
+    if (op.kron) {
+        op.depth = 0;  // no V-cycle; a step captured with one is captured again
+        CK(cudaGetLastError());
+        return TOPO_OK;
     }
     // adaptive depth: stop at the first level whose Jacobi-scaled operator is
     // well conditioned (bound hi/lo <= adaptive_kappa); a full-spectrum
@@ -896,28 +905,31 @@ static int setup_operator(TopoLE *le, int o) {
     k_coarse_assemble<<<ew_blocks((long long)n * n), EW, 0, s>>>(lc.g, lc.fixed, kfp, lc.mfd, op.sK, op.sM, le->KEc,
                                                                  le->MEc, op.Ainv_d);
     // FP64 Cholesky factor of the coarsest operator, then its inverse from the
-    // factor (k_chol_*): A^-1 = L^-T L^-1
-    for (int k = 0; k < n; k++) {
+    // factor (k_chol_*): A^-1 = L^-T L^-1, written over the factor's storage
+    // (the Gram product reads W alone)
+    double *A = op.Ainv_d, *W = le->chol_w, *Uc = le->chol_col, *Qc = le->chol_col + (size_t)CH * n;
+    auto tiles = [](int m) { return (unsigned)((m + CH - 1) / CH); };
+    for (int k0 = 0; k0 < n; k0 += CH) {
         count_launch();
-        k_chol_save<<<(n + EW - 1) / EW, EW, 0, s>>>(op.Ainv_d, n, k, le->chol_col);
+        k_chol_panel<<<tiles(n - k0), 32, 0, s>>>(A, n, k0, Uc, Qc);
+        const int m = n - k0 - CH;  // rows below the panel (which then is a whole one)
+        if (m <= 0) break;
         count_launch();
-        k_chol_update<<<ew_blocks((long long)(n - k) * (n - k)), EW, 0, s>>>(op.Ainv_d, n, k, le->chol_col);
+        k_chol_update<<<dim3(tiles(m), tiles(m)), 256, 0, s>>>(A, n, k0 + CH, k0 + CH, n, Qc, CH, Uc, CH, 1, 1);
     }
     count_launch();
-    k_chol_identity<<<ew_blocks((long long)n * n), EW, 0, s>>>(le->chol_w, n);
-    for (int i = 0; i < n; i++) {
+    k_chol_identity<<<ew_blocks((long long)n * n), EW, 0, s>>>(W, n);
+    for (int i0 = 0; i0 < n; i0 += CH) {
+        const int c1 = std::min(n, i0 + CH), m = n - i0 - CH;
         count_launch();
-        k_chol_trsv_scale<<<(i + EW) / EW, EW, 0, s>>>(op.Ainv_d, le->chol_w, n, i);
-        if (i + 1 < n) {
-            count_launch();
-            k_chol_trsv_update<<<ew_blocks((long long)(n - i - 1) * (i + 1)), EW, 0, s>>>(op.Ainv_d, le->chol_w,
-                                                                                           n, i);
-        }
+        k_chol_trsv<<<tiles(c1), 32, 0, s>>>(A, W, n, i0);
+        if (m <= 0) break;
+        count_launch();
+        k_chol_update<<<dim3(tiles(c1), tiles(m)), 256, 0, s>>>(W, n, i0 + CH, 0, c1, A + i0, n, W + (size_t)i0 * n, n,
+                                                                 0, 0);
     }
     count_launch();
-    k_chol_gram<<<ew_blocks((long long)n * n), EW, 0, s>>>(le->chol_w, n, op.Ainv_d);
-    count_launch();
-    k_d2f<<<ew_blocks((long long)n * n), EW, 0, s>>>((long long)n * n, op.Ainv_d, op.Ainv_f);
+    k_chol_gram<<<dim3(tiles(n), tiles(n)), 256, 0, s>>>(W, n, A, op.Ainv_f);
     CK(cudaGetLastError());
     return TOPO_OK;
 }
