@@ -79,6 +79,8 @@ struct ElemConst {
     T g[3];      // 2 / h_a
     T lam, mu;   // Lame parameters for E = 1 (LinearElasticity.cc:3134-3135)
     T K[KH_NNZ]; // Khat blocks, row-major per block, blocks in kh_idx order
+    T Q[7];      // equal edges: the distinct entries of Khat (mode_cube)
+    int cube;    // 1: hx = hy = hz
 };
 
 template <class T>
@@ -198,6 +200,13 @@ inline ElemConst<T> make_elem_const(double hx, double hy, double hz, double nu) 
     for (int b = 0; b < KH_NB; b++)
         for (int r = 0; r < kh_size(b); r++)
             for (int s = 0; s < kh_size(b); s++) c.K[k++] = (T)Kh[kh_idx(b, r)][kh_idx(b, s)];
+    // mode_cube: g^2 W_n times Lame combinations, g = 2 / h and W_n the weight
+    // of n difference modes
+    const double g2 = d.g[0] * d.g[0], w0 = g2 * d.W[0], w1 = g2 * d.W[1], w2 = g2 * d.W[3];
+    const double q[7] = {2.0 * d.mu * w0, d.lam * w0,  d.mu * w0, d.mu * w1, (d.lam + 3.0 * d.mu) * w1,
+                         d.lam * w1,      (d.lam + 4.0 * d.mu) * w2};
+    for (int i = 0; i < 7; i++) c.Q[i] = (T)q[i];
+    c.cube = (hx == hy && hy == hz) ? 1 : 0;
     return c;
 }
 
@@ -247,6 +256,84 @@ __host__ __device__ __forceinline__ void mode_khat_mass(const ElemConst<T> &C, T
             Y[ir / 8][ir % 8] = MASS ? tadd(tmul(ck, acc), tmul(cw[ir % 8], U[ir / 8][ir % 8])) : tmul(ck, acc);
         }
         k += n * n;
+    }
+}
+
+// Y = ck Khat U + cm W .* U of an element with three equal edges, from the
+// structure of its Khat blocks: per weight there are only two coefficients,
+//   {1,10,20}  own-axis differences:  out_i = 2 mu a_i + lam (a + b + c)
+//   {2,9} {4,17} {12,18}  shear pairs: both rows mu (a + b)
+//   {6,13,19}  mixed pairs:           out_i = mu (a_i + a + b + c)
+//   {3,22} {5,14} {11,21}:            (lam + 3 mu) a + lam b and its mirror
+//   {7} {15} {23}:                    (lam + 4 mu) a
+// With the mass added to the diagonal coefficients once per element this takes
+// 35 products and 25 sums (stiffness alone 25 and 19) against the 45 and 24 of
+// the stored blocks plus 45 and 24 for the two weights.
+template <bool HK, bool HM, class T>
+__host__ __device__ __forceinline__ void mode_cube(const ElemConst<T> &C, T ck, T cm, const T U[3][8], T Y[3][8]) {
+    static_assert(HK, "the mass alone is diagonal");
+    const T q0 = tmul(ck, C.Q[0]), q1 = tmul(ck, C.Q[1]), q2 = tmul(ck, C.Q[2]), q3 = tmul(ck, C.Q[3]),
+            q4 = tmul(ck, C.Q[4]), q5 = tmul(ck, C.Q[5]), q6 = tmul(ck, C.Q[6]);
+    const T m0 = HM ? tmul(cm, C.W[0]) : T(0), m1 = HM ? tmul(cm, C.W[1]) : T(0), m2 = HM ? tmul(cm, C.W[3]) : T(0),
+            m3 = HM ? tmul(cm, C.W[7]) : T(0);
+    {  // own-axis differences
+        const T a = U[0][1], b = U[1][2], c = U[2][4];
+        const T s = tmul(q1, tadd(tadd(a, b), c)), d = HM ? tadd(q0, m1) : q0;
+        Y[0][1] = tadd(tmul(d, a), s);
+        Y[1][2] = tadd(tmul(d, b), s);
+        Y[2][4] = tadd(tmul(d, c), s);
+    }
+#pragma unroll
+    for (int p = 0; p < 3; p++) {  // axes (c0, c1): component c0 along c1 with component c1 along c0
+        const int c0 = p == 2 ? 1 : 0, c1 = p == 0 ? 1 : 2, i0 = 1 << c1, i1 = 1 << c0;
+        const T a = U[c0][i0], b = U[c1][i1], t = tmul(q2, tadd(a, b));
+        Y[c0][i0] = HM ? tadd(t, tmul(m1, a)) : t;
+        Y[c1][i1] = HM ? tadd(t, tmul(m1, b)) : t;
+    }
+    {  // mixed pairs
+        const T a = U[0][6], b = U[1][5], c = U[2][3], s = tadd(tadd(a, b), c);
+        if (HM) {
+            const T t = tmul(q3, s), d = tadd(q3, m2);
+            Y[0][6] = tadd(tmul(d, a), t);
+            Y[1][5] = tadd(tmul(d, b), t);
+            Y[2][3] = tadd(tmul(d, c), t);
+        } else {
+            Y[0][6] = tmul(q3, tadd(a, s));
+            Y[1][5] = tmul(q3, tadd(b, s));
+            Y[2][3] = tmul(q3, tadd(c, s));
+        }
+    }
+    const T d2 = HM ? tadd(q4, m2) : q4;
+#pragma unroll
+    for (int p = 0; p < 3; p++) {  // axes (c0, c1), the difference along the third axis dropped
+        const int c0 = p == 2 ? 1 : 0, c1 = p == 0 ? 1 : 2, s = 7 & ~((1 << c0) | (1 << c1));
+        const int i0 = (1 << c0) | s, i1 = (1 << c1) | s;
+        const T a = U[c0][i0], b = U[c1][i1];
+        Y[c0][i0] = tadd(tmul(d2, a), tmul(q5, b));
+        Y[c1][i1] = tadd(tmul(d2, b), tmul(q5, a));
+    }
+    const T d3 = HM ? tadd(q6, m3) : q6;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        Y[c][7] = tmul(d3, U[c][7]);
+        Y[c][0] = HM ? tmul(m0, U[c][0]) : T(0);
+    }
+}
+
+// the element operator of the operator kernel: Y = ck Khat U + cm W .* U
+template <bool CUBE, bool HK, bool HM, class T>
+__host__ __device__ __forceinline__ void mode_apply(const ElemConst<T> &C, T ck, T cm, const T U[3][8], T Y[3][8]) {
+    if constexpr (!HK) {
+#pragma unroll
+        for (int m = 0; m < 8; m++) {
+            const T w = tmul(cm, C.W[m]);
+#pragma unroll
+            for (int c = 0; c < 3; c++) Y[c][m] = tmul(w, U[c][m]);
+        }
+    } else if constexpr (CUBE) {
+        mode_cube<HK, HM>(C, ck, cm, U, Y);
+    } else {
+        mode_khat_mass<HM>(C, ck, cm, U, Y);
     }
 }
 
@@ -362,4 +449,89 @@ __device__ __forceinline__ bool grid_reduce(const float vf[NV], const Partials<N
     return grid_reduce_blocks<NT, NV>(v, P, tot, sred);
 }
 
+// The same sums in another order, for the kernels of the FP64 solves: a third of
+// the FP64 instructions.  The kernels of the mixed path keep grid_reduce's order:
+// their results pass through FP32 roundings that turn a change in the last bit of
+// a sum into one of 1e-8 of the sensitivities.
+// CTA sums in thread 0, from one value per thread (NT: the largest CTA, nt: the
+// threads of this one, whole warps).  GB300 issues an FP64 instruction of a warp
+// every 16 clocks of an SM, so a shuffle tree in every warp (5 additions each)
+// keeps the FP64 pipe busy for over a thousand clocks; here one warp adds the
+// columns of the CTA's values (NT / 32 + 5 additions in all).
+template <int NT, int NV>
+struct RedSmem {
+    double v[NV][NT];
+};
+template <int NT, int NV>
+__device__ __forceinline__ void block_reduce64(double v[NV], RedSmem<NT, NV> &sm, int nt = NT) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+    for (int i = 0; i < NV; i++) sm.v[i][threadIdx.x] = v[i];
+    __syncthreads();
+    if (wid == 0) {
+#pragma unroll
+        for (int i = 0; i < NV; i++) {
+            double s = sm.v[i][lane];
+            for (int t = lane + 32; t < nt; t += 32) s += sm.v[i][t];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            v[i] = s;
+        }
+    }
+}
+
+// the grid stage of grid_reduce64: v holds the CTA sums in thread 0.  In the last
+// CTA one warp a value adds the partials, eight strides of loads in flight at
+// once (one round trip to L2 for 256 CTAs), so the summation order depends only
+// on the grid size.
+template <int NV>
+__device__ __forceinline__ bool grid_reduce64_blocks(double v[NV], const Partials<NV> &P, double tot[NV], int nt) {
+    __shared__ bool last;
+    __shared__ double stot[NV];
+    const unsigned int nblk = gridDim.x * gridDim.y * gridDim.z;
+    const unsigned int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int i = 0; i < NV; i++) P.part[(size_t)bid * NV + i] = v[i];
+        __threadfence();
+        unsigned int t = atomicAdd(P.counter, 1u);
+        last = (t == nblk - 1);
+    }
+    __syncthreads();
+    if (!last) return false;
+    __threadfence();
+    const int lane = threadIdx.x & 31;
+    for (int i = threadIdx.x >> 5; i < NV; i += nt / 32) {
+        double s = 0.0;
+        for (unsigned int b = lane; b < nblk; b += 256) {
+            double t[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+                t[u] = b + 32 * u < nblk ? ((volatile double *)P.part)[(size_t)(b + 32 * u) * NV + i] : 0.0;
+#pragma unroll
+            for (int u = 0; u < 8; u++) s += t[u];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) stot[i] = s;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int j = 0; j < NV; j++) tot[j] = stot[j];
+        *P.counter = 0u;
+        return true;
+    }
+    return false;
+}
+
+// Called by every thread of every CTA (1D-linearised block id; NT: the largest
+// CTA, nt: the threads of this one, whole warps).  Returns true in exactly one thread (thread 0 of the last CTA to
+// finish); on that thread `tot` holds the grid sums.
+template <int NT, int NV>
+__device__ __forceinline__ bool grid_reduce64(double v[NV], const Partials<NV> &P, double tot[NV], int nt = NT) {
+    __shared__ RedSmem<NT, NV> sred;
+    block_reduce64<NT, NV>(v, sred, nt);
+    return grid_reduce64_blocks<NV>(v, P, tot, nt);
+}
 }  // namespace topo

@@ -485,7 +485,7 @@ static __global__ void k_fcg_dot(long long ndof, const TZ *__restrict__ z, const
         v[1] += zi * q[i];
     }
     double tot[2];
-    if (grid_reduce<EW, 2>(v, part, tot)) {
+    if (grid_reduce64<EW, 2>(v, part, tot)) {
         S->rho = tot[0];
         S->gam = tot[1];
         S->beta = (S->it == 0) ? 0.0 : -tot[1] / S->pq;
@@ -516,7 +516,7 @@ static __global__ void k_fcg_update(long long ndof, double *x, double *r, float 
         v[0] += rv * rv;
     }
     double tot[1];
-    if (grid_reduce<EW, 1>(v, part, tot)) {
+    if (grid_reduce64<EW, 1>(v, part, tot)) {
         S->rr = tot[0];
         S->it += 1;
         S->total_it += 1;

@@ -93,17 +93,23 @@ struct KronDot {
 };
 
 constexpr int KRON_THREADS = 256;
-constexpr size_t KRON_SMEM_MAX = 200 * 1024;    // per-CTA staging limit (the selection checks it)
+constexpr size_t KRON_SMEM_MAX = 211328;    // per-CTA staging limit (the selection checks it)
 constexpr int KRON_MP = 8;                      // outputs per thread along a line
 constexpr int KRON_WIN = KRON_MP + 2 * KRON_B;  // register window
+constexpr int KRON_TAPS = 3 * KRON_W * (1 + 2 * KRON_B);  // staged taps of one axis: interior, then the end rows
 
-// interior taps of one axis for the three components: the exact row at the
-// middle of the line (lines shorter than 2 KRON_B + 1 have no interior)
+// taps of one axis for the three components in shared memory: the interior ones
+// (the exact row at the middle of the line; lines shorter than 2 KRON_B + 1 have
+// no interior), then the exact rows of the 2 KRON_B positions at the ends, which
+// are half of a line of 25.  Read from global memory where they are used, a row
+// a lane in the x pass, they cost 24.8 instead of 15.3 us in FP64 at 49x25x25 and
+// 11.8 instead of 10.4 us a pass in FP32 at 62x38x31
 template <class T>
-__device__ __forceinline__ void kron_stage_interior(const KronBand<T> &B, int axis, int len, T *tint) {
-    for (int t = threadIdx.x; t < 3 * KRON_W; t += blockDim.x) {
-        const int c = t / KRON_W, d = t - c * KRON_W;
-        tint[t] = B.row(axis, c, len / 2)[d];
+__device__ __forceinline__ void kron_stage_taps(const KronBand<T> &B, int axis, int len, T *taps) {
+    const int ne = len < 2 * KRON_B ? len : 2 * KRON_B;
+    for (int t = threadIdx.x; t < 3 * KRON_W * (1 + ne); t += blockDim.x) {
+        const int row = t / KRON_W, d = t - row * KRON_W, e = row / 3, c = row - 3 * e;
+        taps[t] = B.row(axis, c, e == 0 ? len / 2 : (e <= KRON_B || len < 2 * KRON_B ? e - 1 : len - 2 * KRON_B + e - 1))[d];
     }
 }
 
@@ -111,7 +117,7 @@ __device__ __forceinline__ void kron_stage_interior(const KronBand<T> &B, int ax
 // src[p * sstride]); outputs past the line end are computed but not used
 template <class T>
 __device__ __forceinline__ void kron_line(const T *src, int sstride, int len, int p0, const T *tint,
-                                          const KronBand<T> &B, int axis, int c, T out[KRON_MP]) {
+                                          int c, T out[KRON_MP]) {
     T win[KRON_WIN];
 #pragma unroll
     for (int k = 0; k < KRON_WIN; k++) {
@@ -135,8 +141,9 @@ __device__ __forceinline__ void kron_line(const T *src, int sstride, int len, in
 #pragma unroll
     for (int k = 0; k < KRON_MP; k++) {
         const int pos = p0 + k;
-        const T *tp = (pos >= KRON_B && pos < len - KRON_B) ? tint + c * KRON_W
-                                                            : B.row(axis, c, pos < len ? pos : len - 1);
+        const int q = pos < len ? pos : len - 1;
+        const int e = q < KRON_B || len < 2 * KRON_B ? q + 1 : (q < len - KRON_B ? 0 : q - len + 2 * KRON_B + 1);
+        const T *tp = tint + (3 * e + c) * KRON_W;
         T acc = T(0);
 #pragma unroll
         for (int d = 0; d < KRON_W; d++) acc += tp[d] * win[k + d];
@@ -157,7 +164,7 @@ __host__ inline int kx_lines(const GridDesc &g, size_t elem) {
     return L < 1 ? 1 : (L > 8 ? 8 : L);
 }
 __host__ inline size_t kron_x_smem(const GridDesc &g, size_t elem, int kx = 0) {
-    return elem * ((size_t)(kx > 0 ? kx : kx_lines(g, elem)) * 2 * 3 * kx_pitch(g.nx) + 3 * KRON_W);
+    return elem * ((size_t)(kx > 0 ? kx : kx_lines(g, elem)) * 2 * 3 * kx_pitch(g.nx) + KRON_TAPS);
 }
 // lines per CTA for a launch: the shared-memory cap, lowered so that the grid
 // still fills one wave of `slots` resident CTAs
@@ -176,14 +183,14 @@ __device__ __forceinline__ void kron_x_body(const GridDesc &g, int kx, R *r, con
     const int LP = kx_pitch(g.nx);
     T *tile = reinterpret_cast<T *>(kron_smem);  // [kx][3][LP]
     T *otile = tile + kx * 3 * LP;               // [kx][3][LP]
-    T *tint = otile + kx * 3 * LP;               // [3][KRON_W]
+    T *tint = otile + kx * 3 * LP;               // [KRON_TAPS]
     const int row = 3 * g.nx;
     const long long nlines = (long long)g.ny * g.nz;
     const long long line0 = (long long)blockIdx.x * kx;
     const int nl = (int)(nlines - line0 < kx ? nlines - line0 : kx);
     const bool rs = S != nullptr && S->rescale != 0;
     const ScaleF64 sg = scale_split(rs ? S->sigma : 1.0);
-    kron_stage_interior(B, 0, g.nx, tint);
+    kron_stage_taps(B, 0, g.nx, tint);
     const long long q0 = line0 * row;
     const int nv = nl * row;
     // t / row by a multiply-high with ceil(2^32 / row), exact for t < 2^32 / row
@@ -212,7 +219,7 @@ __device__ __forceinline__ void kron_x_body(const GridDesc &g, int kx, R *r, con
         const int c = rw % 3;
         const int p0 = grp * KRON_MP;
         T o[KRON_MP];
-        kron_line(tile + rw * LP, 1, g.nx, p0, tint, B, 0, c, o);
+        kron_line(tile + rw * LP, 1, g.nx, p0, tint, c, o);
 #pragma unroll
         for (int k = 0; k < KRON_MP; k++)
             if (p0 + k < g.nx) otile[rw * LP + p0 + k] = o[k];
@@ -246,7 +253,7 @@ __host__ inline unsigned kron_yz_blocks(const GridDesc &g, int axis) {
 }
 __host__ inline size_t kron_yz_smem(const GridDesc &g, int axis, size_t elem, bool dot = false) {
     const size_t len = (size_t)(axis == 1 ? g.ny : g.nz);
-    return elem * (KW * len * (axis == 2 ? 3 : 1) + 3 * KRON_W) + (dot ? sizeof(float) * KW * len : 0);
+    return elem * (KW * len * (axis == 2 ? 3 : 1) + KRON_TAPS) + (dot ? sizeof(float) * KW * len : 0);
 }
 
 template <class T, class R, int AXIS, bool DOT>
@@ -256,8 +263,8 @@ static __global__ void __launch_bounds__(KRON_THREADS, sizeof(T) == 4 ? 4 : 2)
     TOPO_DYNAMIC_SMEM(unsigned char, kron_smem);
     const int len = AXIS == 1 ? g.ny : g.nz;
     T *tile = reinterpret_cast<T *>(kron_smem);  // [len][KW]
-    T *tint = tile + (size_t)len * KW;           // [3][KRON_W]
-    T *rt = tint + 3 * KRON_W;                   // AXIS 2: r [len][KW]
+    T *tint = tile + (size_t)len * KW;           // [KRON_TAPS]
+    T *rt = tint + KRON_TAPS;                    // AXIS 2: r [len][KW]
     T *mt = rt + (size_t)len * KW;               // AXIS 2: masked scale [len][KW]
     float *qt = reinterpret_cast<float *>(mt + (size_t)len * KW);  // DOT: q [len][KW]
     const int row = 3 * g.nx;
@@ -266,7 +273,7 @@ static __global__ void __launch_bounds__(KRON_THREADS, sizeof(T) == 4 ? 4 : 2)
     const int w0 = chunk * KW, wn = (row - w0 < KW) ? row - w0 : KW;
     const long long S = AXIS == 1 ? (long long)row : (long long)row * g.ny;
     const long long base = AXIS == 1 ? (long long)other * row * g.ny + w0 : (long long)other * row + w0;
-    kron_stage_interior(B, AXIS, len, tint);
+    kron_stage_taps(B, AXIS, len, tint);
     // the staging is a pure copy: cp.async puts every copy of the chunk in
     // flight at once, with no register round trip
     static_assert(std::is_same<T, R>::value, "staged r is copied, not converted");
@@ -295,7 +302,7 @@ static __global__ void __launch_bounds__(KRON_THREADS, sizeof(T) == 4 ? 4 : 2)
         const int c = (w0 + w) % 3;
         const int p0 = grp * KRON_MP;
         T o[KRON_MP];
-        kron_line(tile + w, KW, len, p0, tint, B, AXIS, c, o);
+        kron_line(tile + w, KW, len, p0, tint, c, o);
 #pragma unroll
         for (int k = 0; k < KRON_MP; k++) {
             const int p = p0 + k;

@@ -263,29 +263,59 @@ constexpr int tile_class() {
                                                                                                : -1;
 }
 
-// FP32 tile kernels and kernels staged by asynchronous copies are persistent: as many
-// CTAs as are resident on the device at once (occupancy of this instantiation
-// x SM count), capped by the brick count; the others launch one CTA per brick
+// SMs of the current device
+static int sm_count() {
+    static int nsm_dev[MAX_DEVICES] = {};
+    int &nsm = nsm_dev[device_slot()];
+    if (!nsm) {
+        int dev = 0, n = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        nsm = std::max(n, 1);
+    }
+    return nsm;
+}
+
+// FP64: columns of elements (march.cuh).  A smoothing step takes 22 us instead
+// of 38 over the levels of 48x24x24 (a brick alone took 35 us of its SM's FP64
+// pipe on every level), the product of the FCG at 48x24x24 33 instead of 46
+template <class Pol>
+static void launch_march(const GridDesc &g, const ElemConst<double> &C, const Pol &pol, cudaStream_t s) {
+    const MarchDims d = march_config(g, sm_count());
+    const size_t sm = march_smem_bytes(d.tx, d.ty, Pol::M_IN);  // at most 40 KB
+    const unsigned grid = (unsigned)((long long)d.ntx * d.nty * d.ncz);
+    count_launch();
+    if (Pol::HAS_K && C.cube)
+        k_march<Pol, true><<<grid, d.tx * d.ty, sm, s>>>(g, C, pol, d);
+    else
+        k_march<Pol, false><<<grid, d.tx * d.ty, sm, s>>>(g, C, pol, d);
+}
+// FP32 and double-float: bricks.  FP32 kernels and kernels staged by asynchronous
+// copies are persistent: as many CTAs as are resident on the device at once
+// (occupancy of this instantiation x SM count), capped by the brick count; the
+// others launch one CTA per brick
 template <class T, class Pol>
 static void launch_tile(const GridDesc &g, const ElemConst<T> &C, const Pol &pol, cudaStream_t s) {
-    static int resident_dev[MAX_DEVICES] = {};
-    int &resident = resident_dev[device_slot()];
-    const size_t sm = TileSmem<T, Pol>::bytes;
-    if (!resident) {
-        cudaFuncSetAttribute(k_tile<T, Pol>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        int dev = 0, nsm = 0, per_sm = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tile<T, Pol>, TILE_THREADS, sm);
-        resident = std::max(1, per_sm) * std::max(1, nsm);
+    if constexpr (std::is_same<T, double>::value) {
+        launch_march(g, C, pol, s);
+    } else {
+        static int resident_dev[MAX_DEVICES] = {};
+        int &resident = resident_dev[device_slot()];
+        const size_t sm = TileSmem<T, Pol>::bytes;
+        if (!resident) {
+            cudaFuncSetAttribute(k_tile<T, Pol>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            int per_sm = 0;
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tile<T, Pol>, TILE_THREADS, sm);
+            resident = std::max(1, per_sm) * sm_count();
+        }
+        int ntx, nty;
+        const int ntiles = tile_count(g, ntx, nty);
+        const bool timed = tile_class<T, Pol>() >= 0 && timer_begin(tile_class<T, Pol>(), g.nn(), s);
+        count_launch();
+        const int grid = (tile_persistent<T>() || tile_async<T, Pol>()) ? std::min(ntiles, resident) : ntiles;
+        k_tile<T, Pol><<<(unsigned)grid, TILE_THREADS, sm, s>>>(g, C, pol);
+        timer_end(timed, s);
     }
-    int ntx, nty;
-    const int ntiles = tile_count(g, ntx, nty);
-    const bool timed = tile_class<T, Pol>() >= 0 && timer_begin(tile_class<T, Pol>(), g.nn(), s);
-    count_launch();
-    const int grid = (tile_persistent<T>() || tile_async<T, Pol>()) ? std::min(ntiles, resident) : ntiles;
-    k_tile<T, Pol><<<(unsigned)grid, TILE_THREADS, sm, s>>>(g, C, pol);
-    timer_end(timed, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -1079,15 +1109,7 @@ static T *kron_apply(TopoLE *le, int o, T *r, VFuse *fz = nullptr) {
     const T *sc = kron_scale<T>(le->ops[o]);
     const bool mixed = fz && std::is_same<T, float>::value;
     const long long nlines = (long long)g.ny * g.nz;
-    static int nsm_dev[MAX_DEVICES] = {};
-    int &nsm = nsm_dev[device_slot()];
-    if (!nsm) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        nsm = std::max(nsm, 1);
-    }
-    const int kx = kx_lines_launch(g, sizeof(T), 4LL * nsm);  // 4 resident CTAs of the x pass per SM
+    const int kx = kx_lines_launch(g, sizeof(T), 4LL * sm_count());  // 4 resident CTAs of the x pass per SM
     const size_t smx = kron_x_smem(g, sizeof(T), kx), smy = kron_yz_smem(g, 1, sizeof(T));
     static bool attr_dev[MAX_DEVICES] = {};
     bool &attr = attr_dev[device_slot()];
@@ -1349,15 +1371,14 @@ static int solve(TopoLE *le, int o, const double *b, bool capturing) {
 // ---------------------------------------------------------------------------
 // forward step j of block c (SolveStateBlock, LinearElasticity.cc:1317-1385)
 // ---------------------------------------------------------------------------
-template <class A>
-static void fwd_rhs_t(TopoLE *le) {
+static void fwd_rhs(TopoLE *le) {
     const LEParams &p = le->p;
     Level &l0 = le->L[0];
     const double *a = le->a;
-    PolRhsFwd<A> pr;
+    PolRhsFwd<double> pr;
     memset(&pr, 0, sizeof(pr));
     pr.fixed = l0.fixed;
-    pr.w = fine_weights<A>(le, true, true, nullptr, 1.0, 1.0);
+    pr.w = fine_weights<double>(le, true, true, nullptr, 1.0, 1.0);
     pr.cp = le->cp;
     pr.Uh = le->Uh;
     pr.DUh = le->DUh;
@@ -1389,13 +1410,7 @@ static void fwd_rhs_t(TopoLE *le) {
     pr.st = le->st;
     pr.b = le->sb;
     pr.x0 = le->sx;
-    launch_tile<A>(l0.g, fine_const<A>(le), pr, le->stream);
-}
-static void fwd_rhs(TopoLE *le) {
-    if (le->p.mixed)
-        fwd_rhs_t<df>(le);
-    else
-        fwd_rhs_t<double>(le);
+    launch_tile<double>(l0.g, l0.Cd, pr, le->stream);
 }
 
 // coefficients of the next-step preparation (k_newmark_track, k_fwd_prep)

@@ -1,4 +1,5 @@
-// policies.cuh -- fused epilogues for the matrix-free tile kernel (tile.cuh).
+// policies.cuh -- fused epilogues for the matrix-free operator kernels (tile.cuh
+// for FP32 and double-float, march.cuh for FP64).
 //
 // Masking convention: the Dirichlet vector N of the reference
 // (LinearElasticity.cc:552-574) is stored as a per-node bitmask `fixed`
@@ -9,6 +10,7 @@
 #pragma once
 #include "df.cuh"
 #include "tile.cuh"
+#include "march.cuh"
 
 namespace topo {
 
@@ -104,6 +106,11 @@ struct PolInitResid {
         v[0][2] = T(x[3 * n + 2]);
         mask3(fixed[n], v[0]);
     }
+    // FP64 form (march.cuh)
+    static constexpr int M_SRC = 1, M_IN = 1;
+    __device__ const double *msrc(int) const { return x; }
+    __device__ void mval(const double raw[1], double v[1]) const { v[0] = raw[0]; }
+    __device__ const uint8_t *mmask() const { return fixed; }
     __device__ void coef(long long e, T &ck, T &cm) const { w.get(e, ck, cm); }
     __device__ void epilogue(long long n, int, int, int, const T y[3], double red[2]) const {
         uint8_t f = fixed[n];
@@ -138,6 +145,11 @@ struct PolPQ {
         v[0][2] = p[3 * n + 2];
         mask3(fixed[n], v[0]);
     }
+    // FP64 form (march.cuh)
+    static constexpr int M_SRC = 1, M_IN = 1;
+    __device__ const T *msrc(int) const { return p; }
+    __device__ void mval(const double raw[1], double v[1]) const { v[0] = raw[0]; }
+    __device__ const uint8_t *mmask() const { return fixed; }
     __device__ void coef(long long e, T &ck, T &cm) const { w.get(e, ck, cm); }
     __device__ void epilogue(long long n, int, int, int, const T y[3], double red[1]) const {
         uint8_t f = fixed[n];
@@ -352,6 +364,11 @@ struct PolCheb {
         v[0][2] = x_in[3 * n + 2];
         mask3(fixed[n], v[0]);
     }
+    // FP64 form (march.cuh)
+    static constexpr int M_SRC = 1, M_IN = 1;
+    __device__ const T *msrc(int) const { return x_in; }
+    __device__ void mval(const double raw[1], double v[1]) const { v[0] = raw[0]; }
+    __device__ const uint8_t *mmask() const { return fixed; }
     __device__ void coef(long long e, T &ck, T &cm) const { w.get(e, ck, cm); }
     struct Pre {
         T x[3], b[3], di[3], d[3];
@@ -461,6 +478,11 @@ struct PolResid {
         v[0][2] = x[3 * n + 2];
         mask3(fixed[n], v[0]);
     }
+    // FP64 form (march.cuh)
+    static constexpr int M_SRC = 1, M_IN = 1;
+    __device__ const T *msrc(int) const { return x; }
+    __device__ void mval(const double raw[1], double v[1]) const { v[0] = raw[0]; }
+    __device__ const uint8_t *mmask() const { return fixed; }
     __device__ void coef(long long e, T &ck, T &cm) const { w.get(e, ck, cm); }
     __device__ void epilogue(long long n, int, int, int, const T y[3], double *) const {
         uint8_t f = fixed[n];
@@ -494,6 +516,11 @@ struct PolProduct {
     __device__ void xform(const double raw[][3], uint8_t, T v[1][3]) const {
         for (int c = 0; c < 3; c++) v[0][c] = T(raw[0][c]);
     }
+    // FP64 form (march.cuh)
+    static constexpr int M_SRC = 1, M_IN = 1;
+    __device__ const double *msrc(int) const { return x; }
+    __device__ void mval(const double raw[1], double v[1]) const { v[0] = raw[0]; }
+    __device__ const uint8_t *mmask() const { return nullptr; }
     __device__ void coef(long long e, T &ck, T &cm) const { w.get(e, ck, cm); }
     __device__ void epilogue(long long n, int, int, int, const T yv[3], double *) const {
         y[3 * n] = todbl(yv[0]);
@@ -549,7 +576,7 @@ static __global__ void k_load_table(int Ts, double dt, int which, double scale, 
 // ---------------------------------------------------------------------------
 template <class T>
 struct PolRhsFwd {
-    static constexpr int NIN = 2, NRED = 0;
+    static constexpr int M_SRC = 3, M_IN = 2, NRED = 0;
     static constexpr bool HAS_K = true, HAS_M = true;
     const uint8_t *fixed;
     Weights<T> w;
@@ -579,18 +606,16 @@ struct PolRhsFwd {
             ddu = DDUh + (long long)(j - 1) * ndof;
         }
     }
-    __device__ void load(long long n, T v[2][3]) const {
+    __device__ const double *msrc(int a) const {
         const double *u, *du, *ddu;
         prev(u, du, ddu);
-        for (int c = 0; c < 3; c++) {
-            double a = u[3 * n + c], bb = du[3 * n + c], cc = ddu[3 * n + c];
-            v[0][c] = T(cK[0] * a + cK[1] * bb + cK[2] * cc);
-            v[1][c] = T(cM[0] * a + cM[1] * bb + cM[2] * cc);
-        }
-        mask3(fixed[n], v[0]);
-        mask3(fixed[n], v[1]);
+        return a == 0 ? u : (a == 1 ? du : ddu);
     }
-    __device__ void coef(long long e, T &ck, T &cm) const { w.get(e, ck, cm); }
+    __device__ void mval(const double r[3], double v[2]) const {
+        v[0] = cK[0] * r[0] + cK[1] * r[1] + cK[2] * r[2];
+        v[1] = cM[0] * r[0] + cM[1] * r[1] + cM[2] * r[2];
+    }
+    __device__ const uint8_t *mmask() const { return fixed; }
     __device__ void epilogue(long long n, int, int, int, const T y[3], double *) const {
         const double *u, *du, *ddu;
         prev(u, du, ddu);
