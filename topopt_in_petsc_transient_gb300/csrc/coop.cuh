@@ -57,27 +57,47 @@ __device__ __forceinline__ void grid_leave(const GridBar &b) {
     }
 }
 
-// CTA sums of NV values per thread into out[v * stride], v = 0..NV-1, in the
-// type of the values.  Every thread of the CTA calls it; `sm` is free again
-// after the caller's next barrier.  (A scalar FP64 instruction in every thread
-// of a CTA of 256 takes the SM 128 clocks: sums that may be FP32 stay FP32,
-// and scalar algebra belongs in one thread.)
-template <int NT, int NV, class V>
-__device__ __forceinline__ void cta_sums(const V v[NV], V *sm /* NV * NT / 32 */, V *out, size_t stride) {
+// CTA sums of NV FP32 values per thread into out[v * stride], v = 0..NV-1.
+// Every thread of the CTA calls it; `sm` is free again after the caller's next
+// barrier.
+template <int NT, int NV>
+__device__ __forceinline__ void cta_sums(const float v[NV], float *sm /* NV * NT / 32 */, float *out, size_t stride) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
     for (int i = 0; i < NV; i++) {
-        V x = v[i];
+        float x = v[i];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
         if (lane == 0) sm[i * (NT / 32) + wid] = x;
     }
     __syncthreads();
     if (threadIdx.x < NV) {
-        V s = V(0);
+        float s = 0.0f;
 #pragma unroll
         for (int w = 0; w < NT / 32; w++) s += sm[threadIdx.x * (NT / 32) + w];
         out[threadIdx.x * stride] = s;
+    }
+}
+// The same in FP64.  A scheduler of GB300 issues an FP64 instruction every 64
+// clocks, so the additions are spread over the first warps, a value each (one on
+// each scheduler for up to four values): NT / 32 + 5 of them in a row instead of
+// 5 NV for each of a scheduler's warps and NT / 32 in one thread (MMA update of
+// 1769472 variables 1.87 -> 1.84 ms, of 27648 0.212 -> 0.206).  (For the same
+// reason scalar FP64 algebra belongs in one thread, not in all.)
+template <int NT, int NV>
+__device__ __forceinline__ void cta_sums(const double v[NV], double *sm /* NV * NT */, double *out, size_t stride) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+    for (int i = 0; i < NV; i++) sm[i * NT + threadIdx.x] = v[i];
+    __syncthreads();
+    if (wid < NV) {
+        const double *p = sm + wid * NT;
+        double s = p[lane];
+#pragma unroll
+        for (int t = 32; t < NT; t += 32) s += p[lane + t];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) out[wid * stride] = s;
     }
 }
 // after the barrier: the grid's sums of the nv <= NT / 32 values whose CTA sums

@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(FT_N, 3) k_filt_solve(const FiltArgs A) {
         int done, idle;
     };
     __shared__ __align__(16) double pl64[2 * FT_PLANE];
-    __shared__ double sred64[FT_N / 32], stot64[FILT_RHS];
+    __shared__ double sred64[FT_N], stot64[FILT_RHS];
     __shared__ float sred[FILT_RHS][NV * FT_N / 32], stot[FILT_RHS * NV];
     __shared__ Rhs R[FILT_RHS];
     __shared__ int s_status;

@@ -217,7 +217,7 @@ __device__ __forceinline__ void mma_sums(const MMAArgs &A, const double *lam, do
 template <int M>
 static __global__ void __launch_bounds__(MMA_NT, 4) k_mma_update(const MMAArgs A) {
     constexpr int NV = M + M * (M + 1) / 2;
-    __shared__ double sred[NV * MMA_NT / 32], stot[NV];
+    __shared__ double sred[NV * MMA_NT], stot[NV];
     __shared__ MMADual<M> D;
     const MMAScalars *S = A.S;
     const long long n = A.n, t0 = blockIdx.x * (long long)MMA_NT + threadIdx.x, ts = (long long)gridDim.x * MMA_NT;
