@@ -32,6 +32,18 @@ namespace topo {
 constexpr int FILT_RHS = 2;        // right-hand sides solved at once
 constexpr int FT_N = 256;          // threads: node columns of a CTA, tx x ty of them
 constexpr int FT_PLANE = 2 * FT_N;  // most values of a staged plane: the columns and one node around
+constexpr int FT_RING = 4;          // planes whose raw values are in flight or in use
+constexpr int FT_RAW = 12;          // most bytes of a node's raw values
+struct FiltSmem {
+    double plane[2][FT_PLANE];
+    unsigned char ring[FT_RING][FT_PLANE * FT_RAW];
+};
+template <int NB>
+__device__ __forceinline__ void filt_copy(void *dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+                 "n"(NB)
+                 : "memory");
+}
 
 // Operator of the unit-scaled filter K / V (V the element volume).  The 1-D
 // assembled mass and stiffness are h [1 4 1] / 6 and [-1 2 -1] / h inside, and
@@ -70,15 +82,18 @@ struct FiltArgs {
 
 // A applied to a field in runs of planes along z, a column of nodes per thread.
 // F supplies the field and takes the products:
-//   Raw load(n); T val(Raw, s)        value of a staged node, s = 1 / d
+//   copy(ring, v, n); T val(ring, v, s)   raw values of node n into slot v of a ring plane (asynchronous
+//                                         copies); the node's value from them, s = 1 / d
 //   Own own(n); put(n, d, Own, v, y)  node n: boundary factor, operands, own value, product
 // In-plane neighbours come from one staged plane; of the two planes beside it
 // only Q, the in-plane sum with the weights of a neighbour along z, is needed,
 // kept in registers: 15 operations a node instead of 27 multiply-adds.  Bound by
-// the latency of its loads (24 warps an SM), so the staged ones are issued two
-// planes ahead of their use and the node's own one plane ahead.
+// the latency of its loads (24 warps an SM), so the staged ones are issued three
+// planes ahead of their use (2.68 -> 2.58 ms against two planes ahead in
+// registers), into slots of shared memory that only their thread
+// reads, and the node's own one plane ahead.
 template <class T, class F>
-__device__ __forceinline__ void filt_apply(const FiltArgs &A, const FiltOp<T> &K, T *plane /* [2][FT_PLANE] */, F &f) {
+__device__ __forceinline__ void filt_apply(const FiltArgs &A, const FiltOp<T> &K, FiltSmem &sm, F &f) {
     const GridDesc &g = A.g;
     const int tid = threadIdx.x, ty = tid / A.tx, tx = tid - ty * A.tx;
     const int row = A.tx + 2, nst = row * (A.ty + 2);
@@ -102,24 +117,27 @@ __device__ __forceinline__ void filt_apply(const FiltArgs &A, const FiltOp<T> &K
             sn[q] = v < nst ? si + g.nx * sj : -1;
             ss[q] = ((si == 0 || si == g.nx - 1) ? 2.0f : 1.0f) * ((sj == 0 || sj == g.ny - 1) ? 2.0f : 1.0f);
         }
-        typename F::Raw raw[2][2];  // staged values of planes k and k + 1
-        typename F::Own own[2];     // of the planes k (being staged) and k - 1 (being completed)
-        auto fetch = [&](int k, typename F::Raw v[2]) {
-            const unsigned o = nxy * (unsigned)mirror(k, g.nz);
+        typename F::Own own[2];  // of the planes k (being staged) and k - 1 (being completed)
+        auto fetch = [&](int k) {  // one group of copies a plane, empty past the run
+            if (k <= k1) {
+                const unsigned o = nxy * (unsigned)mirror(k, g.nz);
 #pragma unroll
-            for (int q = 0; q < 2; q++)
-                if (sn[q] >= 0) v[q] = f.load(o + sn[q]);
+                for (int q = 0; q < 2; q++)
+                    if (sn[q] >= 0) f.copy(sm.ring[k & (FT_RING - 1)], tid + q * FT_N, o + sn[q]);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
         };
         T vc = T(0), P = T(0), Q = T(0), Ql = T(0);
-        auto step = [&](int k, typename F::Raw v[2], typename F::Own &ok, const typename F::Own &okm1) {
-            T *pl = plane + (k & 1) * FT_PLANE;
+        auto step = [&](int k, typename F::Own &ok, const typename F::Own &okm1) {
+            T *pl = reinterpret_cast<T *>(sm.plane[k & 1]);
+            asm volatile("cp.async.wait_group %0;" ::"n"(FT_RING - 2) : "memory");  // this thread's copies of plane k
             const float sz = (k <= 0 || k >= g.nz - 1) && k != -1 && k != g.nz ? 2.0f : 1.0f;
             // beyond an end the mirrored plane 1 or nz - 2 is staged, itself an end plane when nz = 2
             const float s2 = (k == -1 || k == g.nz) && g.nz == 2 ? 2.0f : sz;
 #pragma unroll
             for (int q = 0; q < 2; q++)
-                if (sn[q] >= 0) pl[tid + q * FT_N] = f.val(v[q], s2 * ss[q]);
-            if (k + 1 < k1) fetch(k + 2, v);
+                if (sn[q] >= 0) pl[tid + q * FT_N] = f.val(sm.ring[k & (FT_RING - 1)], tid + q * FT_N, s2 * ss[q]);
+            fetch(k + FT_RING - 1);
             if (in && k >= k0 && k < k1) ok = f.own(nij + nxy * (unsigned)k);
             __syncthreads();  // one barrier a plane: the other buffer was last read before the previous one
             if (in) {
@@ -135,12 +153,13 @@ __device__ __forceinline__ void filt_apply(const FiltArgs &A, const FiltOp<T> &K
                 vc = c;
             }
         };
-        fetch(k0 - 1, raw[0]);
-        fetch(k0, raw[1]);
-        for (int k = k0 - 1; k <= k1; k += 2) {  // by two: the buffers swap by name, no copies that wait for loads
-            step(k, raw[0], own[0], own[1]);
-            if (k + 1 <= k1) step(k + 1, raw[1], own[1], own[0]);
+#pragma unroll
+        for (int k = 0; k < FT_RING - 1; k++) fetch(k0 - 1 + k);
+        for (int k = k0 - 1; k <= k1; k += 2) {  // by two: the operands swap by name, no copies that wait for loads
+            step(k, own[0], own[1]);
+            if (k + 1 <= k1) step(k + 1, own[1], own[0]);
         }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();  // the planes are restaged by the next run
     }
 }
@@ -150,10 +169,11 @@ struct FiltStart {
     const double *r64;
     ScaleF64 sg;
     float dinv, *r, *w, *d, sum[3];
-    using Raw = double;
     using Own = double;
-    __device__ Raw load(unsigned n) const { return r64[n]; }
-    __device__ float val(Raw v, float s) const { return s * dinv * scaled_f32(v, sg); }
+    __device__ void copy(unsigned char *ring, int v, unsigned n) const { filt_copy<8>((double *)ring + v, r64 + n); }
+    __device__ float val(const unsigned char *ring, int v, float s) const {
+        return s * dinv * scaled_f32(((const double *)ring)[v], sg);
+    }
     __device__ Own own(unsigned n) const { return r64[n]; }
     __device__ void put(unsigned n, float bd, Own v, float z, float y) {
         const float rv = scaled_f32(v, sg), wv = bd * y;
@@ -169,16 +189,21 @@ struct FiltIter {
     float al, be, dinv;
     const float *ro, *so, *wo;
     float *rn, *sn, *wn, *p, *d, sum[3];
-    struct Raw {
-        float r, w, s;
-    };
     struct Own {
         float r, w, s, p, d;
     };
     // beta = 0 (the first step): s and p may hold anything
     __device__ float snew(float w, float s) const { return be == 0.0f ? w : w + be * s; }
-    __device__ Raw load(unsigned n) const { return {ro[n], wo[n], so[n]}; }
-    __device__ float val(const Raw &v, float s) const { return s * dinv * (v.r - al * snew(v.w, v.s)); }
+    __device__ void copy(unsigned char *ring, int v, unsigned n) const {
+        float *q = (float *)ring + v;
+        filt_copy<4>(q, ro + n);
+        filt_copy<4>(q + FT_PLANE, wo + n);
+        filt_copy<4>(q + 2 * FT_PLANE, so + n);
+    }
+    __device__ float val(const unsigned char *ring, int v, float s) const {
+        const float *q = (const float *)ring + v;
+        return s * dinv * (q[0] - al * snew(q[FT_PLANE], q[2 * FT_PLANE]));
+    }
     __device__ Own own(unsigned n) const { return {ro[n], wo[n], so[n], p[n], d[n]}; }
     __device__ void put(unsigned n, float bd, const Own &o, float z, float y) {
         const float sv = snew(o.w, o.s), rv = o.r - al * sv, zold = dinv * o.r * (bd == 1.0f ? 1.0f : 1.0f / bd);
@@ -198,13 +223,14 @@ struct FiltResid {
     const double *uo, *b;
     const float *d;
     double is, *un, *r, sum;
-    struct Raw {
-        double u;
-        float d;
-    };
     using Own = double;
-    __device__ Raw load(unsigned n) const { return {uo[n], d[n]}; }
-    __device__ double val(const Raw &v, float) const { return fma(is, f32_to_f64(v.d), v.u); }
+    __device__ void copy(unsigned char *ring, int v, unsigned n) const {
+        filt_copy<8>((double *)ring + v, uo + n);
+        filt_copy<4>((float *)(ring + 8 * FT_PLANE) + v, d + n);
+    }
+    __device__ double val(const unsigned char *ring, int v, float) const {
+        return fma(is, f32_to_f64(((const float *)(ring + 8 * FT_PLANE))[v]), ((const double *)ring)[v]);
+    }
     __device__ Own own(unsigned n) const { return b[n]; }
     __device__ void put(unsigned n, float bd, Own bv, double v, double y) {
         un[n] = v;
@@ -224,7 +250,7 @@ struct FiltResid {
 //   gamma = r.z, delta = w.z -> beta, alpha
 // where the new r of the neighbours is formed while staging, so an iteration
 // is one pass and one grid barrier.  Filter and chain rule of three fields take
-// 2.9 ms at 192x96x96 and 0.39 ms at 48x24x24, against 13.7 and 1.49 ms of FP64 CG
+// 2.6 ms at 192x96x96 and 0.35 ms at 48x24x24, against 13.7 and 1.49 ms of FP64 CG
 // with three launches an iteration and 64 FP64 multiply-adds a node; the result
 // is 3.1e-11 instead of 4.5e-11 from the exact one at rtol 1e-10.
 __global__ void __launch_bounds__(FT_N, 3) k_filt_solve(const FiltArgs A) {
@@ -235,12 +261,11 @@ __global__ void __launch_bounds__(FT_N, 3) k_filt_solve(const FiltArgs A) {
         float gam, alpha, beta, goal;
         int done, idle;
     };
-    __shared__ __align__(16) double pl64[2 * FT_PLANE];
+    __shared__ __align__(16) FiltSmem sm;
     __shared__ double sred64[FT_N], stot64[FILT_RHS];
     __shared__ float sred[FILT_RHS][NV * FT_N / 32], stot[FILT_RHS * NV];
     __shared__ Rhs R[FILT_RHS];
     __shared__ int s_status;
-    float *pl32 = reinterpret_cast<float *>(pl64);
     const GridDesc g = A.g;
     const long long nn = g.nn(), nel = g.nel();
     const long long t0 = blockIdx.x * (long long)FT_N + threadIdx.x, ts = (long long)gridDim.x * FT_N;
@@ -310,7 +335,7 @@ __global__ void __launch_bounds__(FT_N, 3) k_filt_solve(const FiltArgs A) {
         for (int r = 0; r < A.nr; r++) {
             if (R[r].done) continue;
             FiltStart f{A.r[r], scale_split(1.0 / R[r].rms), dinv, A.r32[r][0], A.w32[r][0], A.d32[r], {}};
-            filt_apply<float>(A, A.Kf, pl32, f);
+            filt_apply<float>(A, A.Kf, sm, f);
             sums(r, f.sum);
         }
         if (!finish()) return;
@@ -336,7 +361,7 @@ __global__ void __launch_bounds__(FT_N, 3) k_filt_solve(const FiltArgs A) {
                 if (R[r].idle) continue;
                 FiltIter f{R[r].alpha, R[r].beta, dinv, A.r32[r][o], A.s32[r][o], A.w32[r][o],
                            A.r32[r][w], A.s32[r][w], A.w32[r][w], A.p32[r], A.d32[r], {}};
-                filt_apply<float>(A, A.Kf, pl32, f);
+                filt_apply<float>(A, A.Kf, sm, f);
                 sums(r, f.sum);
             }
             if (!finish()) return;
@@ -358,7 +383,7 @@ __global__ void __launch_bounds__(FT_N, 3) k_filt_solve(const FiltArgs A) {
                 continue;
             }
             FiltResid f{A.u[r][ub], A.b[r], A.d32[r], R[r].rms, A.u[r][ub ^ 1], A.r[r], 0.0};
-            filt_apply<double>(A, A.Kd, pl64, f);
+            filt_apply<double>(A, A.Kd, sm, f);
             sum64(r, f.sum);
         }
         if (!finish64()) return;
