@@ -31,6 +31,41 @@ inline long long &launch_counter() {
     return c;
 }
 inline void count_launch(long long n = 1) { launch_counter() += n; }
+
+// Dependent launches.  A step is a chain of kernels of 2 to 10 us on small grids,
+// each of which reads what the one before it wrote.  With the programmatic launch
+// attribute the next kernel is launched while the last CTAs of this one still run
+// (from the grid reduction on, where there is one) and waits on the device for
+// its completion and its writes.  Every kernel so launched waits first, so a
+// kernel's completion implies that of all before it.  What a predecessor wrote is
+// read by ordinary loads: no pointer of these kernels is __restrict__, which the
+// compiler would turn into read-only loads, not ordered by the wait.
+// Letting the next kernel in from this one's start was slower (FP64 solves of
+// 48x24x24 123 instead of 101 ms, 104 without): its CTAs fill the SMs in the order
+// in which these become free, and the load is uneven.
+// Up to this many nodes of a grid: 96x48x48 (233 thousand) takes 190.9 instead of
+// 193.6 ms, 192x96x96 (1.8 million) 215 instead of 211: the launch is short beside
+// kernels of 100 us, and early CTAs disturb the persistent ones.
+constexpr long long DEP_NODES = 400000;
+__device__ __forceinline__ void grid_dep_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <class... P, class... A>
+inline void launch_dep(long long nn, void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args) {
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    c.attrs = &at;
+    c.numAttrs = nn <= DEP_NODES ? 1 : 0;
+    cudaLaunchKernelEx(&c, k, static_cast<A &&>(args)...);
+}
+
 // ---------------------------------------------------------------------------
 // one level of the structured node/element grid
 // ---------------------------------------------------------------------------
@@ -436,6 +471,7 @@ __device__ __forceinline__ bool grid_reduce_blocks(double v[NV], const Partials<
 // `tot` holds the grid sums.
 template <int NT, int NV>
 __device__ __forceinline__ bool grid_reduce(double v[NV], const Partials<NV> &P, double tot[NV]) {
+    grid_dep_launch();
     __shared__ double sred[NV * (NT / 32)];
     block_reduce<NT, NV>(v, sred);
     return grid_reduce_blocks<NT, NV>(v, P, tot, sred);
@@ -443,6 +479,7 @@ __device__ __forceinline__ bool grid_reduce(double v[NV], const Partials<NV> &P,
 // the same from FP32 per-thread partials (block_reduce_f32)
 template <int NT, int NV>
 __device__ __forceinline__ bool grid_reduce(const float vf[NV], const Partials<NV> &P, double tot[NV]) {
+    grid_dep_launch();
     __shared__ double sred[NV * (NT / 32)];
     double v[NV];
     block_reduce_f32<NT, NV>(vf, v, sred);
@@ -530,6 +567,7 @@ __device__ __forceinline__ bool grid_reduce64_blocks(double v[NV], const Partial
 // finish); on that thread `tot` holds the grid sums.
 template <int NT, int NV>
 __device__ __forceinline__ bool grid_reduce64(double v[NV], const Partials<NV> &P, double tot[NV], int nt = NT) {
+    grid_dep_launch();
     __shared__ RedSmem<NT, NV> sred;
     block_reduce64<NT, NV>(v, sred, nt);
     return grid_reduce64_blocks<NV>(v, P, tot, nt);

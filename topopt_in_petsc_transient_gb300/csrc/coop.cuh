@@ -86,6 +86,7 @@ __device__ __forceinline__ void cta_sums(const float v[NV], float *sm /* NV * NT
 // reason scalar FP64 algebra belongs in one thread, not in all.)
 template <int NT, int NV>
 __device__ __forceinline__ void cta_sums(const double v[NV], double *sm /* NV * NT */, double *out, size_t stride) {
+    static_assert(NV <= NT / 32, "a warp per value");
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
     for (int i = 0; i < NV; i++) sm[i * NT + threadIdx.x] = v[i];

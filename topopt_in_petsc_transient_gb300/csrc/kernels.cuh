@@ -193,8 +193,9 @@ static __global__ void k_bounds_final(const unsigned long long *bits, double rat
 
 // first Chebyshev step from a zero initial guess: d = Dinv b / theta, x = d
 template <class T>
-static __global__ void k_cheb0(long long ndof, const T *__restrict__ b, const T *__restrict__ dinv, const double *coef,
+static __global__ void k_cheb0(long long ndof, const T *b, const T *dinv, const double *coef,
                                T *x, T *d) {
+    grid_dep_wait();
     const T c2 = (T)coef[1];
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < ndof; i += (long long)gridDim.x * blockDim.x) {
         T v = c2 * dinv[i] * b[i];
@@ -206,9 +207,10 @@ static __global__ void k_cheb0(long long ndof, const T *__restrict__ b, const T 
 // The fine-level first Chebyshev step of the mixed-precision FCG.  After a
 // residual replacement (S->rescale) the FP32 right-hand side is re-formed
 // here as r32 = sigma r from the scaled FP64 residual before the step uses it.
-static __global__ void k_cheb0_rescale(long long ndof, const double *__restrict__ r, float *b,
-                                       const float *__restrict__ dinv, const double *coef, float *x, float *d,
+static __global__ void k_cheb0_rescale(long long ndof, const double *r, float *b,
+                                       const float *dinv, const double *coef, float *x, float *d,
                                        const SolveScalars *S) {
+    grid_dep_wait();
     const float c2 = (float)coef[1];
     const bool rs = S->rescale != 0;
     const ScaleF64 sg = scale_split(S->sigma);
@@ -230,7 +232,8 @@ static __global__ void k_cheb0_rescale(long long ndof, const double *__restrict_
 // interpolation of DMCreateInterpolation, LinearElasticity.cc:2838-2842):
 // coarse node gathers fine nodes 2I-1..2I+1 with weights 1/2, 1, 1/2 per axis.
 template <class T>
-static __global__ void k_restrict(GridDesc gf, GridDesc gc, const uint8_t *__restrict__ fixc, const T *__restrict__ rf, T *bc) {
+static __global__ void k_restrict(GridDesc gf, GridDesc gc, const uint8_t *fixc, const T *rf, T *bc) {
+    grid_dep_wait();
     long long nn = gc.nn();
     for (long long N = blockIdx.x * (long long)blockDim.x + threadIdx.x; N < nn; N += (long long)gridDim.x * blockDim.x) {
         int I = (int)(N % gc.nx), J = (int)((N / gc.nx) % gc.ny), K = (int)(N / ((long long)gc.nx * gc.ny));
@@ -263,7 +266,8 @@ static __global__ void k_restrict(GridDesc gf, GridDesc gc, const uint8_t *__res
 
 // x_f += P x_c (trilinear), clamped DOFs untouched
 template <class T>
-static __global__ void k_prolong(GridDesc gf, GridDesc gc, const uint8_t *__restrict__ fixf, const T *__restrict__ xc, T *xf) {
+static __global__ void k_prolong(GridDesc gf, GridDesc gc, const uint8_t *fixf, const T *xc, T *xf) {
+    grid_dep_wait();
     long long nn = gf.nn();
     for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < nn; n += (long long)gridDim.x * blockDim.x) {
         int i = (int)(n % gf.nx), j = (int)((n / gf.nx) % gf.ny), k = (int)(n / ((long long)gf.nx * gf.ny));
@@ -287,7 +291,8 @@ static __global__ void k_prolong(GridDesc gf, GridDesc gc, const uint8_t *__rest
 
 // y = A x for the explicit coarse inverse (one warp per row)
 template <class T>
-static __global__ void k_gemv(int n, const T *__restrict__ A, const T *__restrict__ x, T *y) {
+static __global__ void k_gemv(int n, const T *A, const T *x, T *y) {
+    grid_dep_wait();
     int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (warp >= n) return;
     const T *row = A + (size_t)warp * n;
@@ -476,8 +481,9 @@ static __global__ void k_copy(long long n, const double *__restrict__ a, double 
 // flexible CG (Notay's FCG(1)): p_{k+1} = z_{k+1} - (z_{k+1}.q_k / p_k.q_k) p_k
 // ---------------------------------------------------------------------------
 template <class TZ>
-static __global__ void k_fcg_dot(long long ndof, const TZ *__restrict__ z, const double *__restrict__ r,
-                          const double *__restrict__ q, SolveScalars *S, Partials<2> part) {
+static __global__ void k_fcg_dot(long long ndof, const TZ *z, const double *r,
+                          const double *q, SolveScalars *S, Partials<2> part) {
+    grid_dep_wait();
     double v[2] = {0.0, 0.0};
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < ndof; i += (long long)gridDim.x * blockDim.x) {
         double zi = (double)z[i];
@@ -497,15 +503,17 @@ static __global__ void k_fcg_dot(long long ndof, const TZ *__restrict__ z, const
 }
 
 template <class TZ>
-static __global__ void k_fcg_p(long long ndof, const TZ *__restrict__ z, double *p, const SolveScalars *S) {
+static __global__ void k_fcg_p(long long ndof, const TZ *z, double *p, const SolveScalars *S) {
+    grid_dep_wait();
     double beta = S->beta;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < ndof; i += (long long)gridDim.x * blockDim.x)
         p[i] = (beta == 0.0) ? (double)z[i] : (double)z[i] + beta * p[i];
 }
 
-static __global__ void k_fcg_update(long long ndof, double *x, double *r, float *r32, const double *__restrict__ p,
-                             const double *__restrict__ q, SolveScalars *S, Partials<1> part,
+static __global__ void k_fcg_update(long long ndof, double *x, double *r, float *r32, const double *p,
+                             const double *q, SolveScalars *S, Partials<1> part,
                              cudaGraphConditionalHandle cond, int has_cond) {
+    grid_dep_wait();
     double alpha = S->alpha;
     double v[1] = {0.0};
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < ndof; i += (long long)gridDim.x * blockDim.x) {
@@ -536,15 +544,17 @@ static __global__ void k_fcg_update(long long ndof, double *x, double *r, float 
 
 // mixed-precision FCG pieces (FP32 vectors, FP64 scalars and iterate)
 // r32 = sigma * r after an FP64 residual (init or replacement)
-static __global__ void k_mfcg_scale(long long ndof, const double *__restrict__ r, float *r32, const SolveScalars *S) {
+static __global__ void k_mfcg_scale(long long ndof, const double *r, float *r32, const SolveScalars *S) {
+    grid_dep_wait();
     if (!S->rescale) return;
     const ScaleF64 sg = scale_split(S->sigma);
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < ndof; i += (long long)gridDim.x * blockDim.x)
         r32[i] = scaled_f32(r[i], sg);
 }
 
-static __global__ void k_mfcg_dot(long long ndof, const float *__restrict__ z, const float *__restrict__ r32,
-                                  const float *__restrict__ q32, SolveScalars *S, Partials<2> part) {
+static __global__ void k_mfcg_dot(long long ndof, const float *z, const float *r32,
+                                  const float *q32, SolveScalars *S, Partials<2> part) {
+    grid_dep_wait();
     float s0 = 0.0f, s1 = 0.0f;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < ndof; i += (long long)gridDim.x * blockDim.x) {
         float zi = z[i];
@@ -565,10 +575,11 @@ static __global__ void k_mfcg_dot(long long ndof, const float *__restrict__ z, c
 
 // p is double-buffered (PolPQ32 reads the previous p from pb[it & 1] and
 // writes the new one to pb[(it + 1) & 1])
-static __global__ void k_mfcg_update(long long ndof, double *__restrict__ x, float *__restrict__ r32,
-                                     const float *pb0, const float *pb1, const float *__restrict__ q, SolveScalars *S,
+static __global__ void k_mfcg_update(long long ndof, double *x, float *r32,
+                                     const float *pb0, const float *pb1, const float *q, SolveScalars *S,
                                      Partials<1> part) {
-    const float *__restrict__ p = ((S->it + 1) & 1) ? pb1 : pb0;
+    grid_dep_wait();
+    const float *p = ((S->it + 1) & 1) ? pb1 : pb0;
     // alpha in FP32 and in unscaled units, formed once by PolPQ32 (an FP64
     // division per thread would cost more FP64-pipe time than the x update)
     const float af = S->alpha32;
@@ -621,6 +632,7 @@ static __global__ void k_mfcg_update(long long ndof, double *__restrict__ x, flo
 // almost always a no-op (the solve zeroes x only for a zero right-hand side):
 // launched as one wave of grid-stride CTAs, so the check costs one wave
 static __global__ void k_fcg_zero_x(long long ndof, double *x, const SolveScalars *S) {
+    grid_dep_wait();
     if (!S->zero_x) return;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < ndof; i += (long long)gridDim.x * blockDim.x)
         x[i] = 0.0;
@@ -636,8 +648,9 @@ struct Newmark {
     df da[6];  // the same as double-float pairs (k_newmark_track)
 };
 
-static __global__ void k_newmark(long long ndof, const double *__restrict__ x, const StepCtx *st, const double *cp, double *Uh,
+static __global__ void k_newmark(long long ndof, const double *x, const StepCtx *st, const double *cp, double *Uh,
                           double *DUh, double *DDUh, Newmark nm) {
+    grid_dep_wait();
     int j = st->j;
     const double *u, *du, *ddu;
     if (j == 0) {
@@ -715,6 +728,7 @@ template <bool STD>
 static __global__ void __launch_bounds__(EW, 4) k_newmark_track(long long ndof, double *x, const StepCtx *st, const double *cp, double *Uh,
                                        double *DUh, double *DDUh, Newmark nm, double *b, double *r,
                                        const SolveScalars *S, double *AU, double *AV, double *AA, FwdPrep P) {
+    grid_dep_wait();
     const int j = st->j;
     const double *u, *du, *ddu;
     if (j == 0) {
@@ -776,9 +790,10 @@ struct RhsLoad {
     const double *sig, *sig2;  // per-step load signals (k_load_table)
     long long load2_dof;
 };
-static __global__ void __launch_bounds__(EW, 4) k_rhs_finish(long long ndof, const uint8_t *__restrict__ fixed, const double *__restrict__ y,
-                                    RhsLoad L, const StepCtx *st, double *__restrict__ b, double *__restrict__ r,
+static __global__ void __launch_bounds__(EW, 4) k_rhs_finish(long long ndof, const uint8_t *fixed, const double *y,
+                                    RhsLoad L, const StepCtx *st, double *b, double *r,
                                     SolveScalars *S, cudaGraphConditionalHandle cond, int has_cond, Partials<2> part) {
+    grid_dep_wait();
     const int t = st->tsc * st->block + st->j + 1;
     const double s = L.sig[t];
     double red[2] = {0.0, 0.0};
@@ -829,6 +844,7 @@ static __global__ void k_step_set(StepCtx *st, int block, int j) {
     st->j = j;
 }
 static __global__ void k_step_add(StepCtx *st, int delta) {
+    grid_dep_wait();
     st->j += delta;
     if (delta < 0) st->nadj += 1;
 }

@@ -176,8 +176,8 @@ __host__ inline int kx_lines_launch(const GridDesc &g, size_t elem, long long sl
 }
 
 template <class T, class R>
-__device__ __forceinline__ void kron_x_body(const GridDesc &g, int kx, R *r, const double *__restrict__ r64,
-                                            const SolveScalars *S, const T *__restrict__ ms, const KronBand<T> &B,
+__device__ __forceinline__ void kron_x_body(const GridDesc &g, int kx, R *r, const double *r64,
+                                            const SolveScalars *S, const T *ms, const KronBand<T> &B,
                                             T *out) {
     TOPO_DYNAMIC_SMEM(unsigned char, kron_smem);
     const int LP = kx_pitch(g.nx);
@@ -235,8 +235,9 @@ __device__ __forceinline__ void kron_x_body(const GridDesc &g, int kx, R *r, con
 
 template <class T, class R>
 static __global__ void __launch_bounds__(KRON_THREADS)
-    k_kron_x(GridDesc g, int kx, R *r, const double *__restrict__ r64, const SolveScalars *S, const T *__restrict__ ms,
+    k_kron_x(GridDesc g, int kx, R *r, const double *r64, const SolveScalars *S, const T *ms,
              KronBand<T> B, T *out) {
+    grid_dep_wait();
     kron_x_body<T, R>(g, kx, r, r64, S, ms, B, out);
 }
 // y pass (AXIS 1) and z pass (AXIS 2): a CTA stages a chunk of KW values of
@@ -258,8 +259,9 @@ __host__ inline size_t kron_yz_smem(const GridDesc &g, int axis, size_t elem, bo
 
 template <class T, class R, int AXIS, bool DOT>
 static __global__ void __launch_bounds__(KRON_THREADS, sizeof(T) == 4 ? 4 : 2)
-    k_kron_yz(GridDesc g, const R *__restrict__ r, const T *__restrict__ ms, KronBand<T> B, const T *__restrict__ in,
+    k_kron_yz(GridDesc g, const R *r, const T *ms, KronBand<T> B, const T *in,
               T *out, KronDot kd) {
+    grid_dep_wait();
     TOPO_DYNAMIC_SMEM(unsigned char, kron_smem);
     const int len = AXIS == 1 ? g.ny : g.nz;
     T *tile = reinterpret_cast<T *>(kron_smem);  // [len][KW]

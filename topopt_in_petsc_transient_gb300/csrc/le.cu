@@ -286,9 +286,9 @@ static void launch_march(const GridDesc &g, const ElemConst<double> &C, const Po
     const unsigned grid = (unsigned)((long long)d.ntx * d.nty * d.ncz);
     count_launch();
     if (Pol::HAS_K && C.cube)
-        k_march<Pol, true><<<grid, d.tx * d.ty, sm, s>>>(g, C, pol, d);
+        launch_dep(g.nn(), k_march<Pol, true>, grid, d.tx * d.ty, sm, s, g, C, pol, d);
     else
-        k_march<Pol, false><<<grid, d.tx * d.ty, sm, s>>>(g, C, pol, d);
+        launch_dep(g.nn(), k_march<Pol, false>, grid, d.tx * d.ty, sm, s, g, C, pol, d);
 }
 // FP32 and double-float: bricks.  FP32 kernels and kernels staged by asynchronous
 // copies are persistent: as many CTAs as are resident on the device at once
@@ -313,7 +313,7 @@ static void launch_tile(const GridDesc &g, const ElemConst<T> &C, const Pol &pol
         const bool timed = tile_class<T, Pol>() >= 0 && timer_begin(tile_class<T, Pol>(), g.nn(), s);
         count_launch();
         const int grid = (tile_persistent<T>() || tile_async<T, Pol>()) ? std::min(ntiles, resident) : ntiles;
-        k_tile<T, Pol><<<(unsigned)grid, TILE_THREADS, sm, s>>>(g, C, pol);
+        launch_dep(g.nn(), k_tile<T, Pol>, (unsigned)grid, TILE_THREADS, sm, s, g, C, pol);
         timer_end(timed, s);
     }
 }
@@ -1033,14 +1033,14 @@ static T *vcycle(TopoLE *le, int o, int l, const T *b, VFuse *fz = nullptr) {
         if constexpr (std::is_same<T, float>::value) {
             if (fuse) {
                 count_launch();
-                k_cheb0_rescale<<<ew_blocks(nd), EW, 0, s>>>(nd, fz->r64, const_cast<float *>(b), w.dinv, tab, x, w.d,
+                launch_dep(lv.g.nn(), k_cheb0_rescale, ew_blocks(nd), EW, 0, s, nd, fz->r64, const_cast<float *>(b), w.dinv, tab, x, w.d,
                                                              fz->S);
                 fz->scaled = true;
                 return;
             }
         }
         count_launch();
-        k_cheb0<T><<<ew_blocks(nd), EW, 0, s>>>(nd, b, w.dinv, tab, x, w.d);
+        launch_dep(lv.g.nn(), k_cheb0<T>, ew_blocks(nd), EW, 0, s, nd, b, w.dinv, tab, x, w.d);
     };
     // smoothing step k (one operator application); `last`: this level's
     // final step, whose output is the V-cycle result at the fine level
@@ -1073,7 +1073,7 @@ static T *vcycle(TopoLE *le, int o, int l, const T *b, VFuse *fz = nullptr) {
         if (le->coarse_dense) {
             int n = le->ncoarse;
             count_launch();
-            k_gemv<T><<<(n * 32 + 255) / 256, 256, 0, s>>>(n, ainv<T>(le, o), b, w.xa);
+            launch_dep(lv.g.nn(), k_gemv<T>, (n * 32 + 255) / 256, 256, 0, s, n, ainv<T>(le, o), b, w.xa);
             return w.xa;
         }
         // iterative coarse solve: Chebyshev-Jacobi polynomial from zero
@@ -1089,10 +1089,10 @@ static T *vcycle(TopoLE *le, int o, int l, const T *b, VFuse *fz = nullptr) {
     Level &lc = le->L[l + 1];
     VW<T> wc = vw<T>(le, o, l + 1);
     count_launch();
-    k_restrict<T><<<ew_blocks(lc.g.nn()), EW, 0, s>>>(lv.g, lc.g, lc.fixed, w.r, wc.b);
+    launch_dep(lv.g.nn(), k_restrict<T>, ew_blocks(lc.g.nn()), EW, 0, s, lv.g, lc.g, lc.fixed, w.r, wc.b);
     T *xc = vcycle<T>(le, o, l + 1, wc.b);
     count_launch();
-    k_prolong<T><<<ew_blocks(lv.g.nn()), EW, 0, s>>>(lv.g, lc.g, lv.fixed, xc, x);
+    launch_dep(lv.g.nn(), k_prolong<T>, ew_blocks(lv.g.nn()), EW, 0, s, lv.g, lc.g, lv.fixed, xc, x);
     for (int k = 0; k < nu; k++) step(lohi, k, k == nu - 1);
     return x;
 }
@@ -1123,22 +1123,19 @@ static T *kron_apply(TopoLE *le, int o, T *r, VFuse *fz = nullptr) {
     bool t;
     count_launch();
     t = timer_begin(TOPO_KT_KRON, g.nn(), s);
-    k_kron_x<T, T><<<(unsigned)((nlines + kx - 1) / kx), KRON_THREADS, smx, s>>>(
-        g, kx, r, mixed ? fz->r64 : nullptr, mixed ? fz->S : nullptr, sc, B, w.xa);
+    launch_dep(g.nn(), k_kron_x<T, T>, (unsigned)((nlines + kx - 1) / kx), KRON_THREADS, smx, s, g, kx, r, mixed ? fz->r64 : nullptr, mixed ? fz->S : nullptr, sc, B, w.xa);
     timer_end(t, s);
     count_launch();
     t = timer_begin(TOPO_KT_KRON, g.nn(), s);
-    k_kron_yz<T, T, 1, false><<<kron_yz_blocks(g, 1), KRON_THREADS, smy, s>>>(g, r, sc, B, w.xa, w.xb, KronDot{});
+    launch_dep(g.nn(), k_kron_yz<T, T, 1, false>, kron_yz_blocks(g, 1), KRON_THREADS, smy, s, g, r, sc, B, w.xa, w.xb, KronDot{});
     timer_end(t, s);
     count_launch();
     t = timer_begin(TOPO_KT_KRON, g.nn(), s);
     if (mixed && le->p.mass_precond_smooth <= 0) {
-        k_kron_yz<T, T, 2, true><<<kron_yz_blocks(g, 2), KRON_THREADS, kron_yz_smem(g, 2, sizeof(T), true), s>>>(
-            g, r, sc, B, w.xb, w.xa, KronDot{fz->q32, fz->S, fz->part});
+        launch_dep(g.nn(), k_kron_yz<T, T, 2, true>, kron_yz_blocks(g, 2), KRON_THREADS, kron_yz_smem(g, 2, sizeof(T), true), s, g, r, sc, B, w.xb, w.xa, KronDot{fz->q32, fz->S, fz->part});
         fz->dotted = true;
     } else {
-        k_kron_yz<T, T, 2, false><<<kron_yz_blocks(g, 2), KRON_THREADS, kron_yz_smem(g, 2, sizeof(T)), s>>>(
-            g, r, sc, B, w.xb, w.xa, KronDot{});
+        launch_dep(g.nn(), k_kron_yz<T, T, 2, false>, kron_yz_blocks(g, 2), KRON_THREADS, kron_yz_smem(g, 2, sizeof(T)), s, g, r, sc, B, w.xb, w.xa, KronDot{});
     }
     timer_end(t, s);
     if (mixed) fz->scaled = true;
@@ -1184,6 +1181,7 @@ static T *kron_smooth(TopoLE *le, int o, const T *r, T *z0, VFuse *fz) {
 // flexible CG:  (N A N + I - N) x = b for operator o; sx holds the initial guess
 // ---------------------------------------------------------------------------
 __global__ void k_solve_prime(SolveScalars *S, double tol2, int maxit, double tau2, int kmax, double ndof) {
+    grid_dep_wait();
     S->ndof = ndof;
     S->tol2 = tol2;
     S->maxit = maxit;
@@ -1194,6 +1192,7 @@ __global__ void k_solve_prime(SolveScalars *S, double tol2, int maxit, double ta
     S->it = 0;
 }
 __global__ void k_solve_check(const SolveScalars *S, int *err) {
+    grid_dep_wait();
     if (S->status != 0 && *err == 0) *err = S->status;
 }
 
@@ -1225,7 +1224,7 @@ static void solve_init(TopoLE *le, int o, const double *b, cudaGraphConditionalH
         count_launch();
         // AL mode: x0 is accepted only on a true residual, which keeps
         // A lambda = b - r exact for the stored lambda
-        k_init_pointwise<<<red_blocks(le->ndof), EW, 0, le->stream>>>(le->ndof, b, le->sq, le->sr, le->S,
+        launch_dep(le->nn, k_init_pointwise, red_blocks(le->ndof), EW, 0, le->stream, le->ndof, b, le->sq, le->sr, le->S,
                                                                        mixed_fcg(le) ? 1 : 0, al_mode(le) ? 0 : 1,
                                                                        cond, has_cond, P2(le));
         return;
@@ -1261,19 +1260,19 @@ static void solve_iteration(TopoLE *le, int o, cudaGraphConditionalHandle cond, 
         } else {
             if (le->ops[o].depth == 1 && le->nlev == 1 && le->coarse_dense) {
                 count_launch();  // the dense coarse solve has no smoothing step to carry the rescaling
-                k_mfcg_scale<<<red_blocks(nd), EW, 0, s>>>(nd, le->sr, le->sr32, le->S);
+                launch_dep(le->nn, k_mfcg_scale, red_blocks(nd), EW, 0, s, nd, le->sr, le->sr32, le->S);
             }
             z = vcycle<float>(le, o, 0, le->sr32, &fz);
         }
         if (!fz.dotted) {
             count_launch();
-            k_mfcg_dot<<<red_blocks(nd), EW, 0, s>>>(nd, z, le->sr32, le->sq32, le->S, P2(le));
+            launch_dep(le->nn, k_mfcg_dot, red_blocks(nd), EW, 0, s, nd, z, le->sr32, le->sq32, le->S, P2(le));
         }
         Weights<float> wf{op.sK != 0.0 ? l0.kff : nullptr, l0.mff, nullptr, (float)op.sK, (float)op.sM};
         PolPQ32 pq32{l0.fixed, wf, z, {le->sp32, le->sp32b}, le->sq32, le->S, P1(le)};
         launch_tile<float>(l0.g, l0.Cf, pq32, s);
         count_launch();
-        k_mfcg_update<<<red_blocks(nd), EW, 0, s>>>(nd, le->sx, le->sr32, le->sp32, le->sp32b, le->sq32, le->S,
+        launch_dep(le->nn, k_mfcg_update, red_blocks(nd), EW, 0, s, nd, le->sx, le->sr32, le->sp32, le->sp32b, le->sq32, le->S,
                                                     P1(le));
         Weights<df> wd = fine_weights<df>(le, op.sK != 0.0, true, nullptr, op.sK, op.sM);
         PolReplace<df> rp{l0.fixed, wd, le->sx, cur_b(le), le->sr, le->S, cond, has_cond, P1(le)};
@@ -1283,22 +1282,22 @@ static void solve_iteration(TopoLE *le, int o, cudaGraphConditionalHandle cond, 
         double *z = op.kron ? kron_smooth<double>(le, o, le->sr, kron_apply<double>(le, o, le->sr), nullptr)
                             : vcycle<double>(le, o, 0, le->sr);
         count_launch();
-        k_fcg_dot<double><<<red_blocks(nd), EW, 0, s>>>(nd, z, le->sr, le->sq, le->S, P2(le));
+        launch_dep(le->nn, k_fcg_dot<double>, red_blocks(nd), EW, 0, s, nd, z, le->sr, le->sq, le->S, P2(le));
         count_launch();
-        k_fcg_p<double><<<nb, EW, 0, s>>>(nd, z, le->sp, le->S);
+        launch_dep(le->nn, k_fcg_p<double>, nb, EW, 0, s, nd, z, le->sp, le->S);
     }
     Weights<double> wt{op.sK != 0.0 ? l0.kfd : nullptr, l0.mfd, nullptr, op.sK, op.sM};
     PolPQ<double> pq{l0.fixed, wt, le->sp, le->sq, le->S, P1(le)};
     launch_tile<double>(l0.g, l0.Cd, pq, s);
     count_launch();
-    k_fcg_update<<<red_blocks(nd), EW, 0, s>>>(nd, le->sx, le->sr, mixed_fcg(le) ? le->sr32 : nullptr, le->sp, le->sq, le->S,
+    launch_dep(le->nn, k_fcg_update, red_blocks(nd), EW, 0, s, nd, le->sx, le->sr, mixed_fcg(le) ? le->sr32 : nullptr, le->sp, le->sq, le->S,
                                    P1(le), cond, has_cond);
 }
 
 // direct launches, host checks convergence after every iteration
 static int solve_direct(TopoLE *le, int o, const double *b) {
     count_launch();
-    k_solve_prime<<<1, 1, 0, le->stream>>>(le->S, le->p.rtol * le->p.rtol, le->p.maxit,
+    launch_dep(le->nn, k_solve_prime, 1, 1, 0, le->stream, le->S, le->p.rtol * le->p.rtol, le->p.maxit,
                                               le->p.inner_tol * le->p.inner_tol, le->p.inner_maxit,
                                               (double)le->ndof);
     solve_init(le, o, b, 0, 0);
@@ -1311,9 +1310,9 @@ static int solve_direct(TopoLE *le, int o, const double *b) {
         le->direct_iters++;
     }
     count_launch();
-    k_fcg_zero_x<<<red_blocks(le->ndof), EW, 0, le->stream>>>(le->ndof, le->sx, le->S);
+    launch_dep(le->nn, k_fcg_zero_x, red_blocks(le->ndof), EW, 0, le->stream, le->ndof, le->sx, le->S);
     count_launch();
-    k_solve_check<<<1, 1, 0, le->stream>>>(le->S, le->err);
+    launch_dep(le->nn, k_solve_check, 1, 1, 0, le->stream, le->S, le->err);
     le->nsolves++;
     if (!le->ops[o].kron) le->mg_solves++;
     CK(cudaGetLastError());
@@ -1325,7 +1324,7 @@ static int solve_direct(TopoLE *le, int o, const double *b) {
 static int solve_captured(TopoLE *le, int o, const double *b) {
     cudaStream_t s = le->stream;
     count_launch();
-    k_solve_prime<<<1, 1, 0, s>>>(le->S, le->p.rtol * le->p.rtol, le->p.maxit, le->p.inner_tol * le->p.inner_tol,
+    launch_dep(le->nn, k_solve_prime, 1, 1, 0, s, le->S, le->p.rtol * le->p.rtol, le->p.maxit, le->p.inner_tol * le->p.inner_tol,
                                   le->p.inner_maxit, (double)le->ndof);
     cudaStreamCaptureStatus cs;
     cudaGraph_t graph;
@@ -1358,9 +1357,9 @@ static int solve_captured(TopoLE *le, int o, const double *b) {
     cudaStreamDestroy(bs);
     CK(e1);
     count_launch();
-    k_fcg_zero_x<<<red_blocks(le->ndof), EW, 0, s>>>(le->ndof, le->sx, le->S);
+    launch_dep(le->nn, k_fcg_zero_x, red_blocks(le->ndof), EW, 0, s, le->ndof, le->sx, le->S);
     count_launch();
-    k_solve_check<<<1, 1, 0, s>>>(le->S, le->err);
+    launch_dep(le->nn, k_solve_check, 1, 1, 0, s, le->S, le->err);
     return TOPO_OK;
 }
 
@@ -1466,7 +1465,7 @@ static void fwd_rhs_init(TopoLE *le, cudaGraphConditionalHandle cond, int has_co
     product_t<df, true, false>(le, le->KSt, le->sq, nullptr, 1.0, 0.0);
     RhsLoad L{le->rhs0, le->sigtab, le->sigtab + le->Ts, p.load2_node >= 0 ? 3LL * p.load2_node + 2 : -1};
     count_launch();
-    k_rhs_finish<<<red_blocks(le->ndof), EW, 0, le->stream>>>(le->ndof, le->L[0].fixed, le->sq, L, le->st, le->sb,
+    launch_dep(le->nn, k_rhs_finish, red_blocks(le->ndof), EW, 0, le->stream, le->ndof, le->L[0].fixed, le->sq, L, le->st, le->sb,
                                                                le->sr, le->S, cond, has_cond, P2(le));
 }
 
@@ -1527,18 +1526,18 @@ static int fwd_step(TopoLE *le, bool capturing) {
     for (int i = 0; i < 6; i++) nm.da[i] = f64_to_df(nm.a[i]);
     count_launch();
     if (track && le->a[0] == -1.0 && le->a[1] == 0.0)
-        k_newmark_track<true><<<ew_blocks(le->ndof), EW, 0, s>>>(le->ndof, le->sx, le->st, le->cp, le->Uh, le->DUh,
+        launch_dep(le->nn, k_newmark_track<true>, ew_blocks(le->ndof), EW, 0, s, le->ndof, le->sx, le->st, le->cp, le->Uh, le->DUh,
                                                                  le->DDUh, nm, le->sb, le->sr, le->S, le->AUt,
                                                                  le->AVt, le->AAt, fwd_prep_args(le));
     else if (track)
-        k_newmark_track<false><<<ew_blocks(le->ndof), EW, 0, s>>>(le->ndof, le->sx, le->st, le->cp, le->Uh,
+        launch_dep(le->nn, k_newmark_track<false>, ew_blocks(le->ndof), EW, 0, s, le->ndof, le->sx, le->st, le->cp, le->Uh,
                                                                   le->DUh, le->DDUh, nm, le->sb, le->sr, le->S,
                                                                   le->AUt, le->AVt, le->AAt, fwd_prep_args(le));
     else
-        k_newmark<<<ew_blocks(le->ndof), EW, 0, s>>>(le->ndof, le->sx, le->st, le->cp, le->Uh, le->DUh, le->DDUh,
+        launch_dep(le->nn, k_newmark, ew_blocks(le->ndof), EW, 0, s, le->ndof, le->sx, le->st, le->cp, le->Uh, le->DUh, le->DDUh,
                                                      nm);
     count_launch();
-    k_step_add<<<1, 1, 0, s>>>(le->st, +1);
+    launch_dep(le->nn, k_step_add, 1, 1, 0, s, le->st, +1);
     return TOPO_OK;
 }
 
@@ -1726,9 +1725,9 @@ template <int OBJ>
 static void launch_sens_obj(TopoLE *le, const SensArgs &S) {
     count_launch();
     if (sens_in_fp32(le))
-        k_sens<OBJ, float><<<red_blocks(le->nel), EW, 0, le->stream>>>(S, le->L[0].Cf);
+        launch_dep(le->nn, k_sens<OBJ, float>, red_blocks(le->nel), EW, 0, le->stream, S, le->L[0].Cf);
     else
-        k_sens<OBJ, double><<<red_blocks(le->nel), EW, 0, le->stream>>>(S, le->L[0].Cd);
+        launch_dep(le->nn, k_sens<OBJ, double>, red_blocks(le->nel), EW, 0, le->stream, S, le->L[0].Cd);
 }
 static void launch_sens(TopoLE *le, int t0mode) {
     SensArgs S = sens_args(le, t0mode);
@@ -1745,7 +1744,7 @@ static void launch_sens(TopoLE *le, int t0mode) {
         S.wMd = le->sw64 + nd;
     }
     count_launch();
-    k_sens_nodal<<<ew_blocks(nd), EW, 0, le->stream>>>(S);
+    launch_dep(le->nn, k_sens_nodal, ew_blocks(nd), EW, 0, le->stream, S);
     switch (le->p.objective) {
     case 0: launch_sens_obj<0>(le, S); break;
     case 1: launch_sens_obj<1>(le, S); break;
@@ -1771,9 +1770,9 @@ static void adj_kl(TopoLE *le) {
 // the mixed path forms the adjoint right-hand side in double-float arithmetic
 static void launch_adj_combine(TopoLE *le, const AdjCombine &A) {
     if (le->p.mixed)
-        k_adj_combine<df><<<ew_blocks(le->ndof), EW, 0, le->stream>>>(A);
+        launch_dep(le->nn, k_adj_combine<df>, ew_blocks(le->ndof), EW, 0, le->stream, A);
     else
-        k_adj_combine<double><<<ew_blocks(le->ndof), EW, 0, le->stream>>>(A);
+        launch_dep(le->nn, k_adj_combine<double>, ew_blocks(le->ndof), EW, 0, le->stream, A);
 }
 
 static int adj_step(TopoLE *le, bool capturing) {
@@ -1795,7 +1794,7 @@ static int adj_step(TopoLE *le, bool capturing) {
                                                       KMHist{le->KL, le->ML, le->KLh1, le->MLh1, le->KLh2, le->MLh2,
                                                              al_mode(le) ? le->sb : nullptr, le->sr, le->S});
     count_launch();
-    k_step_add<<<1, 1, 0, s>>>(le->st, -1);
+    launch_dep(le->nn, k_step_add, 1, 1, 0, s, le->st, -1);
     return TOPO_OK;
 }
 

@@ -74,6 +74,7 @@ __device__ __forceinline__ void march_face(const double *lay, int s, int row, do
 template <class Pol, bool CUBE>
 __global__ void __launch_bounds__(MARCH_THREADS, Pol::M_IN == 1 ? 2 : 1)
     k_march(const GridDesc g, const ElemConst<double> C, const Pol pol, const MarchDims D) {
+    grid_dep_wait();
     TOPO_DYNAMIC_SMEM(double, lay0);
     constexpr int NIN = Pol::M_IN, NSRC = Pol::M_SRC;
     const int tid = threadIdx.x, NT = D.tx * D.ty;

@@ -65,6 +65,7 @@ __device__ __forceinline__ df adj_coef<df>(double, const df &f) {
 // DOF otherwise, which GB300 runs at two per clock and SM).
 template <class R>
 static __global__ void k_adj_combine(AdjCombine A) {
+    grid_dep_wait();
     long long nn = A.ndof / 3;
     const double *u, *du, *ddu;
     if (A.t0mode) {
@@ -253,9 +254,10 @@ static __global__ void k_adj_advance(long long ndof, const double *__restrict__ 
 // FCG initial residual from a precomputed (N A N + I - N) x0:
 // r = b - ax0, reductions b.b and r.r, then the same solver-state set-up as
 // the operator-pass initial residual (PolInitResid)
-static __global__ void k_init_pointwise(long long ndof, const double *__restrict__ b, const double *__restrict__ ax0,
+static __global__ void k_init_pointwise(long long ndof, const double *b, const double *ax0,
                                         double *r, SolveScalars *S, int has_r32, int accept_x0,
                                         cudaGraphConditionalHandle cond, int has_cond, Partials<2> part) {
+    grid_dep_wait();
     double red[2] = {0.0, 0.0};
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < ndof; i += (long long)gridDim.x * blockDim.x) {
         const double bv = b[i], rv = bv - ax0[i];
@@ -361,6 +363,7 @@ __host__ __device__ __forceinline__ int comb3_nz(const double c[3]) {
 // part): no FP64 instruction, where the FP64 form was bound by GB300's FP64
 // rate.
 static __global__ void k_sens_nodal(const SensArgs A) {
+    grid_dep_wait();
     const long long ndof = 3 * A.g.nn();
     const double *u, *du, *ddu, *up, *dup, *ddup;
     sens_states(A, ndof, u, du, ddu, up, dup, ddup);
@@ -444,6 +447,7 @@ __device__ __forceinline__ const float *sens_src(const double *, const float *f,
 
 template <int OBJ, class T>
 static __global__ void __launch_bounds__(EW) k_sens(const SensArgs A, const ElemConst<T> C) {
+    grid_dep_wait();
     const GridDesc g = A.g;
     const long long nel = g.nel(), ndof = 3 * g.nn();
     const double *u, *du, *ddu, *up, *dup, *ddup;

@@ -393,6 +393,7 @@ __device__ __forceinline__ void tile_run_async(const GridDesc &g, const ElemCons
 
 template <class T, class Pol>
 __global__ void __launch_bounds__(TILE_THREADS, sizeof(T) == 4 ? 2 : 1) k_tile(const GridDesc g, const ElemConst<T> C, const Pol pol) {
+    grid_dep_wait();
     TOPO_DYNAMIC_SMEM(unsigned char, smem_raw);
     if (pol_skip(pol, 0)) return;
     static_assert(TILE_STAGED <= 2 * TILE_THREADS, "staging assumes two passes");
