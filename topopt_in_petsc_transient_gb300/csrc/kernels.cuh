@@ -480,7 +480,8 @@ static __global__ void k_copy(long long n, const double *__restrict__ a, double 
 // ---------------------------------------------------------------------------
 // flexible CG (Notay's FCG(1)): p_{k+1} = z_{k+1} - (z_{k+1}.q_k / p_k.q_k) p_k
 // ---------------------------------------------------------------------------
-template <class TZ>
+// EXACT: sums in grid_reduce's order (launch_solve_tile)
+template <class TZ, bool EXACT>
 static __global__ void k_fcg_dot(long long ndof, const TZ *z, const double *r,
                           const double *q, SolveScalars *S, Partials<2> part) {
     grid_dep_wait();
@@ -491,7 +492,7 @@ static __global__ void k_fcg_dot(long long ndof, const TZ *z, const double *r,
         v[1] += zi * q[i];
     }
     double tot[2];
-    if (grid_reduce64<EW, 2>(v, part, tot)) {
+    if (EXACT ? grid_reduce<EW, 2>(v, part, tot) : grid_reduce64<EW, 2>(v, part, tot)) {
         S->rho = tot[0];
         S->gam = tot[1];
         S->beta = (S->it == 0) ? 0.0 : -tot[1] / S->pq;
@@ -510,6 +511,7 @@ static __global__ void k_fcg_p(long long ndof, const TZ *z, double *p, const Sol
         p[i] = (beta == 0.0) ? (double)z[i] : (double)z[i] + beta * p[i];
 }
 
+template <bool EXACT>
 static __global__ void k_fcg_update(long long ndof, double *x, double *r, float *r32, const double *p,
                              const double *q, SolveScalars *S, Partials<1> part,
                              cudaGraphConditionalHandle cond, int has_cond) {
@@ -524,7 +526,7 @@ static __global__ void k_fcg_update(long long ndof, double *x, double *r, float 
         v[0] += rv * rv;
     }
     double tot[1];
-    if (grid_reduce64<EW, 1>(v, part, tot)) {
+    if (EXACT ? grid_reduce<EW, 1>(v, part, tot) : grid_reduce64<EW, 1>(v, part, tot)) {
         S->rr = tot[0];
         S->it += 1;
         S->total_it += 1;

@@ -295,27 +295,41 @@ static void launch_march(const GridDesc &g, const ElemConst<double> &C, const Po
 // (occupancy of this instantiation x SM count), capped by the brick count; the
 // others launch one CTA per brick
 template <class T, class Pol>
-static void launch_tile(const GridDesc &g, const ElemConst<T> &C, const Pol &pol, cudaStream_t s) {
-    if constexpr (std::is_same<T, double>::value) {
-        launch_march(g, C, pol, s);
-    } else {
-        static int resident_dev[MAX_DEVICES] = {};
-        int &resident = resident_dev[device_slot()];
-        const size_t sm = TileSmem<T, Pol>::bytes;
-        if (!resident) {
-            cudaFuncSetAttribute(k_tile<T, Pol>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-            int per_sm = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tile<T, Pol>, TILE_THREADS, sm);
-            resident = std::max(1, per_sm) * sm_count();
-        }
-        int ntx, nty;
-        const int ntiles = tile_count(g, ntx, nty);
-        const bool timed = tile_class<T, Pol>() >= 0 && timer_begin(tile_class<T, Pol>(), g.nn(), s);
-        count_launch();
-        const int grid = (tile_persistent<T>() || tile_async<T, Pol>()) ? std::min(ntiles, resident) : ntiles;
-        launch_dep(g.nn(), k_tile<T, Pol>, (unsigned)grid, TILE_THREADS, sm, s, g, C, pol);
-        timer_end(timed, s);
+static void launch_brick(const GridDesc &g, const ElemConst<T> &C, const Pol &pol, cudaStream_t s) {
+    static int resident_dev[MAX_DEVICES] = {};
+    int &resident = resident_dev[device_slot()];
+    const size_t sm = TileSmem<T, Pol>::bytes;
+    if (!resident) {
+        cudaFuncSetAttribute(k_tile<T, Pol>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        int per_sm = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tile<T, Pol>, TILE_THREADS, sm);
+        resident = std::max(1, per_sm) * sm_count();
     }
+    int ntx, nty;
+    const int ntiles = tile_count(g, ntx, nty);
+    const bool timed = tile_class<T, Pol>() >= 0 && timer_begin(tile_class<T, Pol>(), g.nn(), s);
+    count_launch();
+    const int grid = (tile_persistent<T>() || tile_async<T, Pol>()) ? std::min(ntiles, resident) : ntiles;
+    launch_dep(g.nn(), k_tile<T, Pol>, (unsigned)grid, TILE_THREADS, sm, s, g, C, pol);
+    timer_end(timed, s);
+}
+template <class T, class Pol>
+static void launch_tile(const GridDesc &g, const ElemConst<T> &C, const Pol &pol, cudaStream_t s) {
+    if constexpr (std::is_same<T, double>::value)
+        launch_march(g, C, pol, s);
+    else
+        launch_brick<T>(g, C, pol, s);
+}
+// The operator of a solve.  FP64 solves whose result is rounded to FP32 (basis
+// vectors stored in FP32) keep the brick's order of sums: a change in the last
+// bits of a vector moves an entry across a rounding boundary in one set of
+// inputs out of five, and with it the sensitivities by 1.4e-9.
+template <class T, class Pol>
+static void launch_solve_tile(bool bricks, const GridDesc &g, const ElemConst<T> &C, const Pol &pol, cudaStream_t s) {
+    if (bricks)
+        launch_brick<T>(g, C, pol, s);
+    else
+        launch_tile<T>(g, C, pol, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -1017,6 +1031,8 @@ struct VFuse {
     bool scaled = false, dotted = false;
 };
 
+// sums in the order of the brick kernels and grid_reduce (launch_solve_tile)
+static bool brick_order(const TopoLE *le) { return le->fp64_solves && le->basis32; }
 template <class T>
 static T *vcycle(TopoLE *le, int o, int l, const T *b, VFuse *fz = nullptr) {
     cudaStream_t s = le->stream;
@@ -1056,7 +1072,7 @@ static T *vcycle(TopoLE *le, int o, int l, const T *b, VFuse *fz = nullptr) {
         }
         if (!done) {
             PolCheb<T> pc{lv.fixed, wt, x, b, w.dinv, xo, w.d, tab, k, {}};
-            launch_tile<T>(lv.g, *w.C, pc, s);
+            launch_solve_tile<T>(brick_order(le), lv.g, *w.C, pc, s);
         }
         T *t = x;
         x = xo;
@@ -1085,7 +1101,7 @@ static T *vcycle(TopoLE *le, int o, int l, const T *b, VFuse *fz = nullptr) {
     first(lohi);
     for (int k = 1; k < nu; k++) step(lohi, k, false);
     PolResid<T> pr{lv.fixed, wt, x, b, w.r, {}};
-    launch_tile<T>(lv.g, *w.C, pr, s);
+    launch_solve_tile<T>(brick_order(le), lv.g, *w.C, pr, s);
     Level &lc = le->L[l + 1];
     VW<T> wc = vw<T>(le, o, l + 1);
     count_launch();
@@ -1168,7 +1184,7 @@ static T *kron_smooth(TopoLE *le, int o, const T *r, T *z0, VFuse *fz) {
         }
         if (!done) {
             PolCheb<T> pc{l0.fixed, wt, x, r, w.dinv, xo, w.d, tab, k, {}};
-            launch_tile<T>(l0.g, *w.C, pc, s);
+            launch_solve_tile<T>(brick_order(le), l0.g, *w.C, pc, s);
         }
         T *t = x;
         x = xo;
@@ -1209,7 +1225,7 @@ static void solve_init_t(TopoLE *le, int o, const double *b, cudaGraphConditiona
     Operator &op = le->ops[o];
     Weights<A> wt = fine_weights<A>(le, op.sK != 0.0, true, nullptr, op.sK, op.sM);
     PolInitResid<A> pi{l0.fixed, wt, le->sx, b, le->sr, mixed_fcg(le) ? le->sr32 : nullptr, le->S, cond, has_cond, P2(le)};
-    launch_tile<A>(l0.g, fine_const<A>(le), pi, le->stream);
+    launch_solve_tile<A>(brick_order(le), l0.g, fine_const<A>(le), pi, le->stream);
 }
 static void fwd_rhs_init(TopoLE *le, cudaGraphConditionalHandle cond, int has_cond);
 static void solve_init(TopoLE *le, int o, const double *b, cudaGraphConditionalHandle cond, int has_cond) {
@@ -1282,15 +1298,15 @@ static void solve_iteration(TopoLE *le, int o, cudaGraphConditionalHandle cond, 
         double *z = op.kron ? kron_smooth<double>(le, o, le->sr, kron_apply<double>(le, o, le->sr), nullptr)
                             : vcycle<double>(le, o, 0, le->sr);
         count_launch();
-        launch_dep(le->nn, k_fcg_dot<double>, red_blocks(nd), EW, 0, s, nd, z, le->sr, le->sq, le->S, P2(le));
+        launch_dep(le->nn, brick_order(le) ? k_fcg_dot<double, true> : k_fcg_dot<double, false>, red_blocks(nd), EW, 0, s, nd, z, le->sr, le->sq, le->S, P2(le));
         count_launch();
         launch_dep(le->nn, k_fcg_p<double>, nb, EW, 0, s, nd, z, le->sp, le->S);
     }
     Weights<double> wt{op.sK != 0.0 ? l0.kfd : nullptr, l0.mfd, nullptr, op.sK, op.sM};
     PolPQ<double> pq{l0.fixed, wt, le->sp, le->sq, le->S, P1(le)};
-    launch_tile<double>(l0.g, l0.Cd, pq, s);
+    launch_solve_tile<double>(brick_order(le), l0.g, l0.Cd, pq, s);
     count_launch();
-    launch_dep(le->nn, k_fcg_update, red_blocks(nd), EW, 0, s, nd, le->sx, le->sr, mixed_fcg(le) ? le->sr32 : nullptr, le->sp, le->sq, le->S,
+    launch_dep(le->nn, brick_order(le) ? k_fcg_update<true> : k_fcg_update<false>, red_blocks(nd), EW, 0, s, nd, le->sx, le->sr, mixed_fcg(le) ? le->sr32 : nullptr, le->sp, le->sq, le->S,
                                    P1(le), cond, has_cond);
 }
 
@@ -1409,7 +1425,7 @@ static void fwd_rhs(TopoLE *le) {
     pr.st = le->st;
     pr.b = le->sb;
     pr.x0 = le->sx;
-    launch_tile<double>(l0.g, l0.Cd, pr, le->stream);
+    launch_march(l0.g, l0.Cd, pr, le->stream);
 }
 
 // coefficients of the next-step preparation (k_newmark_track, k_fwd_prep)
