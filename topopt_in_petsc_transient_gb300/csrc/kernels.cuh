@@ -193,8 +193,7 @@ static __global__ void k_bounds_final(const unsigned long long *bits, double rat
 
 // first Chebyshev step from a zero initial guess: d = Dinv b / theta, x = d
 template <class T>
-static __global__ void k_cheb0(long long ndof, const T *b, const T *dinv, const double *coef,
-                               T *x, T *d) {
+static __global__ void k_cheb0(long long ndof, const T *b, const T *dinv, const double *coef, T *x, T *d) {
     grid_dep_wait();
     const T c2 = (T)coef[1];
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < ndof; i += (long long)gridDim.x * blockDim.x) {
@@ -231,75 +230,101 @@ static __global__ void k_cheb0_rescale(long long ndof, const double *r, float *b
 // Restriction = transpose of trilinear prolongation (the DMDA Q1
 // interpolation of DMCreateInterpolation, LinearElasticity.cc:2838-2842):
 // coarse node gathers fine nodes 2I-1..2I+1 with weights 1/2, 1, 1/2 per axis.
+// A thread per DOF: the 27 values of a coarse DOF are loaded a plane at a time,
+// and a warp reads runs of consecutive DOFs (2.6 us a level of 64x32x32; a thread
+// per node 5.1: 81 strided loads and 64-bit divisions each).
+template <class T>
+__device__ __forceinline__ void restrict_range(const GridDesc &gf, const GridDesc &gc, const uint8_t *fixc, const T *rf,
+                                               T *bc, long long i0, long long stride) {
+    for (long long m = i0; m < 3 * gc.nn(); m += stride) {
+        const unsigned N = (unsigned)m / 3u;
+        const int c = (int)((unsigned)m - 3u * N);
+        int I, J, K;
+        lex3(N, gc.nx, gc.ny, I, J, K);
+        T acc = T(0);
+        for (int dk = -1; dk <= 1; dk++) {
+            const int k = 2 * K + dk;
+            T v[9];
+#pragma unroll
+            for (int q = 0; q < 9; q++) {
+                const int i = 2 * I + q % 3 - 1, j = 2 * J + q / 3 - 1;
+                const bool in = i >= 0 && i < gf.nx && j >= 0 && j < gf.ny && k >= 0 && k < gf.nz;
+                v[q] = in ? rf[3 * (i + (long long)gf.nx * (j + (long long)gf.ny * k)) + c] : T(0);
+            }
+#pragma unroll
+            for (int q = 0; q < 9; q++)
+                acc += (dk ? T(0.5) : T(1)) * (q / 3 != 1 ? T(0.5) : T(1)) * (q % 3 != 1 ? T(0.5) : T(1)) * v[q];
+        }
+        bc[m] = (fixc[N] >> c) & 1 ? T(0) : acc;
+    }
+}
 template <class T>
 static __global__ void k_restrict(GridDesc gf, GridDesc gc, const uint8_t *fixc, const T *rf, T *bc) {
     grid_dep_wait();
-    long long nn = gc.nn();
-    for (long long N = blockIdx.x * (long long)blockDim.x + threadIdx.x; N < nn; N += (long long)gridDim.x * blockDim.x) {
-        int I = (int)(N % gc.nx), J = (int)((N / gc.nx) % gc.ny), K = (int)(N / ((long long)gc.nx * gc.ny));
-        T acc[3] = {T(0), T(0), T(0)};
-        for (int dk = -1; dk <= 1; dk++) {
-            int k = 2 * K + dk;
-            if (k < 0 || k >= gf.nz) continue;
-            T wk = dk ? T(0.5) : T(1);
-            for (int dj = -1; dj <= 1; dj++) {
-                int j = 2 * J + dj;
-                if (j < 0 || j >= gf.ny) continue;
-                T wj = wk * (dj ? T(0.5) : T(1));
-                for (int di = -1; di <= 1; di++) {
-                    int i = 2 * I + di;
-                    if (i < 0 || i >= gf.nx) continue;
-                    T w = wj * (di ? T(0.5) : T(1));
-                    long long n = i + (long long)gf.nx * (j + (long long)gf.ny * k);
-                    acc[0] += w * rf[3 * n];
-                    acc[1] += w * rf[3 * n + 1];
-                    acc[2] += w * rf[3 * n + 2];
-                }
-            }
-        }
-        mask3(fixc[N], acc);
-        bc[3 * N] = acc[0];
-        bc[3 * N + 1] = acc[1];
-        bc[3 * N + 2] = acc[2];
-    }
+    restrict_range(gf, gc, fixc, rf, bc, blockIdx.x * (long long)blockDim.x + threadIdx.x,
+                   (long long)gridDim.x * blockDim.x);
 }
 
 // x_f += P x_c (trilinear), clamped DOFs untouched
 template <class T>
+__device__ __forceinline__ void prolong_node(const GridDesc &gc, const T *xc, int i, int j, int k, uint8_t f, T x[3]) {
+    int I0 = i >> 1, J0 = j >> 1, K0 = k >> 1;
+    int I1 = I0 + (i & 1), J1 = J0 + (j & 1), K1 = K0 + (k & 1);
+    T acc[3] = {T(0), T(0), T(0)};
+    for (int c = 0; c < 8; c++) {
+        int I = (c & 1) ? I1 : I0, J = ((c >> 1) & 1) ? J1 : J0, K = (c >> 2) ? K1 : K0;
+        // duplicate corners (even index) carry weight 1 split over the two equal picks
+        T w = T(0.125);
+        long long N = I + (long long)gc.nx * (J + (long long)gc.ny * K);
+        acc[0] += w * xc[3 * N];
+        acc[1] += w * xc[3 * N + 1];
+        acc[2] += w * xc[3 * N + 2];
+    }
+    for (int c = 0; c < 3; c++)
+        if (!((f >> c) & 1)) x[c] += acc[c];
+}
+template <class T>
 static __global__ void k_prolong(GridDesc gf, GridDesc gc, const uint8_t *fixf, const T *xc, T *xf) {
     grid_dep_wait();
-    long long nn = gf.nn();
-    for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < nn; n += (long long)gridDim.x * blockDim.x) {
-        int i = (int)(n % gf.nx), j = (int)((n / gf.nx) % gf.ny), k = (int)(n / ((long long)gf.nx * gf.ny));
-        int I0 = i >> 1, J0 = j >> 1, K0 = k >> 1;
-        int I1 = I0 + (i & 1), J1 = J0 + (j & 1), K1 = K0 + (k & 1);
-        T acc[3] = {T(0), T(0), T(0)};
-        for (int c = 0; c < 8; c++) {
-            int I = (c & 1) ? I1 : I0, J = ((c >> 1) & 1) ? J1 : J0, K = (c >> 2) ? K1 : K0;
-            // duplicate corners (even index) carry weight 1 split over the two equal picks
-            T w = T(0.125);
-            long long N = I + (long long)gc.nx * (J + (long long)gc.ny * K);
-            acc[0] += w * xc[3 * N];
-            acc[1] += w * xc[3 * N + 1];
-            acc[2] += w * xc[3 * N + 2];
-        }
-        uint8_t f = fixf[n];
-        for (int c = 0; c < 3; c++)
-            if (!((f >> c) & 1)) xf[3 * n + c] += acc[c];
+    for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < gf.nn(); n += (long long)gridDim.x * blockDim.x) {
+        int i, j, k;
+        lex3(n, gf.nx, gf.ny, i, j, k);
+        T x[3] = {xf[3 * n], xf[3 * n + 1], xf[3 * n + 2]};
+        prolong_node(gc, xc, i, j, k, fixf[n], x);
+        for (int c = 0; c < 3; c++) xf[3 * n + c] = x[c];
     }
 }
 
-// y = A x for the explicit coarse inverse (one warp per row)
+// y = A x for the explicit coarse inverse, GV rows of a warp at once
+template <int GV, class T>
+__device__ __forceinline__ void gemv_range(int n, const T *A, const T *x, T *y, int warp, int warps) {
+    const int lane = threadIdx.x & 31;
+    for (; warp < n; warp += GV * warps) {
+        const T *row[GV];
+        T acc[GV];
+#pragma unroll
+        for (int u = 0; u < GV; u++) {
+            const int i = warp + u * warps;
+            row[u] = A + (size_t)(i < n ? i : n - 1) * n;
+            acc[u] = T(0);
+        }
+#pragma unroll 8
+        for (int j = lane; j < n; j += 32) {
+            const T xj = x[j];
+#pragma unroll
+            for (int u = 0; u < GV; u++) acc[u] += row[u][j] * xj;
+        }
+#pragma unroll
+        for (int u = 0; u < GV; u++) {
+            for (int o = 16; o > 0; o >>= 1) acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], o);
+            if (lane == 0 && warp + u * warps < n) y[warp + u * warps] = acc[u];
+        }
+    }
+}
 template <class T>
 static __global__ void k_gemv(int n, const T *A, const T *x, T *y) {
     grid_dep_wait();
-    int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (warp >= n) return;
-    const T *row = A + (size_t)warp * n;
-    T acc = T(0);
-    for (int j = lane; j < n; j += 32) acc += row[j] * x[j];
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) y[warp] = acc;
+    gemv_range<1>(n, A, x, y, (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), (int)((gridDim.x * blockDim.x) >> 5));
 }
 
 // dense coarsest-level operator, one thread per entry: sum over the (at most 8)

@@ -23,6 +23,7 @@
 
 #include "le.h"
 #include "kron.cuh"
+#include "vtail.cuh"
 #include "mpiio.h"
 #include "sommg.cuh"
 #include "gram.cuh"
@@ -1033,6 +1034,51 @@ struct VFuse {
 
 // sums in the order of the brick kernels and grid_reduce (launch_solve_tile)
 static bool brick_order(const TopoLE *le) { return le->fp64_solves && le->basis32; }
+// CTAs of the largest cluster of k_vtail that the device can hold, a power of two
+// up to VT_CTAS
+static int vtail_ctas() {
+    static int n_dev[MAX_DEVICES] = {};
+    int &n = n_dev[device_slot()];
+    if (!n) {
+        const int sm = (int)TileSmem<float, PolCheb<float>>::bytes;
+        cudaFuncSetAttribute(k_vtail, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+        cudaFuncSetAttribute(k_vtail, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        cudaLaunchConfig_t c = {};
+        c.blockDim = TILE_THREADS;
+        c.dynamicSmemBytes = sm;
+        for (n = VT_CTAS; n > 1; n /= 2) {
+            cudaLaunchAttribute at = {};
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim = {(unsigned)n, 1, 1};
+            c.gridDim = (unsigned)n;
+            c.attrs = &at;
+            c.numAttrs = 1;
+            int clusters = 0;
+            if (cudaOccupancyMaxActiveClusters(&clusters, k_vtail, &c) == cudaSuccess && clusters > 0) break;
+        }
+        cudaGetLastError();  // sizes that the device refuses
+    }
+    return n;
+}
+static void launch_vtail(const VTail &V, const ElemConst<float> &C, int bricks, cudaStream_t s) {
+    unsigned ctas = 1;
+    while ((int)ctas < bricks) ctas *= 2;
+    cudaLaunchAttribute at[2] = {};
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim = {ctas, 1, 1};
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = ctas;
+    c.blockDim = TILE_THREADS;
+    c.dynamicSmemBytes = TileSmem<float, PolCheb<float>>::bytes;
+    c.stream = s;
+    c.attrs = at;
+    c.numAttrs = 2;
+    count_launch();
+    cudaLaunchKernelEx(&c, k_vtail, V, C);
+}
+
 template <class T>
 static T *vcycle(TopoLE *le, int o, int l, const T *b, VFuse *fz = nullptr) {
     cudaStream_t s = le->stream;
@@ -1098,6 +1144,22 @@ static T *vcycle(TopoLE *le, int o, int l, const T *b, VFuse *fz = nullptr) {
         return x;
     }
     const int nu = le->p.smooth;
+    // the last smoothed level in one cluster when it has a CTA for every brick; with
+    // more bricks than CTAs a step takes several rounds on 16 of 152 SMs and the
+    // kernels of their own are faster
+    if constexpr (std::is_same<T, float>::value) {
+        int ntx, nty;
+        const int nt = tile_count(lv.g, ntx, nty);
+        if (l > 0 && l == le->nlev - 2 && le->coarse_dense && op.depth == le->nlev && nu <= VT_SMOOTH &&
+            nt <= vtail_ctas()) {
+            Level &lc = le->L[l + 1];
+            VW<T> wc = vw<T>(le, o, l + 1);
+            launch_vtail(VTail{lv.g, lc.g, lv.fixed, lc.fixed, wt, b, w.dinv, ainv<T>(le, o), w.xa, w.xb, w.r, wc.b,
+                               wc.xa, lohi, nu, le->ncoarse},
+                         *w.C, nt, s);
+            return w.xb;  // 2 nu - 1 steps after the first: an odd number of exchanges
+        }
+    }
     first(lohi);
     for (int k = 1; k < nu; k++) step(lohi, k, false);
     PolResid<T> pr{lv.fixed, wt, x, b, w.r, {}};
@@ -1105,7 +1167,7 @@ static T *vcycle(TopoLE *le, int o, int l, const T *b, VFuse *fz = nullptr) {
     Level &lc = le->L[l + 1];
     VW<T> wc = vw<T>(le, o, l + 1);
     count_launch();
-    launch_dep(lv.g.nn(), k_restrict<T>, ew_blocks(lc.g.nn()), EW, 0, s, lv.g, lc.g, lc.fixed, w.r, wc.b);
+    launch_dep(lv.g.nn(), k_restrict<T>, ew_blocks(3 * lc.g.nn()), EW, 0, s, lv.g, lc.g, lc.fixed, w.r, wc.b);
     T *xc = vcycle<T>(le, o, l + 1, wc.b);
     count_launch();
     launch_dep(lv.g.nn(), k_prolong<T>, ew_blocks(lv.g.nn()), EW, 0, s, lv.g, lc.g, lv.fixed, xc, x);
