@@ -23,13 +23,28 @@ __host__ inline unsigned red_blocks(long long n) {
 // Chebyshev coefficients (c1, c2) of steps k = 0..kmax-1 from the device-side
 // spectrum bounds; computed once per design iteration so that no kernel
 // repeats the FP64 divisions per thread
-// thread 0: the smoothing interval's table, thread 1: the full spectrum's
+// thread 0: the smoothing interval's table, thread 1: the full spectrum's; each in
+// FP64, then rounded to FP32
+constexpr int CHEB_MAX = 64;
+template <class T>
+inline const T *cheb_tab(const double *coef);
+template <>
+inline const double *cheb_tab<double>(const double *coef) {
+    return coef;
+}
+template <>
+inline const float *cheb_tab<float>(const double *coef) {
+    return (const float *)(coef + 2 * CHEB_MAX);
+}
 static __global__ void k_cheb_table(const double *lohi, int kmax, double *smooth, double *full) {
     double *coef = threadIdx.x ? full : smooth, c1, c2;
     for (int k = 0; k < kmax; k++) {
         cheb_coeffs<double>(lohi + 2 * threadIdx.x, k, c1, c2);
         coef[2 * k] = c1;
         coef[2 * k + 1] = c2;
+        float *f = (float *)(coef + 2 * CHEB_MAX);
+        f[2 * k] = (float)c1;
+        f[2 * k + 1] = (float)c2;
     }
 }
 
@@ -193,9 +208,9 @@ static __global__ void k_bounds_final(const unsigned long long *bits, double rat
 
 // first Chebyshev step from a zero initial guess: d = Dinv b / theta, x = d
 template <class T>
-static __global__ void k_cheb0(long long ndof, const T *b, const T *dinv, const double *coef, T *x, T *d) {
+static __global__ void k_cheb0(long long ndof, const T *b, const T *dinv, const T *coef, T *x, T *d) {
     grid_dep_wait();
-    const T c2 = (T)coef[1];
+    const T c2 = coef[1];
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < ndof; i += (long long)gridDim.x * blockDim.x) {
         T v = c2 * dinv[i] * b[i];
         d[i] = v;
@@ -207,10 +222,10 @@ static __global__ void k_cheb0(long long ndof, const T *b, const T *dinv, const 
 // residual replacement (S->rescale) the FP32 right-hand side is re-formed
 // here as r32 = sigma r from the scaled FP64 residual before the step uses it.
 static __global__ void k_cheb0_rescale(long long ndof, const double *r, float *b,
-                                       const float *dinv, const double *coef, float *x, float *d,
+                                       const float *dinv, const float *coef, float *x, float *d,
                                        const SolveScalars *S) {
     grid_dep_wait();
-    const float c2 = (float)coef[1];
+    const float c2 = coef[1];
     const bool rs = S->rescale != 0;
     const ScaleF64 sg = scale_split(S->sigma);
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < ndof; i += (long long)gridDim.x * blockDim.x) {

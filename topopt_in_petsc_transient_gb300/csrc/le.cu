@@ -832,8 +832,8 @@ int le_alloc(TopoLE *le) {
             AG(op.lv[l].dinvd, lnd);
             AG(op.lv[l].dinvf, lnd);
             AG(op.lv[l].lohi, 5);
-            AG(op.lv[l].cheb, 2 * 64);
-            AG(op.lv[l].chebf, 2 * 64);
+            AG(op.lv[l].cheb, 3 * CHEB_MAX);
+            AG(op.lv[l].chebf, 3 * CHEB_MAX);
         }
         if (le->coarse_dense) {
             AG(op.Ainv_d, (size_t)le->ncoarse * le->ncoarse);
@@ -1087,11 +1087,11 @@ static T *vcycle(TopoLE *le, int o, int l, const T *b, VFuse *fz = nullptr) {
     Operator &op = le->ops[o];
     long long nd = 3 * lv.g.nn();
     Weights<T> wt{op.sK != 0.0 ? w.kf : nullptr, w.mf, nullptr, (T)op.sK, (T)op.sM};
-    const double *lohi = op.lv[l].cheb;
+    const T *lohi = cheb_tab<T>(op.lv[l].cheb);
     T *x = w.xa, *xo = w.xb;
     const bool fuse = fz && l == 0 && std::is_same<T, float>::value;
     // first step from zero: x = d = c2 Dinv b
-    auto first = [&](const double *tab) {
+    auto first = [&](const T *tab) {
         if constexpr (std::is_same<T, float>::value) {
             if (fuse) {
                 count_launch();
@@ -1106,7 +1106,7 @@ static T *vcycle(TopoLE *le, int o, int l, const T *b, VFuse *fz = nullptr) {
     };
     // smoothing step k (one operator application); `last`: this level's
     // final step, whose output is the V-cycle result at the fine level
-    auto step = [&](const double *tab, int k, bool last) {
+    auto step = [&](const T *tab, int k, bool last) {
         bool done = false;
         if constexpr (std::is_same<T, float>::value) {
             if (fuse && last) {
@@ -1126,7 +1126,7 @@ static T *vcycle(TopoLE *le, int o, int l, const T *b, VFuse *fz = nullptr) {
     };
     if (l == op.depth - 1 && op.depth < le->nlev) {
         // well-conditioned level: full-spectrum Chebyshev-Jacobi solve from zero
-        const double *full = op.lv[l].chebf;
+        const T *full = cheb_tab<T>(op.lv[l].chebf);
         first(full);
         for (int k = 1; k < le->p.coarse_smooth; k++) step(full, k, k == le->p.coarse_smooth - 1);
         return x;
@@ -1232,7 +1232,7 @@ static T *kron_smooth(TopoLE *le, int o, const T *r, T *z0, VFuse *fz) {
     VW<T> w = vw<T>(le, o, 0);
     Operator &op = le->ops[o];
     Weights<T> wt{op.sK != 0.0 ? w.kf : nullptr, w.mf, nullptr, (T)op.sK, (T)op.sM};
-    const double *tab = op.lv[0].chebf;
+    const T *tab = cheb_tab<T>(op.lv[0].chebf);
     T *x = z0, *xo = (z0 == w.xa) ? w.xb : w.xa;
     for (int k = 0; k < ns; k++) {
         bool done = false;
@@ -2725,7 +2725,7 @@ int le_time_apply(TopoLE *le, int precision, int warmup, int reps, double *ms) {
             launch_tile<double>(l0.g, l0.Cd, pr, s);
         } else if (precision == 3) {
             Weights<float> wt{l0.kff, l0.mff, nullptr, (float)op.sK, (float)op.sM};
-            PolCheb<float> pc{l0.fixed, wt, l0.fr, l0.fb, op.lv[0].dinvf, l0.fxa, l0.fd, op.lv[0].cheb, 1, {}};
+            PolCheb<float> pc{l0.fixed, wt, l0.fr, l0.fb, op.lv[0].dinvf, l0.fxa, l0.fd, cheb_tab<float>(op.lv[0].cheb), 1, {}};
             launch_tile<float>(l0.g, l0.Cf, pc, s);
         } else if (precision == 2) {
             Weights<df> wt = fine_weights<df>(le, true, true, nullptr, op.sK, op.sM);

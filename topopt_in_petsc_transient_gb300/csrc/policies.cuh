@@ -194,9 +194,15 @@ struct PolPQ32 {
     float *q;
     SolveScalars *S;
     Partials<1> part;
+    // read once per thread: after a store the compiler would read them again
+    float beta;
+    bool odd;
+    __device__ void begin() {
+        beta = S->beta32;
+        odd = S->it & 1;
+    }
     __device__ __forceinline__ void pnew(long long n, float v[3]) const {
-        const float beta = S->beta32;
-        const float *pp = (S->it & 1) ? pb[1] : pb[0];  // a select: no local copy of pb
+        const float *pp = odd ? pb[1] : pb[0];  // a select: no local copy of pb
         for (int c = 0; c < 3; c++) v[c] = (beta == 0.0f) ? z[3 * n + c] : z[3 * n + c] + beta * pp[3 * n + c];
     }
     __device__ void load(long long n, float v[1][3]) const {
@@ -216,7 +222,7 @@ struct PolPQ32 {
     }
     using Red = float;  // p.q summed per thread in FP32 (about a dozen nodes), widened once
     __device__ void epilogue(long long n, int, int, int, const float y[3], float red[1], const Pre &r) const {
-        float *pout = (S->it & 1) ? pb[0] : pb[1];
+        float *pout = odd ? pb[0] : pb[1];
         float s = 0.0f;
         for (int c = 0; c < 3; c++) {
             float pv = r.p[c];
@@ -355,7 +361,7 @@ struct PolCheb {
     Weights<T> w;
     const T *x_in, *b, *dinv;
     T *x_out, *d;
-    const double *ctab;  // Chebyshev table [k][2] = (c1, c2), built once per design
+    const T *ctab;  // Chebyshev table [k][2] = (c1, c2), built once per design
     int k;
     Partials<1> part;
     __device__ void load(long long n, T v[1][3]) const {
@@ -386,7 +392,7 @@ struct PolCheb {
         return q;
     }
     __device__ void epilogue(long long n, int, int, int, const T y[3], double *, const Pre &q) const {
-        const T c1 = (T)ctab[2 * k], c2 = (T)ctab[2 * k + 1];
+        const T c1 = ctab[2 * k], c2 = ctab[2 * k + 1];
         for (int c = 0; c < 3; c++) {
             T rv = q.b[c] - (((q.f >> c) & 1) ? q.x[c] : y[c]);
             T dv = c1 * q.d[c] + c2 * q.di[c] * rv;
@@ -408,7 +414,7 @@ struct PolChebDot {
     Weights<float> w;
     const float *x_in, *b, *dinv;
     float *x_out, *d;
-    const double *ctab;
+    const float *ctab;
     int k;
     const float *q32;
     SolveScalars *S;
@@ -438,7 +444,7 @@ struct PolChebDot {
     }
     using Red = float;  // the dot products summed per thread in FP32, widened once
     __device__ void epilogue(long long n, int, int, int, const float y[3], float red[2], const Pre &q) const {
-        const float c1 = (float)ctab[2 * k], c2 = (float)ctab[2 * k + 1];
+        const float c1 = ctab[2 * k], c2 = ctab[2 * k + 1];
         float s0 = 0.0f, s1 = 0.0f;
         for (int c = 0; c < 3; c++) {
             float rv = q.b[c] - (((q.f >> c) & 1) ? q.x[c] : y[c]);

@@ -59,6 +59,14 @@ __device__ __forceinline__ bool pol_skip(const P &, long) {
     return false;
 }
 
+// optional per-thread state read before the first brick: `void begin()`
+template <class P>
+__device__ __forceinline__ auto pol_begin(P &p, int) -> decltype(p.begin()) {
+    p.begin();
+}
+template <class P>
+__device__ __forceinline__ void pol_begin(P &, long) {}
+
 // optional epilogue-operand prefetch: a policy may define `Pre pre(long long n)`
 // and `epilogue(n, i, j, k, y, red, const Pre &)`; the kernel issues pre()
 // before the element phase so the loads overlap the element arithmetic
@@ -392,10 +400,11 @@ __device__ __forceinline__ void tile_run_async(const GridDesc &g, const ElemCons
 }
 
 template <class T, class Pol>
-__global__ void __launch_bounds__(TILE_THREADS, sizeof(T) == 4 ? 2 : 1) k_tile(const GridDesc g, const ElemConst<T> C, const Pol pol) {
+__global__ void __launch_bounds__(TILE_THREADS, sizeof(T) == 4 ? 2 : 1) k_tile(const GridDesc g, const ElemConst<T> C, Pol pol) {
     grid_dep_wait();
     TOPO_DYNAMIC_SMEM(unsigned char, smem_raw);
     if (pol_skip(pol, 0)) return;
+    pol_begin(pol, 0);
     static_assert(TILE_STAGED <= 2 * TILE_THREADS, "staging assumes two passes");
     int ntx, nty;
     const int ntiles = tile_count(g, ntx, nty);

@@ -27,7 +27,7 @@ struct VTail {
     Weights<float> w;
     const float *b, *dinv, *Ainv;
     float *xa, *xb, *r, *bc, *xc;  // the result is left in xb
-    const double *ctab;
+    const float *ctab;
     int nu, n;  // smoothing steps, coarse DOFs
 };
 struct VTElem {  // weights of the thread's element, loaded once
@@ -52,7 +52,7 @@ static __global__ void __launch_bounds__(TILE_THREADS, 1) k_vtail(const VTail V,
     const int ntiles = tile_count(g, ntx, nty), tile = blockIdx.x;
     const bool work = tile < ntiles;
     const int i0 = (tile % ntx) * TILE, j0 = ((tile / ntx) % nty) * TILE, k0 = (tile / (ntx * nty)) * TILE;
-    if (tid < 2 * V.nu) c12[tid] = (float)V.ctab[tid];
+    if (tid < 2 * V.nu) c12[tid] = V.ctab[tid];
     __syncthreads();
     // staged nodes, element and output node of this thread (tile.cuh)
     int sn[2];
