@@ -119,14 +119,11 @@ template <class T>
 __device__ __forceinline__ void kron_line(const T *src, int sstride, int len, int p0, const T *tint,
                                           int c, T out[KRON_MP]) {
     T win[KRON_WIN];
-#pragma unroll
-    for (int k = 0; k < KRON_WIN; k++) {
-        int p = p0 - KRON_B + k;
-        p = p < 0 ? 0 : (p > len - 1 ? len - 1 : p);
-        win[k] = src[p * sstride];
-    }
-    if (p0 >= KRON_B && p0 + KRON_MP <= len - KRON_B) {  // interior group: taps in registers
+    if (p0 >= KRON_B && p0 + KRON_MP <= len - KRON_B) {  // interior group: taps in registers, no clamps
         T tap[KRON_W];
+        const T *s0 = src + (p0 - KRON_B) * sstride;
+#pragma unroll
+        for (int k = 0; k < KRON_WIN; k++) win[k] = s0[k * sstride];
 #pragma unroll
         for (int d = 0; d < KRON_W; d++) tap[d] = tint[c * KRON_W + d];
 #pragma unroll
@@ -137,6 +134,12 @@ __device__ __forceinline__ void kron_line(const T *src, int sstride, int len, in
             out[k] = acc;
         }
         return;
+    }
+#pragma unroll
+    for (int k = 0; k < KRON_WIN; k++) {
+        int p = p0 - KRON_B + k;
+        p = p < 0 ? 0 : (p > len - 1 ? len - 1 : p);
+        win[k] = src[p * sstride];
     }
 #pragma unroll
     for (int k = 0; k < KRON_MP; k++) {
@@ -279,10 +282,11 @@ static __global__ void __launch_bounds__(KRON_THREADS, sizeof(T) == 4 ? 4 : 2)
     // the staging is a pure copy: cp.async puts every copy of the chunk in
     // flight at once, with no register round trip
     static_assert(std::is_same<T, R>::value, "staged r is copied, not converted");
-    for (int t = threadIdx.x; t < len * KW; t += KRON_THREADS) {
-        const int p = t / KW, w = t - p * KW;
-        if (w < wn) {
-            const long long q = base + p * S + w;
+    static_assert(KRON_THREADS % KW == 0, "a thread keeps its value of the row");
+    const int w = threadIdx.x % KW;
+    if (w < wn) {
+        long long q = base + (threadIdx.x / KW) * S + w;
+        for (int t = threadIdx.x; t < len * KW; t += KRON_THREADS, q += (KRON_THREADS / KW) * S) {
             cp_async<(int)sizeof(T)>(tile + t, in + q);
             if (AXIS == 2) {
                 cp_async<(int)sizeof(T)>(rt + t, r + q);
@@ -297,19 +301,18 @@ static __global__ void __launch_bounds__(KRON_THREADS, sizeof(T) == 4 ? 4 : 2)
     // the FCG dot products: FP32 per thread (at most a few dozen terms), FP64
     // across threads (GB300 runs FP64 at 1/64 of the FP32 rate)
     float sr = 0.0f, sq = 0.0f;
+    const int c = (w0 + w) % 3;
     const int ngrp = (len + KRON_MP - 1) / KRON_MP;
     for (int t = threadIdx.x; t < ngrp * KW; t += KRON_THREADS) {
-        const int grp = t / KW, w = t - grp * KW;
         if (w >= wn) continue;
-        const int c = (w0 + w) % 3;
-        const int p0 = grp * KRON_MP;
+        const int p0 = (t / KW) * KRON_MP;
         T o[KRON_MP];
         kron_line(tile + w, KW, len, p0, tint, c, o);
+        long long q = base + p0 * S + w;
 #pragma unroll
-        for (int k = 0; k < KRON_MP; k++) {
+        for (int k = 0; k < KRON_MP; k++, q += S) {
             const int p = p0 + k;
             if (p >= len) break;
-            const long long q = base + p * S + w;
             if (AXIS == 2) {
                 const int sidx = p * KW + w;
                 const T m = mt[sidx], rv = rt[sidx];

@@ -124,6 +124,15 @@ __device__ __forceinline__ TilePos tile_next(TilePos p, TilePos step, int ntx, i
     return p;
 }
 
+// index arithmetic of the kernels in 32 bits (a node index fits, lex3): unsigned
+// comparisons, and widened once for the addresses
+__device__ __forceinline__ bool tile_in(int i, int j, int k, int nx, int ny, int nz) {
+    return (unsigned)i < (unsigned)nx && (unsigned)j < (unsigned)ny && (unsigned)k < (unsigned)nz;
+}
+__device__ __forceinline__ long long tile_index(int i, int j, int k, int nx, int ny) {
+    return (unsigned)i + (unsigned)nx * ((unsigned)j + (unsigned)ny * (unsigned)k);
+}
+
 // staged input nodes of a brick held by this thread (at most two)
 template <class T, class Pol>
 __device__ __forceinline__ void tile_fetch(const Pol &pol, const GridDesc &g, TilePos at, T v[2][Pol::NIN][3]) {
@@ -133,8 +142,8 @@ __device__ __forceinline__ void tile_fetch(const Pol &pol, const GridDesc &g, Ti
         const int s = threadIdx.x + it * TILE_THREADS;
         const int lx = s % TILE_N, ly = (s / TILE_N) % TILE_N, lz = s / (TILE_N * TILE_N);
         const int gi = i0 - 1 + lx, gj = j0 - 1 + ly, gk = k0 - 1 + lz;
-        if (s < TILE_STAGED && gi >= 0 && gi < g.nx && gj >= 0 && gj < g.ny && gk >= 0 && gk < g.nz) {
-            long long n = gi + (long long)g.nx * (gj + (long long)g.ny * gk);
+        if (s < TILE_STAGED && tile_in(gi, gj, gk, g.nx, g.ny, g.nz)) {
+            const long long n = tile_index(gi, gj, gk, g.nx, g.ny);
             pol.load(n, v[it]);
         } else {
 #pragma unroll
@@ -155,8 +164,8 @@ __device__ __forceinline__ void tile_elements(const GridDesc &g, const ElemConst
     const int lx = tid & 7, ly = (tid >> 3) & 7, lz = tid >> 6;
     const int ei = i0 - 1 + lx, ej = j0 - 1 + ly, ek = k0 - 1 + lz;
     T *out = sEl + tid * EL_STRIDE;
-    if (ei >= 0 && ei < g.ex && ej >= 0 && ej < g.ey && ek >= 0 && ek < g.ez) {
-        long long e = ei + (long long)g.ex * (ej + (long long)g.ey * ek);
+    if (tile_in(ei, ej, ek, g.ex, g.ey, g.ez)) {
+        const long long e = tile_index(ei, ej, ek, g.ex, g.ey);
         T ck, cm;
         pol.coef(e, ck, cm);
         T U[3][8];
@@ -273,7 +282,7 @@ __device__ __forceinline__ void tile_brick(const GridDesc &g, const ElemConst<T>
     const int tx = tid % TILE, ty = (tid / TILE) % TILE, tz = tid / (TILE * TILE);
     const int oi = i0 + tx, oj = j0 + ty, ok = k0 + tz;
     const bool has_out = tid < TILE_OUT && oi < g.nx && oj < g.ny && ok < g.nz;
-    const long long on = has_out ? oi + (long long)g.nx * (oj + (long long)g.ny * ok) : 0;
+    const long long on = has_out ? tile_index(oi, oj, ok, g.nx, g.ny) : 0;
     const auto pre = pol_pre(pol, on, 0);
     __syncthreads();
     if (more) tile_fetch<T>(pol, g, next, v);
@@ -354,8 +363,8 @@ __device__ __forceinline__ void tile_fetch_async(const Pol &pol, const GridDesc 
         const int lx = s % TILE_N, ly = (s / TILE_N) % TILE_N, lz = s / (TILE_N * TILE_N);
         const int gi = i0 - 1 + lx, gj = j0 - 1 + ly, gk = k0 - 1 + lz;
         f[it] = 0;
-        if (s < TILE_STAGED && gi >= 0 && gi < g.nx && gj >= 0 && gj < g.ny && gk >= 0 && gk < g.nz) {
-            const long long n = gi + (long long)g.nx * (gj + (long long)g.ny * gk);
+        if (s < TILE_STAGED && tile_in(gi, gj, gk, g.nx, g.ny, g.nz)) {
+            const long long n = tile_index(gi, gj, gk, g.nx, g.ny);
 #pragma unroll
             for (int k = 0; k < Pol::NSRC; k++)
 #pragma unroll
@@ -394,7 +403,7 @@ __device__ __forceinline__ void tile_run_async(const GridDesc &g, const ElemCons
                 const int lx = s % TILE_N, ly = (s / TILE_N) % TILE_N, lz = s / (TILE_N * TILE_N);
                 const int gi = i0 - 1 + lx, gj = j0 - 1 + ly, gk = k0 - 1 + lz;
                 T v[1][3] = {{T(0), T(0), T(0)}};
-                if (gi >= 0 && gi < g.nx && gj >= 0 && gj < g.ny && gk >= 0 && gk < g.nz) {
+                if (tile_in(gi, gj, gk, g.nx, g.ny, g.nz)) {
                     Src rv[Pol::NSRC][3];
 #pragma unroll
                     for (int k = 0; k < Pol::NSRC; k++)
@@ -409,7 +418,7 @@ __device__ __forceinline__ void tile_run_async(const GridDesc &g, const ElemCons
         const int tx = tid % TILE, ty = (tid / TILE) % TILE, tz = tid / (TILE * TILE);
         const int oi = i0 + tx, oj = j0 + ty, ok = k0 + tz;
         const bool has_out = tid < TILE_OUT && oi < g.nx && oj < g.ny && ok < g.nz;
-        const long long on = has_out ? oi + (long long)g.nx * (oj + (long long)g.ny * ok) : 0;
+        const long long on = has_out ? tile_index(oi, oj, ok, g.nx, g.ny) : 0;
         const auto pre = pol_pre(pol, on, 0);
         __syncthreads();
         if (tile + (int)gridDim.x < ntiles) tile_fetch_async<T>(pol, g, next, raw, f);
