@@ -259,6 +259,9 @@ template <class T>
 constexpr bool tile_persistent() {
     return sizeof(T) == 4;
 }
+// Two barriers a brick: the staged nodes are free once the element phase is over,
+// so the next brick is staged beside the gather, and the element outputs once every
+// thread has come to the next staging barrier.
 // one brick: stage (v holds its staged nodes), element phase, gather and
 // epilogue; with `more` the staged nodes of brick `next` are loaded into v while
 // this brick is computed
@@ -425,7 +428,6 @@ __device__ __forceinline__ void tile_run_async(const GridDesc &g, const ElemCons
         tile_elements<T>(g, C, pol, sIn, sEl, i0, j0, k0);
         __syncthreads();
         if (has_out) tile_gather<T>(pol, sEl, on, oi, oj, ok, tx, ty, tz, pre, red);
-        __syncthreads();  // shared memory is restaged for the next brick
     }
 }
 
@@ -455,7 +457,6 @@ __global__ void __launch_bounds__(TILE_THREADS, sizeof(T) == 4 ? 2 : 1) k_tile(c
                 const TilePos next = tile_next(at, step, ntx, nty);
                 tile_brick<T>(g, C, pol, sIn, sEl, at, next, tile + (int)gridDim.x < ntiles, v, red);
                 at = next;
-                __syncthreads();  // shared memory is restaged for the next brick
             }
         } else {
             tile_fetch<T>(pol, g, at, v);
