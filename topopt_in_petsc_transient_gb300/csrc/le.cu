@@ -297,6 +297,22 @@ static void launch_march(const GridDesc &g, const ElemConst<double> &C, const Po
 // others launch one CTA per brick
 template <class T, class Pol>
 static void launch_brick(const GridDesc &g, const ElemConst<T> &C, const Pol &pol, cudaStream_t s) {
+    // FP64: the unit is a warp's elements on one of an SM's four FP64 pipes.  A brick
+    // of 7 is 4 units on one SM however few there are; bricks of 3 (2 warps, 2.4
+    // instead of 1.5 elements a node) spread a coarse level over the SMs.  A
+    // smoothing step at 25x13x13 or 13x7x7 nodes takes 13 us instead of 35 (the reduced
+    // evaluation at 48x24x24 59 ms instead of 88); at 49x25x25 the bricks of 7 are 4 units,
+    // those of 3 would be 5.
+    if constexpr (std::is_same<T, double>::value && Pol::NRED == 0) {
+        int ntx, nty;
+        const int big = tile_count(g, ntx, nty), small = tile_count(g, ntx, nty, TILE_SMALL), nsm = sm_count();
+        if ((2 * ((small + nsm - 1) / nsm) + 3) / 4 < 4 * ((big + nsm - 1) / nsm)) {
+            count_launch();
+            launch_dep(g.nn(), k_tile<T, Pol, TILE_SMALL>, (unsigned)small, TileGeom<TILE_SMALL>::THREADS,
+                       tile_smem_bytes<T, Pol, TILE_SMALL>(), s, g, C, pol);
+            return;
+        }
+    }
     static int resident_dev[MAX_DEVICES] = {};
     int &resident = resident_dev[device_slot()];
     const size_t sm = TileSmem<T, Pol>::bytes;
