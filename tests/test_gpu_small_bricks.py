@@ -1,7 +1,6 @@
-"""FP64 bricks of three nodes an edge (the coarse levels of a basis solve whose
-vectors are stored in FP32): grids of one brick, with remainders in every
-direction, of more bricks than SMs, and one whose fine level keeps bricks of
-seven.
+"""FP64 bricks of 3x3x3 and 7x7x5 nodes (basis solves whose vectors are stored in
+FP32): grids of one brick, with remainders in every direction, of more bricks than
+SMs, and two whose fine level takes bricks of 7x7x5, with remainders and without.
 
 Tolerance: the basis vectors of both modes solve the same FP64 systems to rtol
 1e-13; the first row of the mixed one is that of the plain path rounded to FP32,
@@ -17,7 +16,7 @@ M6 = (1e-9, 1.0, 1e-3, 1.0, 3.0, 1.0)
 
 
 @pytest.mark.parametrize("n,nlvls", [((2, 2, 2), 2), ((6, 2, 4), 2), ((8, 4, 4), 3), ((28, 16, 12), 3),
-                                     ((48, 24, 24), 4)])
+                                     ((44, 24, 24), 3), ((48, 24, 24), 4)])
 def test_small_bricks(gpu, n, nlvls):
     from topopt_in_petsc_transient_gb300 import LinearElasticity
     x = 0.3 + 0.1 * np.random.default_rng(sum(n)).random(np.prod(n))

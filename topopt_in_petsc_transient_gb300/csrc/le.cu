@@ -291,6 +291,21 @@ static void launch_march(const GridDesc &g, const ElemConst<double> &C, const Po
     else
         launch_dep(g.nn(), k_march<Pol, false>, grid, d.tx * d.ty, sm, s, g, C, pol, d);
 }
+// FP64 bricks of another shape, for operators without reductions (one CTA a brick)
+template <class Pol, int TL, int TZ>
+static void launch_brick_of(const GridDesc &g, const ElemConst<double> &C, const Pol &pol, cudaStream_t s) {
+    constexpr size_t sm = tile_smem_bytes<double, Pol, TL, TZ>();
+    static bool attr_dev[MAX_DEVICES] = {};
+    bool &attr = attr_dev[device_slot()];
+    if (!attr) {
+        cudaFuncSetAttribute(k_tile<double, Pol, TL, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        attr = true;
+    }
+    int ntx, nty;
+    const int n = tile_count(g, ntx, nty, TL, TZ);
+    count_launch();
+    launch_dep(g.nn(), k_tile<double, Pol, TL, TZ>, (unsigned)n, TileGeom<TL, TZ>::THREADS, sm, s, g, C, pol);
+}
 // FP32 and double-float: bricks.  FP32 kernels and kernels staged by asynchronous
 // copies are persistent: as many CTAs as are resident on the device at once
 // (occupancy of this instantiation x SM count), capped by the brick count; the
@@ -298,20 +313,20 @@ static void launch_march(const GridDesc &g, const ElemConst<double> &C, const Po
 template <class T, class Pol>
 static void launch_brick(const GridDesc &g, const ElemConst<T> &C, const Pol &pol, cudaStream_t s) {
     // FP64: the unit is a warp's elements on one of an SM's four FP64 pipes.  A brick
-    // of 7 is 4 units on one SM however few there are; bricks of 3 (2 warps, 2.4
-    // instead of 1.5 elements a node) spread a coarse level over the SMs.  A
-    // smoothing step at 25x13x13 or 13x7x7 nodes takes 13 us instead of 35 (the reduced
-    // evaluation at 48x24x24 59 ms instead of 88); at 49x25x25 the bricks of 7 are 4 units,
-    // those of 3 would be 5.
+    // of 7x7x7 is 4 units on one SM however few there are, one of 7x7x5 3, and those
+    // of 3x3x3 (2 warps, 2.4 instead of 1.5 elements a node) spread a coarse level over
+    // the SMs.  A smoothing step takes 13 us instead of 35 at 25x13x13 or 13x7x7 nodes
+    // (1 unit; the reduced evaluation at 48x24x24 59 ms instead of 88) and 32 instead
+    // of 42 at 49x25x25 (140 bricks of 3 units; 4 with 7x7x7, 5 with 3x3x3; 52.6 ms).
     if constexpr (std::is_same<T, double>::value && Pol::NRED == 0) {
-        int ntx, nty;
-        const int big = tile_count(g, ntx, nty), small = tile_count(g, ntx, nty, TILE_SMALL), nsm = sm_count();
-        if ((2 * ((small + nsm - 1) / nsm) + 3) / 4 < 4 * ((big + nsm - 1) / nsm)) {
-            count_launch();
-            launch_dep(g.nn(), k_tile<T, Pol, TILE_SMALL>, (unsigned)small, TileGeom<TILE_SMALL>::THREADS,
-                       tile_smem_bytes<T, Pol, TILE_SMALL>(), s, g, C, pol);
-            return;
-        }
+        const int nsm = sm_count();
+        auto units = [&](int tl, int tz, int warps) {
+            int ntx, nty;
+            return (warps * ((tile_count(g, ntx, nty, tl, tz) + nsm - 1) / nsm) + 3) / 4;
+        };
+        const int u7 = units(7, 7, 16), u5 = units(7, 5, 12), u3 = units(3, 3, 2);
+        if (u3 < u7 && u3 <= u5) return launch_brick_of<Pol, 3, 3>(g, C, pol, s);
+        if (u5 < u7) return launch_brick_of<Pol, 7, 5>(g, C, pol, s);
     }
     static int resident_dev[MAX_DEVICES] = {};
     int &resident = resident_dev[device_slot()];
@@ -1070,9 +1085,10 @@ static int vtail_ctas() {
             c.attrs = &at;
             c.numAttrs = 1;
             int clusters = 0;
-            if (cudaOccupancyMaxActiveClusters(&clusters, k_vtail, &c) == cudaSuccess && clusters > 0) break;
+            const cudaError_t e = cudaOccupancyMaxActiveClusters(&clusters, k_vtail, &c);
+            if (e == cudaSuccess && clusters > 0) break;
+            if (e != cudaSuccess) cudaGetLastError();  // a size that the device refuses
         }
-        cudaGetLastError();  // sizes that the device refuses
     }
     return n;
 }

@@ -26,25 +26,26 @@ constexpr int TILE_THREADS = 512;     // == TILE_E^3
 constexpr int TILE_STAGED = TILE_N * TILE_N * TILE_N;  // 729
 constexpr int TILE_OUT = TILE * TILE * TILE;            // 343
 constexpr int EL_STRIDE = 25;         // padded element-output row (bank spread)
-// the same of bricks of TL output nodes an edge: 7, or 3 (launch_brick)
-constexpr int TILE_SMALL = 3;
-template <int TL>
+// the same of bricks of TL x TL x TZ output nodes: 7x7x7, in FP64 also 7x7x5 and
+// 3x3x3 (launch_brick)
+template <int TL, int TZ>
 struct TileGeom {
-    static constexpr int E = TL + 1, N = TL + 2, THREADS = E * E * E, STAGED = N * N * N, OUT = TL * TL * TL;
+    static constexpr int E = TL + 1, N = TL + 2, THREADS = E * E * (TZ + 1), STAGED = N * N * (TZ + 2);
+    static constexpr int OUT = TL * TL * TZ;
     static constexpr int LOG = E == 8 ? 3 : 2;  // E = 2^LOG
     static_assert(E == 1 << LOG && STAGED <= 2 * THREADS, "staging in two passes");
 };
 
-template <class T, class Pol, int TL = TILE>
+template <class T, class Pol, int TL = TILE, int TZ = TILE>
 constexpr size_t tile_smem_bytes() {
     return sizeof(T) *
-           ((size_t)Pol::NIN * TileGeom<TL>::STAGED * 3 + (size_t)TileGeom<TL>::THREADS * EL_STRIDE);
+           ((size_t)Pol::NIN * TileGeom<TL, TZ>::STAGED * 3 + (size_t)TileGeom<TL, TZ>::THREADS * EL_STRIDE);
 }
 
-__host__ __device__ inline int tile_count(const GridDesc &g, int &ntx, int &nty, int tl = TILE) {
+__host__ __device__ inline int tile_count(const GridDesc &g, int &ntx, int &nty, int tl = TILE, int tz = TILE) {
     ntx = (g.nx + tl - 1) / tl;
     nty = (g.ny + tl - 1) / tl;
-    return ntx * nty * ((g.nz + tl - 1) / tl);
+    return ntx * nty * ((g.nz + tz - 1) / tz);
 }
 
 // Policy interface:
@@ -143,10 +144,10 @@ __device__ __forceinline__ long long tile_index(int i, int j, int k, int nx, int
 }
 
 // staged input nodes of a brick held by this thread (at most two)
-template <class T, int TL = TILE, class Pol>
+template <class T, int TL = TILE, int TZ = TILE, class Pol>
 __device__ __forceinline__ void tile_fetch(const Pol &pol, const GridDesc &g, TilePos at, T v[2][Pol::NIN][3]) {
-    using G = TileGeom<TL>;
-    const int i0 = at.i * TL, j0 = at.j * TL, k0 = at.k * TL;
+    using G = TileGeom<TL, TZ>;
+    const int i0 = at.i * TL, j0 = at.j * TL, k0 = at.k * TZ;
 #pragma unroll
     for (int it = 0; it < 2; it++) {
         const int s = threadIdx.x + it * G::THREADS;
@@ -167,10 +168,10 @@ __device__ __forceinline__ void tile_fetch(const Pol &pol, const GridDesc &g, Ti
 // ---------------------------------------------------------------------------
 // one element per thread: the 24 outputs of element (lx, ly, lz) of the brick
 // at (i0, j0, k0) from the staged nodes sIn into sEl
-template <class T, int TL = TILE, class Pol>
+template <class T, int TL = TILE, int TZ = TILE, class Pol>
 __device__ __forceinline__ void tile_elements(const GridDesc &g, const ElemConst<T> &C, const Pol &pol, const T *sIn,
                                               T *sEl, int i0, int j0, int k0) {
-    using G = TileGeom<TL>;
+    using G = TileGeom<TL, TZ>;
     const int tid = threadIdx.x;
     const int lx = tid & (G::E - 1), ly = (tid >> G::LOG) & (G::E - 1), lz = tid >> (2 * G::LOG);
     const int ei = i0 - 1 + lx, ej = j0 - 1 + ly, ek = k0 - 1 + lz;
@@ -240,10 +241,10 @@ __device__ __forceinline__ void tile_elements(const GridDesc &g, const ElemConst
 
 // the output node (tx, ty, tz) of this thread: its 8 element contributions
 // from sEl, then the policy epilogue
-template <class T, int TL = TILE, class Pol, class R>
+template <class T, int TL = TILE, int TZ = TILE, class Pol, class R>
 __device__ __forceinline__ void tile_gather(const Pol &pol, const T *sEl, long long on, int oi, int oj, int ok, int tx,
                                             int ty, int tz, const R &pre, pol_red_t<Pol> *red) {
-    constexpr int E = TileGeom<TL>::E;
+    constexpr int E = TileGeom<TL, TZ>::E;
     T y[3] = {T(0), T(0), T(0)};
 #pragma unroll
     for (int L = 0; L < 8; L++) {
@@ -277,13 +278,13 @@ constexpr bool tile_persistent() {
 // one brick: stage (v holds its staged nodes), element phase, gather and
 // epilogue; with `more` the staged nodes of brick `next` are loaded into v while
 // this brick is computed
-template <class T, int TL = TILE, class Pol>
+template <class T, int TL = TILE, int TZ = TILE, class Pol>
 __device__ __forceinline__ void tile_brick(const GridDesc &g, const ElemConst<T> &C, const Pol &pol, T *sIn, T *sEl,
                                            TilePos at, TilePos next, bool more, T v[2][Pol::NIN][3],
                                            pol_red_t<Pol> *red) {
-    using G = TileGeom<TL>;
+    using G = TileGeom<TL, TZ>;
     const int tid = threadIdx.x;
-    const int i0 = at.i * TL, j0 = at.j * TL, k0 = at.k * TL;
+    const int i0 = at.i * TL, j0 = at.j * TL, k0 = at.k * TZ;
 #pragma unroll
     for (int it = 0; it < 2; it++) {
         const int s = tid + it * G::THREADS;
@@ -301,10 +302,10 @@ __device__ __forceinline__ void tile_brick(const GridDesc &g, const ElemConst<T>
     const long long on = has_out ? tile_index(oi, oj, ok, g.nx, g.ny) : 0;
     const auto pre = pol_pre(pol, on, 0);
     __syncthreads();
-    if (more) tile_fetch<T, TL>(pol, g, next, v);
-    tile_elements<T, TL>(g, C, pol, sIn, sEl, i0, j0, k0);
+    if (more) tile_fetch<T, TL, TZ>(pol, g, next, v);
+    tile_elements<T, TL, TZ>(g, C, pol, sIn, sEl, i0, j0, k0);
     __syncthreads();
-    if (has_out) tile_gather<T, TL>(pol, sEl, on, oi, oj, ok, tx, ty, tz, pre, red);
+    if (has_out) tile_gather<T, TL, TZ>(pol, sEl, on, oi, oj, ok, tx, ty, tz, pre, red);
 }
 
 // ---------------------------------------------------------------------------
@@ -444,41 +445,41 @@ __device__ __forceinline__ void tile_run_async(const GridDesc &g, const ElemCons
     }
 }
 
-template <class T, class Pol, int TL = TILE>
-__global__ void __launch_bounds__(TileGeom<TL>::THREADS, sizeof(T) == 4 ? 2 : 1) k_tile(const GridDesc g, const ElemConst<T> C, Pol pol) {
+template <class T, class Pol, int TL = TILE, int TZ = TILE>
+__global__ void __launch_bounds__(TileGeom<TL, TZ>::THREADS, sizeof(T) == 4 ? 2 : 1) k_tile(const GridDesc g, const ElemConst<T> C, Pol pol) {
     grid_dep_wait();
     TOPO_DYNAMIC_SMEM(unsigned char, smem_raw);
     if (pol_skip(pol, 0)) return;
     pol_begin(pol, 0);
     int ntx, nty;
-    const int ntiles = tile_count(g, ntx, nty, TL);
+    const int ntiles = tile_count(g, ntx, nty, TL, TZ);
     pol_red_t<Pol> red[Pol::NRED > 0 ? Pol::NRED : 1];
 #pragma unroll
     for (int r = 0; r < (Pol::NRED > 0 ? Pol::NRED : 1); r++) red[r] = 0;
-    static_assert(TL == TILE || !(tile_async<T, Pol>() || tile_persistent<T>()), "small bricks: one a CTA");
+    static_assert((TL == TILE && TZ == TILE) || !(tile_async<T, Pol>() || tile_persistent<T>()), "other bricks: one a CTA");
     if constexpr (tile_async<T, Pol>()) {
         tile_run_async<T>(g, C, pol, smem_raw, ntiles, ntx, nty, red);
     } else {
         T *sIn = reinterpret_cast<T *>(smem_raw);
-        T *sEl = sIn + Pol::NIN * TileGeom<TL>::STAGED * 3;
+        T *sEl = sIn + Pol::NIN * TileGeom<TL, TZ>::STAGED * 3;
         T v[2][Pol::NIN][3];
         TilePos at = tile_pos(blockIdx.x, ntx, nty);
         if constexpr (tile_persistent<T>()) {
             const TilePos step = tile_pos(gridDim.x, ntx, nty);
-            if ((int)blockIdx.x < ntiles) tile_fetch<T, TL>(pol, g, at, v);
+            if ((int)blockIdx.x < ntiles) tile_fetch<T, TL, TZ>(pol, g, at, v);
             for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
                 const TilePos next = tile_next(at, step, ntx, nty);
-                tile_brick<T, TL>(g, C, pol, sIn, sEl, at, next, tile + (int)gridDim.x < ntiles, v, red);
+                tile_brick<T, TL, TZ>(g, C, pol, sIn, sEl, at, next, tile + (int)gridDim.x < ntiles, v, red);
                 at = next;
             }
         } else {
-            tile_fetch<T, TL>(pol, g, at, v);
-            tile_brick<T, TL>(g, C, pol, sIn, sEl, at, at, false, v, red);
+            tile_fetch<T, TL, TZ>(pol, g, at, v);
+            tile_brick<T, TL, TZ>(g, C, pol, sIn, sEl, at, at, false, v, red);
         }
     }
     if constexpr (Pol::NRED > 0) {
         double tot[Pol::NRED];
-        if (grid_reduce<TileGeom<TL>::THREADS, Pol::NRED>(red, pol.part, tot)) pol.finish(tot);
+        if (grid_reduce<TileGeom<TL, TZ>::THREADS, Pol::NRED>(red, pol.part, tot)) pol.finish(tot);
     }
 }
 
