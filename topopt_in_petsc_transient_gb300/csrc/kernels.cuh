@@ -388,8 +388,10 @@ static __global__ void k_coarse_assemble(GridDesc g, const uint8_t *__restrict__
 // took two: 8 ms of launches for n = 675 become 0.6.
 constexpr int CH = 32;
 // panel k0: rows k0 + 32 b .. of block b, one row a lane, the diagonal block
-// factored by every CTA for itself.  Uc, Qc [n][CH]: unscaled columns and c_i / c_k.
-static __global__ void __launch_bounds__(32) k_chol_panel(double *A, int n, int k0, double *Uc, double *Qc) {
+// factored by every CTA for itself.  Uc, Qc [n][CH]: unscaled columns and c_i / c_k
+// of the rows below the diagonal block.  The factor of that block goes to its own
+// rows of Uc, not over A: other CTAs of the launch may have yet to read it there.
+__device__ __forceinline__ void chol_panel(double *A, int n, int k0, double *Uc, double *Qc, int block) {
     const int lane = threadIdx.x, w = min(CH, n - k0);
     double d[CH], a[CH];
 #pragma unroll
@@ -401,13 +403,13 @@ static __global__ void __launch_bounds__(32) k_chol_panel(double *A, int n, int 
 #pragma unroll
         for (int j = k + 1; j < CH; j++) d[j] -= q * __shfl_sync(0xffffffffu, d[k], j);
     }
-    const int row = k0 + CH * blockIdx.x + lane;  // block 0: the diagonal block's own rows
-    if (blockIdx.x == 0) {
+    const int row = k0 + CH * block + lane;  // block 0: the diagonal block's own rows
+    if (block == 0) {
 #pragma unroll
         for (int k = 0; k < CH; k++) {
             if (k >= w) break;
             const double p = __shfl_sync(0xffffffffu, d[k], k), r = sqrt(p);
-            if (lane < w && k <= lane) A[(size_t)row * n + k0 + k] = k == lane ? r : d[k] / r;
+            if (lane < w && k <= lane) Uc[(size_t)row * CH + k] = k == lane ? r : d[k] / r;
         }
         return;
     }
@@ -425,6 +427,9 @@ static __global__ void __launch_bounds__(32) k_chol_panel(double *A, int n, int 
             A[(size_t)row * n + k0 + k] = a[k] / sqrt(p);
         }
     }
+}
+static __global__ void __launch_bounds__(32) k_chol_panel(double *A, int n, int k0, double *Uc, double *Qc) {
+    chol_panel(A, n, k0, Uc, Qc, blockIdx.x);
 }
 // C(i, j) -= sum over the CH columns k of X(i, k) Y(k, j), k ascending, on 32 x 32
 // tiles at rows r0.. and columns c0..; sx, sy: row strides, ty: Y given as Y(j, k).
@@ -457,11 +462,12 @@ static __global__ void k_chol_identity(double *W, int n) {
         W[t] = (t / n == t % n) ? 1.0 : 0.0;
 }
 // forward substitution within the rows i0 .. i0 + 31 of W, one column a lane:
-// row i divided by L(i, i), then L(r, i) times it taken from the rows r below
-static __global__ void __launch_bounds__(32) k_chol_trsv(const double *L, double *W, int n, int i0) {
+// row i divided by L(i, i), then L(r, i) times it taken from the rows r below.
+// D: the diagonal blocks of L (k_chol_panel's Uc)
+static __global__ void __launch_bounds__(32) k_chol_trsv(const double *D, double *W, int n, int i0) {
     __shared__ double Ld[CH][CH + 1];
     const int lane = threadIdx.x, h = min(CH, n - i0), c = CH * blockIdx.x + lane;
-    for (int r = 0; r < h; r++) Ld[r][lane] = lane < h ? L[(size_t)(i0 + r) * n + i0 + lane] : 0.0;
+    for (int r = 0; r < h; r++) Ld[r][lane] = lane <= r ? D[(size_t)(i0 + r) * CH + lane] : 0.0;
     __syncwarp();
     double w[CH];
 #pragma unroll
@@ -505,6 +511,34 @@ static __global__ void __launch_bounds__(256) k_chol_gram(const double *__restri
             Ainvf[(size_t)i * n + j] = (float)s[u];
         }
     }
+}
+
+// inverse of the SPD matrix at A (lower triangle read) in A and, rounded, in Ainvf;
+// W: n x n, U: 2 CH n scratch.  The Gram product reads W alone, so it may go over
+// the factor's storage.
+static inline void chol_inverse(double *A, float *Ainvf, int n, double *W, double *U, cudaStream_t s) {
+    double *Q = U + (size_t)CH * n;
+    auto tiles = [](int m) { return (unsigned)((m + CH - 1) / CH); };
+    for (int k0 = 0; k0 < n; k0 += CH) {
+        count_launch();
+        k_chol_panel<<<tiles(n - k0), 32, 0, s>>>(A, n, k0, U, Q);
+        const int m = n - k0 - CH;  // rows below the panel (which then is a whole one)
+        if (m <= 0) break;
+        count_launch();
+        k_chol_update<<<dim3(tiles(m), tiles(m)), 256, 0, s>>>(A, n, k0 + CH, k0 + CH, n, Q, CH, U, CH, 1, 1);
+    }
+    count_launch();
+    k_chol_identity<<<ew_blocks((long long)n * n), EW, 0, s>>>(W, n);
+    for (int i0 = 0; i0 < n; i0 += CH) {
+        const int c1 = n < i0 + CH ? n : i0 + CH, m = n - i0 - CH;
+        count_launch();
+        k_chol_trsv<<<tiles(c1), 32, 0, s>>>(U, W, n, i0);
+        if (m <= 0) break;
+        count_launch();
+        k_chol_update<<<dim3(tiles(c1), tiles(m)), 256, 0, s>>>(W, n, i0 + CH, 0, c1, A + i0, n, W + (size_t)i0 * n, n, 0, 0);
+    }
+    count_launch();
+    k_chol_gram<<<dim3(tiles(n), tiles(n)), 256, 0, s>>>(W, n, A, Ainvf);
 }
 
 static __global__ void k_d2f(long long n, const double *__restrict__ a, float *b) {

@@ -980,32 +980,8 @@ static int setup_operator(TopoLE *le, int o) {
     count_launch();
     k_coarse_assemble<<<ew_blocks((long long)n * n), EW, 0, s>>>(lc.g, lc.fixed, kfp, lc.mfd, op.sK, op.sM, le->KEc,
                                                                  le->MEc, op.Ainv_d);
-    // FP64 Cholesky factor of the coarsest operator, then its inverse from the
-    // factor (k_chol_*): A^-1 = L^-T L^-1, written over the factor's storage
-    // (the Gram product reads W alone)
-    double *A = op.Ainv_d, *W = le->chol_w, *Uc = le->chol_col, *Qc = le->chol_col + (size_t)CH * n;
-    auto tiles = [](int m) { return (unsigned)((m + CH - 1) / CH); };
-    for (int k0 = 0; k0 < n; k0 += CH) {
-        count_launch();
-        k_chol_panel<<<tiles(n - k0), 32, 0, s>>>(A, n, k0, Uc, Qc);
-        const int m = n - k0 - CH;  // rows below the panel (which then is a whole one)
-        if (m <= 0) break;
-        count_launch();
-        k_chol_update<<<dim3(tiles(m), tiles(m)), 256, 0, s>>>(A, n, k0 + CH, k0 + CH, n, Qc, CH, Uc, CH, 1, 1);
-    }
-    count_launch();
-    k_chol_identity<<<ew_blocks((long long)n * n), EW, 0, s>>>(W, n);
-    for (int i0 = 0; i0 < n; i0 += CH) {
-        const int c1 = std::min(n, i0 + CH), m = n - i0 - CH;
-        count_launch();
-        k_chol_trsv<<<tiles(c1), 32, 0, s>>>(A, W, n, i0);
-        if (m <= 0) break;
-        count_launch();
-        k_chol_update<<<dim3(tiles(c1), tiles(m)), 256, 0, s>>>(W, n, i0 + CH, 0, c1, A + i0, n, W + (size_t)i0 * n, n,
-                                                                 0, 0);
-    }
-    count_launch();
-    k_chol_gram<<<dim3(tiles(n), tiles(n)), 256, 0, s>>>(W, n, A, op.Ainv_f);
+    // FP64 Cholesky factor of the coarsest operator, then its inverse from the factor
+    chol_inverse(op.Ainv_d, op.Ainv_f, n, le->chol_w, le->chol_col, s);
     CK(cudaGetLastError());
     return TOPO_OK;
 }
