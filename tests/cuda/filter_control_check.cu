@@ -1,0 +1,155 @@
+// filter_control_check.cu -- the PDE filter's solve (filter.cu) with its scalars
+// (filtctl.cuh) on the host, node by node in the kernel's arithmetic: fields and
+// radii for which a correction cannot take a step have to end all the same.
+// Prints "control OK".
+#include <algorithm>
+#include <cstdio>
+#include <vector>
+
+#include "filtctl.cuh"
+
+using namespace topo;
+
+struct Result {
+    int status, its, corrections;
+    double residual;  // |b - K u| / |b|
+};
+struct Model {
+    int n[3];  // elements
+    double h[3], R, c64[8];
+    float c32[8];
+    long long nn;
+    std::vector<double> b, u, r;
+    std::vector<float> bd;
+    Model(int ex, int ey, int ez, double rmin) : n{ex, ey, ez}, h{1.0, 1.0, 1.0}, R(rmin / 2.0 / std::sqrt(3.0)) {
+        filt_stencil(h, R, c64);
+        for (int S = 0; S < 8; S++) c32[S] = (float)c64[S];
+        nn = (long long)(ex + 1) * (ey + 1) * (ez + 1);
+        bd.resize(nn);
+        for (long long q = 0; q < nn; q++) {
+            int i[3];
+            node(q, i);
+            bd[q] = 1.0f;
+            for (int a = 0; a < 3; a++)
+                if (i[a] == 0 || i[a] == n[a]) bd[q] *= 0.5f;
+        }
+    }
+    void node(long long q, int i[3]) const {
+        i[0] = (int)(q % (n[0] + 1));
+        i[1] = (int)(q / (n[0] + 1) % (n[1] + 1));
+        i[2] = (int)(q / ((long long)(n[0] + 1) * (n[1] + 1)));
+    }
+    template <class T>
+    void product(const T *c, const std::vector<T> &v, std::vector<T> &y) const {
+        y.resize(nn);
+        for (long long q = 0; q < nn; q++) {
+            int i[3];
+            node(q, i);
+            T s = T(0);
+            for (int k = 0; k < 27; k++) {
+                int d[3] = {k % 3 - 1, k / 3 % 3 - 1, k / 9 - 1}, S = 0;
+                for (int a = 0; a < 3; a++) {
+                    if (d[a]) S |= 1 << a;
+                    d[a] += i[a];
+                    d[a] = d[a] < 0 ? 1 : (d[a] > n[a] ? n[a] - 1 : d[a]);  // mirrored
+                }
+                s += c[S] * v[d[0] + (long long)(n[0] + 1) * (d[1] + (long long)(n[1] + 1) * d[2])];
+            }
+            y[q] = (T)bd[q] * s;
+        }
+    }
+    void rhs(const std::vector<double> &x) {
+        b.assign(nn, 0.0);
+        for (int e = 0; e < n[0] * n[1] * n[2]; e++)
+            for (int L = 0; L < 8; L++)
+                b[e % n[0] + (L & 1) + (long long)(n[0] + 1) * (e / n[0] % n[1] + (L >> 1 & 1) +
+                  (long long)(n[1] + 1) * (e / (n[0] * n[1]) + (L >> 2)))] += 0.125 * x[e];
+    }
+    static double dot(const std::vector<double> &a, const std::vector<double> &b) {
+        double s = 0.0;
+        for (size_t q = 0; q < a.size(); q++) s += a[q] * b[q];
+        return s;
+    }
+    static float dot(const std::vector<float> &a, const std::vector<float> &b) {
+        double s = 0.0;
+        for (size_t q = 0; q < a.size(); q++) s += (double)a[q] * b[q];
+        return (float)s;
+    }
+    Result solve(const std::vector<double> &x, double tol, int maxit) {
+        rhs(x);
+        u.assign(nn, 0.0);
+        r = b;
+        FiltRhs q{};
+        Result out{TOPO_OK, 0, 0, 0.0};
+        q.bb = q.rr = dot(b, b);
+        q.done = q.bb == 0.0;
+        std::vector<float> r32(nn), z(nn), w, s(nn), p(nn), d(nn);
+        std::vector<double> y;
+        const float dinv = 1.0f / c32[0];
+        while (out.status == TOPO_OK && !q.done) {
+            if (++out.corrections > 10000) return out;
+            q.rms = std::sqrt(q.rr / (double)nn);
+            for (long long k = 0; k < nn; k++) {
+                r32[k] = (float)(r[k] * (1.0 / q.rms));
+                z[k] = dinv / bd[k] * r32[k];
+                d[k] = 0.0f;
+            }
+            product(c32, z, w);
+            filt_begin(q, dot(r32, z), dot(w, z), tol, nn);
+            for (int it = 0; it < FILT_CAP && !q.idle && out.its < maxit; it++, out.its++) {
+                for (long long k = 0; k < nn; k++) {
+                    s[k] = q.beta == 0.0f ? w[k] : w[k] + q.beta * s[k];
+                    p[k] = q.beta == 0.0f ? z[k] : z[k] + q.beta * p[k];
+                    r32[k] -= q.alpha * s[k];
+                    d[k] += q.alpha * p[k];
+                }
+                for (long long k = 0; k < nn; k++) z[k] = dinv / bd[k] * r32[k];
+                product(c32, z, w);
+                const float t[3] = {dot(r32, z), dot(w, z), dot(r32, r32)};
+                filt_advance(q, t);
+            }
+            for (long long k = 0; k < nn; k++) u[k] += q.rms * (double)d[k];
+            product(c64, u, y);
+            for (long long k = 0; k < nn; k++) r[k] = b[k] - y[k];
+            out.status = filt_judge(q, dot(r, r), tol, out.its, maxit);
+        }
+        out.residual = q.bb > 0.0 ? std::sqrt(q.rr / q.bb) : 0.0;
+        return out;
+    }
+};
+
+static std::vector<double> field(int n, int kind, double scale) {
+    std::vector<double> x(n);
+    unsigned long long s = 88172645463325252ull;
+    for (double &v : x) {
+        s ^= s << 13, s ^= s >> 7, s ^= s << 17;
+        v = scale * (kind ? (double)(s >> 11) / 9007199254740992.0 : 1.0);
+    }
+    return x;
+}
+
+int main() {
+    int bad = 0;
+    auto run = [&](double rmin, int kind, double scale, double tol, int maxit) {
+        Model m(16, 8, 8, rmin);
+        const Result o = m.solve(field(16 * 8 * 8, kind, scale), tol, maxit);
+        printf("rmin %g, %s field of %g, rtol %g: status %d, %d iterations, %d corrections, residual %.1e\n", rmin,
+               kind ? "random" : "uniform", scale, tol, o.status, o.its, o.corrections, o.residual);
+        return o;
+    };
+    auto want = [&](bool ok, const char *what) {
+        if (!ok) printf("  NOT OK: %s\n", what), bad = 1;
+    };
+    // every call returns, and says that it is solved only when the residual says so
+    for (double rmin : {2.0, 1e5, 1e12, 1e25})
+        for (int kind : {0, 1})
+            for (double scale : {1.0, 1e-161, 1e150}) {
+                const Result o = run(rmin, kind, scale, 1e-10, 5000);
+                want(o.corrections < 100, "the corrections do not end");
+                want(o.status != TOPO_OK || o.residual <= 1e-10, "reported as solved");
+            }
+    want(run(2.0, 1, 1.0, 1e-10, 5000).status == TOPO_OK, "default radius");
+    want(run(2.0, 1, 1.0, 1e-10, 3).status == TOPO_ERR_NOT_CONVERGED, "iteration limit");
+    if (!bad) printf("control OK\n");
+    return bad;
+}

@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "coop.cuh"
+#include "filtctl.cuh"
 #include "filter.h"
 #include "kernels.cuh"
 #include "planes.cuh"
@@ -256,16 +257,10 @@ struct FiltResid {
 // is 3.1e-11 instead of 4.5e-11 from the exact one at rtol 1e-10.
 __global__ void __launch_bounds__(FT_N, 3) k_filt_solve(const FiltArgs A) {
     constexpr int NV = 3;
-    // scalars of a right-hand side, formed by one thread of every CTA alike
-    struct Rhs {
-        double bb, rr, rms;
-        float gam, alpha, beta, goal;
-        int done, idle;
-    };
     __shared__ __align__(16) FiltSmem sm;
     __shared__ double sred64[FT_N], stot64[FILT_RHS];
     __shared__ float sred[FILT_RHS][NV * FT_N / 32], stot[FILT_RHS * NV];
-    __shared__ Rhs R[FILT_RHS];
+    __shared__ FiltRhs R[FILT_RHS];
     __shared__ int s_status;
     const GridDesc g = A.g;
     const long long nn = g.nn(), nel = g.nel();
@@ -340,23 +335,10 @@ __global__ void __launch_bounds__(FT_N, 3) k_filt_solve(const FiltArgs A) {
             sums(r, f.sum);
         }
         if (!finish()) return;
-        if (threadIdx.x < FILT_RHS) {
-            const int r = threadIdx.x;
-            Rhs &q = R[r];
-            q.idle = q.done;
-            if (!q.done) {
-                q.gam = stot[NV * r];
-                q.beta = 0.0f;
-                q.alpha = q.gam / stot[NV * r + 1];
-                if (!(q.alpha > 0.0f) || !isfinite(q.alpha)) q.idle = 1;
-                // reduction asked of this correction: half of what is left to the
-                // tolerance, at most 1e-6 (what the FP32 recurrence holds)
-                const double left = fmax(1e-6, 0.5 * A.tol * sqrt(q.bb / q.rr));
-                q.goal = (float)(left * left * (double)nn);
-            }
-        }
+        if (threadIdx.x < FILT_RHS)
+            filt_begin(R[threadIdx.x], stot[NV * threadIdx.x], stot[NV * threadIdx.x + 1], A.tol, nn);
         __syncthreads();
-        for (int it = 0; it < 64 && !(R[0].idle && R[1].idle) && its < A.maxit; it++, its++) {
+        for (int it = 0; it < FILT_CAP && !(R[0].idle && R[1].idle) && its < A.maxit; it++, its++) {
             const int o = it & 1, w = o ^ 1;  // buffers read and written
             for (int r = 0; r < A.nr; r++) {
                 if (R[r].idle) continue;
@@ -366,15 +348,7 @@ __global__ void __launch_bounds__(FT_N, 3) k_filt_solve(const FiltArgs A) {
                 sums(r, f.sum);
             }
             if (!finish()) return;
-            if (threadIdx.x < A.nr && !R[threadIdx.x].idle) {
-                Rhs &q = R[threadIdx.x];
-                const float *t = stot + NV * threadIdx.x, be = t[0] / q.gam;
-                q.beta = be;
-                q.alpha = t[0] / (t[1] - be * t[0] / q.alpha);
-                q.gam = t[0];
-                // at the goal, or rounding has used the correction up
-                if (!(t[2] > q.goal) || !(q.alpha > 0.0f) || !isfinite(q.alpha)) q.idle = 1;
-            }
+            if (threadIdx.x < A.nr) filt_advance(R[threadIdx.x], stot + NV * threadIdx.x);
             __syncthreads();
         }
         // u += d / sigma (into the other buffer), r = b - K u, r.r
@@ -391,15 +365,8 @@ __global__ void __launch_bounds__(FT_N, 3) k_filt_solve(const FiltArgs A) {
         ub ^= 1;
         if (threadIdx.x == 0)
             for (int r = 0; r < A.nr; r++) {
-                Rhs &q = R[r];
-                if (q.done) continue;
-                const double s = stot64[r], was = q.rr;
-                q.rr = s;
-                if (!isfinite(s)) s_status = TOPO_ERR_NAN;
-                // a residual that a correction no longer halves, below 1e-12, is the
-                // rounding of b - K u: tolerances under it are met as far as FP64 goes
-                else if (s <= A.tol * A.tol * q.bb || (s > 0.25 * was && s <= 1e-24 * q.bb)) q.done = 1;
-                else if (its >= A.maxit) s_status = TOPO_ERR_NOT_CONVERGED;
+                const int st = filt_judge(R[r], stot64[r], A.tol, its, A.maxit);
+                if (st) s_status = st;
             }
         __syncthreads();
     }
@@ -505,17 +472,9 @@ int pdefilt_create(TopoPDEFilt **out, int nx, int ny, int nz, double hx, double 
             for (int L = 0; L < 8; L++) f->KF[L * 8 + col] = v[L];
         }
     }
-    {
-        const double m[2] = {4.0 / 6.0, 1.0 / 6.0}, k[2] = {2.0, -1.0};  // own node, a neighbour
-        const double rho[3] = {R * R / (hx * hx), R * R / (hy * hy), R * R / (hz * hz)};
-        for (int S = 0; S < 8; S++) {
-            const int b[3] = {S & 1, (S >> 1) & 1, S >> 2};
-            double c = m[b[0]] * m[b[1]] * m[b[2]];
-            for (int a = 0; a < 3; a++) c += rho[a] * k[b[a]] * m[b[(a + 1) % 3]] * m[b[(a + 2) % 3]];
-            f->args.Kd.c[S] = c;
-            f->args.Kf.c[S] = (float)c;
-        }
-    }
+    const double hh[3] = {hx, hy, hz};
+    filt_stencil(hh, R, f->args.Kd.c);
+    for (int S = 0; S < 8; S++) f->args.Kf.c[S] = (float)f->args.Kd.c[S];
     cudaError_t e = cudaStreamCreateWithFlags(&f->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) {
         set_error(std::string("cudaStreamCreate: ") + cudaGetErrorString(e));
