@@ -1,7 +1,8 @@
 """The control of the PDE filter's solve (csrc/filtctl.cuh) on the host:
 tests/cuda/filter_control_check.cu steps the solve in the kernel's arithmetic with
 the kernel's own scalars, for fields and radii from the usual ones to those that
-FP32 cannot represent, and checks that every solve ends."""
+FP32 cannot represent, and checks that every solve ends and that what CG in FP64
+alone solves is solved."""
 import os
 import shutil
 import subprocess
@@ -11,7 +12,7 @@ import pytest
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
-def test_every_solve_ends(tmp_path):
+def test_every_solve_ends_as_fp64_alone_would(tmp_path):
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not os.path.exists(nvcc):
         pytest.skip("nvcc not found")

@@ -24,12 +24,13 @@ struct FiltRhs {
     double bb, rr, rms;  // b.b, r.r of the FP64 residual, its root mean square
     float gam, alpha, beta, goal;
     int done, idle;  // solved; no further iteration of this correction
+    int hard;        // left to FP64 (FiltCg)
 };
 
 // first step of a correction from its sums r.z and w.z
 __host__ __device__ inline void filt_begin(FiltRhs &q, float rz, float wz, double tol, long long nn) {
-    q.idle = q.done;
-    if (q.done) return;
+    q.idle = q.done || q.hard;
+    if (q.idle) return;
     q.gam = rz;
     q.beta = 0.0f;
     q.alpha = rz / wz;
@@ -49,19 +50,42 @@ __host__ __device__ inline void filt_advance(FiltRhs &q, const float t[3]) {
     // at the goal, or rounding has used the correction up
     if (!(t[2] > q.goal) || !(q.alpha > 0.0f) || !isfinite(q.alpha)) q.idle = 1;
 }
-// after a correction, from the FP64 residual's r.r: status of the solve
-__host__ __device__ inline int filt_judge(FiltRhs &q, double rr, double tol, int its, int maxit) {
-    if (q.done) return TOPO_OK;
+// After a correction, from the FP64 residual's r.r.  A correction that does not
+// halve the residual is at what FP32, or b - K u itself, can resolve; the next one
+// would start where this one did.
+__host__ __device__ inline void filt_judge(FiltRhs &q, double rr, double tol, int its, int maxit) {
+    if (q.done || q.hard) return;
     const double was = q.rr;
     q.rr = rr;
-    if (!isfinite(rr)) return TOPO_ERR_NAN;
-    // a residual that a correction no longer halves, below 1e-12, is the
-    // rounding of b - K u: tolerances under it are met as far as FP64 goes
-    if (rr <= tol * tol * q.bb || (rr > 0.25 * was && rr <= 1e-24 * q.bb)) q.done = 1;
-    // a correction that leaves the residual where it was leaves the next one nothing
-    // else to start from: FP32 cannot solve this system, and `its` need not have moved
-    else if (its >= maxit || !(rr < was)) return TOPO_ERR_NOT_CONVERGED;
-    return TOPO_OK;
+    if (rr <= tol * tol * q.bb) q.done = 1;
+    else if (its >= maxit || !(rr <= 0.25 * was)) q.hard = 1;
+}
+
+// Jacobi CG in FP64 from u = 0, which has the last word on what FP32 leaves over:
+// it ends on its recurrence's residual or with the status of the solve
+struct FiltCg {
+    double rz, alpha, beta;
+    int it, done, status;
+};
+__host__ __device__ inline void filt_cg_begin(FiltCg &c, double rz) { c = FiltCg{rz, 0.0, 0.0, 0, 0, TOPO_OK}; }
+// after the product, from p.q
+__host__ __device__ inline void filt_cg_step(FiltCg &c, double pq) {
+    c.alpha = c.rz / pq;
+    if (!(pq > 0.0)) {
+        c.done = 1;
+        c.status = isfinite(pq) ? TOPO_ERR_BREAKDOWN : TOPO_ERR_NAN;
+    }
+}
+// after the update, from r.r and r.z
+__host__ __device__ inline void filt_cg_judge(FiltCg &c, double rr, double rz, double tol, double bb, int maxit) {
+    c.beta = rz / c.rz;
+    c.rz = rz;
+    c.it++;
+    c.done = 1;
+    if (!isfinite(rr)) c.status = TOPO_ERR_NAN;
+    else if (rr <= tol * tol * bb) c.status = TOPO_OK;
+    else if (c.it >= maxit) c.status = TOPO_ERR_NOT_CONVERGED;
+    else c.done = 0;
 }
 
 }  // namespace topo

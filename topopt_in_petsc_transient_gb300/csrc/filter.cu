@@ -60,7 +60,8 @@ struct FiltOp {
 };
 
 struct FiltStatus {
-    int status, it;
+    int status;
+    int hard, cur;  // bit r set for a right-hand side left to k_filt_cg; which u the others stand in
 };
 
 struct FiltArgs {
@@ -73,6 +74,7 @@ struct FiltArgs {
     int clamp;
     Projection proj;
     double *u[FILT_RHS][2], *b[FILT_RHS], *r[FILT_RHS];
+    double *q[FILT_RHS];                // k_filt_cg: K p, in the storage of r32
     float *r32[FILT_RHS][2], *s32[FILT_RHS][2], *w32[FILT_RHS][2], *p32[FILT_RHS], *d32[FILT_RHS];
     double tol;
     int maxit;
@@ -242,6 +244,41 @@ struct FiltResid {
     }
 };
 
+// K p of k_filt_cg
+struct FiltMul {
+    const double *p;
+    double *q, sum;
+    struct Own {};
+    __device__ void copy(unsigned char *ring, int v, unsigned n) const { filt_copy<8>((double *)ring + v, p + n); }
+    __device__ double val(const unsigned char *ring, int v, float) const { return ((const double *)ring)[v]; }
+    __device__ Own own(unsigned) const { return {}; }
+    __device__ void put(unsigned n, float bd, Own, double v, double y) {
+        const double qv = (double)bd * y;
+        q[n] = qv;
+        sum += v * qv;
+    }
+};
+
+// xout = T^t u; optional clamp to [0,1] and smoothed Heaviside projection
+// (Filter.cc:83-113, Filter.h:80-83)
+__device__ __forceinline__ void filt_out(const FiltArgs &A, int r, const double *u) {
+    const GridDesc &g = A.g;
+    for (long long e = blockIdx.x * (long long)FT_N + threadIdx.x; e < g.nel(); e += (long long)gridDim.x * FT_N) {
+        int i, j, k;
+        lex3(e, g.ex, g.ey, i, j, k);
+        double acc = 0.0;
+        for (int L = 0; L < 8; L++)
+            acc += u[(i + (L & 1)) + (long long)g.nx * ((j + ((L >> 1) & 1)) + (long long)g.ny * (k + (L >> 2)))];
+        acc *= 0.125;
+        if (A.clamp) {
+            if (acc < 0.0) acc = 0.0;
+            if (acc > 1.0) acc = 1.0;
+        }
+        A.xout[r][e] = acc;
+        if (A.xphys) A.xphys[e] = project(A.proj, acc);
+    }
+}
+
 // One or two filter solves: u = K^-1 (T x), then T^t u (and the projection).
 // FP64 iterative refinement: the residual b - K u and u in FP64, each
 // correction by Jacobi CG in FP32 on the residual scaled to unit mean square
@@ -255,6 +292,9 @@ struct FiltResid {
 // 2.6 ms at 192x96x96 and 0.35 ms at 48x24x24, against 13.7 and 1.49 ms of FP64 CG
 // with three launches an iteration and 64 FP64 multiply-adds a node; the result
 // is 3.1e-11 instead of 4.5e-11 from the exact one at rtol 1e-10.
+// A correction gains a factor of about 1e6 h^2 / R^2, and b - K u resolves about
+// 1e-17 R^2 / h^2 of b: what this leaves over (radii of hundreds of elements,
+// tolerances of 1e-12 and less with tens) is left to k_filt_cg.
 __global__ void __launch_bounds__(FT_N, 3) k_filt_solve(const FiltArgs A) {
     constexpr int NV = 3;
     __shared__ __align__(16) FiltSmem sm;
@@ -263,7 +303,7 @@ __global__ void __launch_bounds__(FT_N, 3) k_filt_solve(const FiltArgs A) {
     __shared__ FiltRhs R[FILT_RHS];
     __shared__ int s_status;
     const GridDesc g = A.g;
-    const long long nn = g.nn(), nel = g.nel();
+    const long long nn = g.nn();
     const long long t0 = blockIdx.x * (long long)FT_N + threadIdx.x, ts = (long long)gridDim.x * FT_N;
     unsigned arrivals = 0;
     int slot = 0;
@@ -316,6 +356,7 @@ __global__ void __launch_bounds__(FT_N, 3) k_filt_solve(const FiltArgs A) {
         s_status = TOPO_OK;
         for (int r = 0; r < FILT_RHS; r++) {
             R[r].done = 1;
+            R[r].hard = 0;
             if (r >= A.nr) continue;
             R[r].bb = R[r].rr = stot64[r];
             R[r].done = stot64[r] == 0.0;
@@ -324,12 +365,13 @@ __global__ void __launch_bounds__(FT_N, 3) k_filt_solve(const FiltArgs A) {
     }
     __syncthreads();
     int its = 0, ub = 0;  // ub: which u is current
-    while (s_status == TOPO_OK && !(R[0].done && R[1].done)) {
-        if (threadIdx.x < FILT_RHS && !R[threadIdx.x].done) R[threadIdx.x].rms = sqrt(R[threadIdx.x].rr / (double)nn);
+    auto out = [&](int r) { return R[r].done || R[r].hard; };
+    while (s_status == TOPO_OK && !(out(0) && out(1))) {
+        if (threadIdx.x < FILT_RHS && !out(threadIdx.x)) R[threadIdx.x].rms = sqrt(R[threadIdx.x].rr / (double)nn);
         __syncthreads();
         // r32 = r / rms(r), z, w = K z, correction 0
         for (int r = 0; r < A.nr; r++) {
-            if (R[r].done) continue;
+            if (out(r)) continue;
             FiltStart f{A.r[r], scale_split(1.0 / R[r].rms), dinv, A.r32[r][0], A.w32[r][0], A.d32[r], {}};
             filt_apply<float>(A, A.Kf, sm, f);
             sums(r, f.sum);
@@ -357,48 +399,105 @@ __global__ void __launch_bounds__(FT_N, 3) k_filt_solve(const FiltArgs A) {
                 for (long long n = t0; n < nn; n += ts) A.u[r][ub ^ 1][n] = A.u[r][ub][n];
                 continue;
             }
+            if (R[r].hard) continue;
             FiltResid f{A.u[r][ub], A.b[r], A.d32[r], R[r].rms, A.u[r][ub ^ 1], A.r[r], 0.0};
             filt_apply<double>(A, A.Kd, sm, f);
             sum64(r, f.sum);
         }
         if (!finish64()) return;
         ub ^= 1;
-        if (threadIdx.x == 0)
-            for (int r = 0; r < A.nr; r++) {
-                const int st = filt_judge(R[r], stot64[r], A.tol, its, A.maxit);
-                if (st) s_status = st;
-            }
+        if (threadIdx.x < A.nr) filt_judge(R[threadIdx.x], stot64[threadIdx.x], A.tol, its, A.maxit);
         __syncthreads();
     }
     const int status = s_status;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         A.out->status = status;
-        A.out->it = its;
+        A.out->hard = (R[0].hard ? 1 : 0) | (R[1].hard ? 2 : 0);
+        A.out->cur = ub;
         __threadfence_system();
     }
-    if (status == TOPO_OK) {
-        // xout = T^t u; optional clamp to [0,1] and smoothed Heaviside projection
-        // (Filter.cc:83-113, Filter.h:80-83)
-        for (int r = 0; r < A.nr; r++) {
-            const double *u = A.u[r][ub];
-            for (long long e = t0; e < nel; e += ts) {
-                int i, j, k;
-                lex3(e, g.ex, g.ey, i, j, k);
-                double acc = 0.0;
-                for (int L = 0; L < 8; L++)
-                    acc += u[(i + (L & 1)) + (long long)g.nx * ((j + ((L >> 1) & 1)) + (long long)g.ny * (k + (L >> 2)))];
-                acc *= 0.125;
-                if (A.clamp) {
-                    if (acc < 0.0) acc = 0.0;
-                    if (acc > 1.0) acc = 1.0;
-                }
-                A.xout[r][e] = acc;
-                if (A.xphys) A.xphys[e] = project(A.proj, acc);
-            }
-        }
+    if (status == TOPO_OK && !R[0].hard && !R[1].hard) {
+        for (int r = 0; r < A.nr; r++) filt_out(A, r, A.u[r][ub]);
     }
     grid_leave(A.bar);
 }
+
+// Jacobi CG in FP64 on right-hand side r, whose b = T x stands in A.b[r], from u = 0:
+// the product, the update and the direction in turn, a grid barrier after each.  A
+// kernel of its own: within k_filt_solve it cost that one 5% in registers.
+__global__ void __launch_bounds__(FT_N, 3) k_filt_cg(const FiltArgs A, int r) {
+    __shared__ __align__(16) FiltSmem sm;
+    __shared__ double sred[FT_N], stot[2], bb;
+    __shared__ FiltCg cg;
+    const GridDesc g = A.g;
+    const long long nn = g.nn(), t0 = blockIdx.x * (long long)FT_N + threadIdx.x, ts = (long long)gridDim.x * FT_N;
+    unsigned arrivals = 0;
+    int slot = 0;
+    auto reduce = [&](double v0, double v1) {  // grid sums into stot
+        double *part = A.part + (size_t)slot * 2 * gridDim.x;
+        cta_sums<FT_N, 1>(&v0, sred, part + blockIdx.x, gridDim.x);
+        __syncthreads();
+        cta_sums<FT_N, 1>(&v1, sred, part + gridDim.x + blockIdx.x, gridDim.x);
+        if (!grid_sync(A.bar, arrivals)) return false;
+        grid_totals<FT_N>(part, 2, stot);
+        slot ^= 1;
+        return true;
+    };
+    const double dinv = 1.0 / A.Kd.c[0];
+    auto prec = [&](long long n, double v) {  // Dinv v
+        int i, j, k;
+        lex3(n, g.nx, g.ny, i, j, k);
+        const int ends = (i == 0 || i == g.nx - 1) + (j == 0 || j == g.ny - 1) + (k == 0 || k == g.nz - 1);
+        return v * (dinv * (double)(1 << ends));
+    };
+    double *x = A.u[r][0], *p = A.u[r][1], *res = A.r[r], *q = A.q[r];
+    double s0 = 0.0, s1 = 0.0;
+    for (long long n = t0; n < nn; n += ts) {
+        const double b = A.b[r][n], z = prec(n, b);
+        x[n] = 0.0;
+        res[n] = b;
+        p[n] = z;
+        s0 += b * b;
+        s1 += b * z;
+    }
+    if (!reduce(s0, s1)) return;
+    if (threadIdx.x == 0) {
+        bb = stot[0];
+        filt_cg_begin(cg, stot[1]);
+    }
+    __syncthreads();
+    for (;;) {
+        FiltMul f{p, q, 0.0};
+        filt_apply<double>(A, A.Kd, sm, f);
+        if (!reduce(f.sum, 0.0)) return;
+        if (threadIdx.x == 0) filt_cg_step(cg, stot[0]);
+        __syncthreads();
+        if (cg.done) break;
+        const double al = cg.alpha;
+        s0 = s1 = 0.0;
+        for (long long n = t0; n < nn; n += ts) {
+            x[n] += al * p[n];
+            const double v = res[n] - al * q[n];
+            res[n] = v;
+            s0 += v * v;
+            s1 += v * prec(n, v);
+        }
+        if (!reduce(s0, s1)) return;
+        if (threadIdx.x == 0) filt_cg_judge(cg, stot[0], stot[1], A.tol, bb, A.maxit);
+        __syncthreads();
+        if (cg.done) break;
+        const double be = cg.beta;
+        for (long long n = t0; n < nn; n += ts) p[n] = prec(n, res[n]) + be * p[n];
+        if (!grid_sync(A.bar, arrivals)) return;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        A.out->status = cg.status;
+        __threadfence_system();
+    }
+    grid_leave(A.bar);
+}
+
+static __global__ void k_filt_out(const FiltArgs A, int r, const double *u) { filt_out(A, r, u); }
 
 struct TopoPDEFilt {
     GridDesc g;
@@ -491,9 +590,9 @@ int pdefilt_create(TopoPDEFilt **out, int nx, int ny, int nz, double hx, double 
     for (int r = 0; r < FILT_RHS; r++) {
         for (int k = 0; k < 2; k++) {
             get(&A.u[r][k], nn);
-            for (float **q : {&A.r32[r][k], &A.s32[r][k], &A.w32[r][k]}) get(q, nn);
+            for (float **q : {&A.s32[r][k], &A.w32[r][k]}) get(q, nn);
         }
-        for (double **q : {&A.b[r], &A.r[r]}) get(q, nn);
+        for (double **q : {&A.b[r], &A.r[r], &A.q[r]}) get(q, nn);
         for (float **q : {&A.p32[r], &A.d32[r]}) get(q, nn);
     }
     get(&f->mnd, 1);
@@ -513,6 +612,10 @@ int pdefilt_create(TopoPDEFilt **out, int nx, int ny, int nz, double hx, double 
             *w.first = mem;
             mem += (w.second + 255) / 256 * 256;
         }
+        for (int r = 0; r < FILT_RHS; r++) {
+            A.r32[r][0] = (float *)A.q[r];
+            A.r32[r][1] = A.r32[r][0] + nn;
+        }
     }
     if (rc) {
         pdefilt_destroy(f);
@@ -521,17 +624,18 @@ int pdefilt_create(TopoPDEFilt **out, int nx, int ny, int nz, double hx, double 
     e = cudaHostAlloc((void **)&f->status, sizeof(FiltStatus), cudaHostAllocMapped);
     if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&A.out, f->status, 0);
     // resident CTAs, and runs of planes that give each about one: a run reads two planes more than it completes
-    int dev = 0, nsm = 0, per_sm = 0;
+    int dev = 0, nsm = 0, per_sm = 0, per_cg = 0;
     if (e == cudaSuccess) e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_filt_solve, FT_N, 0);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_cg, k_filt_cg, FT_N, 0);
     if (e == cudaSuccess) e = cudaStreamSynchronize(f->stream);
-    if (e != cudaSuccess || per_sm < 1) {
+    if (e != cudaSuccess || per_sm < 1 || per_cg < 1) {
         set_error(std::string("PDE filter setup: ") + cudaGetErrorString(e));
         pdefilt_destroy(f);
         return TOPO_ERR_CUDA;
     }
-    const int resident = per_sm * nsm;
+    const int resident = std::min(per_sm, per_cg) * nsm;
     const Patch pt = plane_patch(nx, ny, FT_N, 1, FT_PLANE);
     A.tx = pt.tx;
     A.ty = pt.ty;
@@ -574,12 +678,28 @@ static int filt_solve(TopoPDEFilt *f, int nr, const double *const *xin, double *
     A.xphys = xphys;
     A.clamp = clamp;
     A.proj = make_projection(projection, beta, eta);
-    f->status->status = TOPO_ERR_CUDA;
+    auto launch = [&](const void *kernel, void **args) -> int {
+        f->status->status = TOPO_ERR_CUDA;
+        count_launch();
+        FCK(cudaLaunchCooperativeKernel(kernel, dim3(f->grid), dim3(FT_N), args, 0, s));
+        FCK(cudaStreamSynchronize(s));
+        return *(volatile int *)&f->status->status;
+    };
     void *args[] = {&A};
-    count_launch();
-    FCK(cudaLaunchCooperativeKernel((const void *)k_filt_solve, dim3(f->grid), dim3(FT_N), args, 0, s));
-    FCK(cudaStreamSynchronize(s));
-    const int st = *(volatile int *)&f->status->status;
+    int st = launch((const void *)k_filt_solve, args);
+    const int hard = f->status->hard, cur = f->status->cur;
+    if (st == TOPO_OK && hard) {
+        for (int r = 0; r < nr && st == TOPO_OK; r++) {
+            void *cargs[] = {&A, &r};
+            if ((hard >> r) & 1) st = launch((const void *)k_filt_cg, cargs);
+        }
+        for (int r = 0; r < nr && st == TOPO_OK; r++) {  // no result before all are solved
+            count_launch();
+            k_filt_out<<<f->grid, FT_N, 0, s>>>(A, r, A.u[r][(hard >> r) & 1 ? 0 : cur]);
+        }
+        FCK(cudaGetLastError());
+        FCK(cudaStreamSynchronize(s));
+    }
     if (st == TOPO_OK) return TOPO_OK;
     if (st == TOPO_ERR_CUDA) {  // the grid barrier gave up
         FCK(cudaMemsetAsync(f->counter + 1, 0, 3 * sizeof(unsigned), s));
