@@ -7,8 +7,6 @@
 
 namespace topo {
 
-constexpr int FILT_CAP = 64;  // iterations of a correction
-
 // weights of A (FiltOp, filter.cu) for element edges h and length scale R: c[S] of a
 // neighbour displaced along the axes in S
 inline void filt_stencil(const double h[3], double R, double c[8]) {
