@@ -107,7 +107,7 @@ struct Model {
         Result out{TOPO_OK, 0, 0};
         q.bb = q.rr = dot(b, b);
         q.done = q.bb == 0.0;
-        q.hard = fp64 && !q.done;
+        q.hard = (fp64 || filt_in_fp64(h, R, tol)) && !q.done;
         std::vector<float> r32(nn), z(nn), w, s(nn), p(nn), d(nn);
         std::vector<double> y;
         const float dinv = 1.0f / c32[0];
@@ -171,6 +171,14 @@ int main() {
                                f.status, f.its);
                         bad = 1;
                     }
+    // where the corrections come first, what they spend without solving stays below five CG solves
+    for (double rmin : {64.0, 256.0, 900.0, 2048.0})
+        for (double tol : {1e-10, 1e-12, 1e-13}) {
+            Model m(16, 8, 8, rmin);
+            const std::vector<double> x = field(16 * 8 * 8, 1, 1.0);
+            const Result f = m.solve(x, tol, 5000, true), o = m.solve(x, tol, 5000);
+            if (o.its > 6 * f.its) printf("rmin %g, rtol %g: %d iterations, FP64 alone %d\n", rmin, tol, o.its, f.its), bad = 1;
+        }
     // at 128 h three corrections reach 1e-10, none of which is asked for as much as the
     // whole of the FP64 solve
     {

@@ -18,6 +18,18 @@ inline void filt_stencil(const double h[3], double R, double c[8]) {
     }
 }
 
+// FP64 from the start?  rho = max_a (R / h_a)^2 is the size of K's entries against
+// its row sums.  A correction gains a factor of about 1e6 / rho, and b - K u resolves
+// about 3e-16 rho of b, so past either line the corrections only come before the CG
+// that they leave the solve to.  Measured, corrections against FP64 CG at rtol 1e-10:
+// rho = 2e4 (512 elements) 3.0 against 2.7 ms at 48x24x24, 9.6 : 12.2 at 96x48x48 and
+// 47 : 85 at 192x96x96; rho = 8e4 3.2 : 2.8, 11.9 : 12.8 and 58 : 88; at 3.5e5 they
+// end unsolved after 1500 iterations.
+inline bool filt_in_fp64(const double h[3], double R, double tol) {
+    const double hm = fmin(h[0], fmin(h[1], h[2])), rho = R / hm * (R / hm);
+    return rho > fmin(1e5, 1e15 * fabs(tol));
+}
+
 struct FiltRhs {
     double bb, rr, rms;  // b.b, r.r of the FP64 residual, its root mean square
     float gam, alpha, beta, goal;

@@ -77,7 +77,7 @@ struct FiltArgs {
     double *q[FILT_RHS];                // k_filt_cg: K p, in the storage of r32
     float *r32[FILT_RHS][2], *s32[FILT_RHS][2], *w32[FILT_RHS][2], *p32[FILT_RHS], *d32[FILT_RHS];
     double tol;
-    int maxit;
+    int maxit, fp64;                    // fp64: no corrections (filt_in_fp64)
     double *part;                       // [2 slots][FILT_RHS][gridDim] FP64 sums, then [2][FILT_RHS][3][gridDim] FP32 ones
     GridBar bar;
     FiltStatus *out;                    // mapped host memory
@@ -292,9 +292,7 @@ __device__ __forceinline__ void filt_out(const FiltArgs &A, int r, const double 
 // 2.6 ms at 192x96x96 and 0.35 ms at 48x24x24, against 13.7 and 1.49 ms of FP64 CG
 // with three launches an iteration and 64 FP64 multiply-adds a node; the result
 // is 3.1e-11 instead of 4.5e-11 from the exact one at rtol 1e-10.
-// A correction gains a factor of about 1e6 h^2 / R^2, and b - K u resolves about
-// 1e-17 R^2 / h^2 of b: what this leaves over (radii of hundreds of elements,
-// tolerances of 1e-12 and less with tens) is left to k_filt_cg.
+// What corrections cannot solve is left to k_filt_cg (filt_in_fp64, filt_judge).
 __global__ void __launch_bounds__(FT_N, 3) k_filt_solve(const FiltArgs A) {
     constexpr int NV = 3;
     __shared__ __align__(16) FiltSmem sm;
@@ -360,6 +358,7 @@ __global__ void __launch_bounds__(FT_N, 3) k_filt_solve(const FiltArgs A) {
             if (r >= A.nr) continue;
             R[r].bb = R[r].rr = stot64[r];
             R[r].done = stot64[r] == 0.0;
+            R[r].hard = A.fp64 && !R[r].done;
             if (!isfinite(stot64[r])) s_status = TOPO_ERR_NAN;
         }
     }
@@ -649,6 +648,7 @@ int pdefilt_create(TopoPDEFilt **out, int nx, int ny, int nz, double hx, double 
     f->grid = (unsigned)std::min(resident, A.ntx * A.nty * A.ncz);
     A.tol = rtol;
     A.maxit = maxit;
+    A.fp64 = filt_in_fp64(hh, R, rtol);
     A.part = f->part;
     A.bar = GridBar{f->counter + 1, f->counter + 2, f->counter + 3};
     *out = f;
