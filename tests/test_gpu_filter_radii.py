@@ -71,3 +71,27 @@ def test_iteration_limit_counts_fp64_iterations(gpu):
     _check(out, n, 32.0, 1e-10, x)
     with pytest.raises(_lib.TopoError):
         PDEFilt(*n, 32.0, maxit=60).FilterProject(x, out)
+
+
+@pytest.mark.parametrize("h,scale", [(1.0, 1.0), (1e-3, 1e155), (1e-3, 1e-140), (1e3, 1e-160), (1e3, 1e140)])
+def test_range_of_fields(gpu, h, scale):
+    """|b| with the element volume in T, V |T x|, is from 1e-150 to 1e148 here."""
+    from topopt_in_petsc_transient_gb300 import PDEFilt
+    n, x = (16, 8, 8), np.random.default_rng(5).random(16 * 8 * 8)
+    out = np.zeros(x.size)
+    PDEFilt(*n, 2.0 * h, h=(h, h, h)).FilterProject(scale * x, out)
+    _check(out / scale, n, 2.0, 1e-10, x)
+
+
+@pytest.mark.parametrize("scale", [1e-157, 1e-161, 1e-165])
+def test_fields_that_underflow_end(gpu, scale):
+    """Sums of squares below FP64's range: an error or a result, and the filter works on."""
+    from topopt_in_petsc_transient_gb300 import PDEFilt, _lib
+    n, x = (16, 8, 8), np.random.default_rng(5).random(16 * 8 * 8)
+    f, out = PDEFilt(*n, 2.0), np.zeros(x.size)
+    try:
+        f.FilterProject(scale * x, out)
+    except _lib.TopoError:
+        pass
+    f.FilterProject(x, out)
+    _check(out, n, 2.0, 1e-10, x)

@@ -76,6 +76,9 @@ struct FiltArgs {
     double *u[FILT_RHS][2], *b[FILT_RHS], *r[FILT_RHS];
     double *q[FILT_RHS];                // k_filt_cg: K p, in the storage of r32
     float *r32[FILT_RHS][2], *s32[FILT_RHS][2], *w32[FILT_RHS][2], *p32[FILT_RHS], *d32[FILT_RHS];
+    // b and u are those of the element volume's power of two times the fields, so that
+    // b.b keeps the range that it has with K and T of volume V
+    double sb, sx;                      // T and T^t: an eighth times it, an eighth over it
     double tol;
     int maxit, fp64;                    // fp64: no corrections (filt_in_fp64)
     double *part;                       // [2 slots][FILT_RHS][gridDim] FP64 sums, then [2][FILT_RHS][3][gridDim] FP32 ones
@@ -269,7 +272,7 @@ __device__ __forceinline__ void filt_out(const FiltArgs &A, int r, const double 
         double acc = 0.0;
         for (int L = 0; L < 8; L++)
             acc += u[(i + (L & 1)) + (long long)g.nx * ((j + ((L >> 1) & 1)) + (long long)g.ny * (k + (L >> 2)))];
-        acc *= 0.125;
+        acc *= A.sx;
         if (A.clamp) {
             if (acc < 0.0) acc = 0.0;
             if (acc > 1.0) acc = 1.0;
@@ -341,7 +344,7 @@ __global__ void __launch_bounds__(FT_N, 3) k_filt_solve(const FiltArgs A) {
                 if (ei < 0 || ej < 0 || ek < 0 || ei >= g.ex || ej >= g.ey || ek >= g.ez) continue;
                 acc += A.xin[r][ei + (long long)g.ex * (ej + (long long)g.ey * ek)];
             }
-            acc *= 0.125;
+            acc *= A.sb;
             A.b[r][n] = acc;
             A.r[r][n] = acc;
             A.u[r][0][n] = 0.0;
@@ -646,6 +649,9 @@ int pdefilt_create(TopoPDEFilt **out, int nx, int ny, int nz, double hx, double 
     A.cz = (nz + runs - 1) / runs;
     A.ncz = (nz + A.cz - 1) / A.cz;
     f->grid = (unsigned)std::min(resident, A.ntx * A.nty * A.ncz);
+    const int ve = std::max(-1000, std::min(1000, std::ilogb(hx * hy * hz)));
+    A.sb = std::ldexp(0.125, ve);
+    A.sx = std::ldexp(0.125, -ve);
     A.tol = rtol;
     A.maxit = maxit;
     A.fp64 = filt_in_fp64(hh, R, rtol);
