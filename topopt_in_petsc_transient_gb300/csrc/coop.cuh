@@ -3,7 +3,9 @@
 // Iterations whose kernels are shorter than a launch run as one cooperative
 // kernel whose CTAs (all resident, cudaLaunchCooperativeKernel) meet at a
 // counter in global memory.  Every wait is bounded: a CTA that gives up sets
-// `fail`, on which every other CTA leaves too, and the host reads it.
+// `fail`, on which every other CTA that still waits leaves too.  The status of the
+// kernel is written by the last CTA to finish (grid_leave), so it is written only
+// if none gave up; otherwise the host sets the counters back.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -13,8 +15,8 @@ struct GridBar {
     unsigned *count;  // arrivals of this launch; zero between launches
     unsigned *left;   // CTAs that have finished; the last one zeroes both
     unsigned *fail;   // set by a CTA whose wait ran out
+    unsigned polls = 1u << 23;  // limit of a wait: some seconds
 };
-constexpr unsigned GRID_BAR_POLLS = 1u << 23;  // about a second
 
 __device__ __forceinline__ unsigned ld_poll(const unsigned *p) {
     unsigned v;
@@ -32,8 +34,8 @@ __device__ __forceinline__ bool grid_sync(const GridBar &b, unsigned &arrivals) 
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(b.count) : "memory");
         const unsigned target = arrivals * gridDim.x;
         unsigned polls = 0;
-        while (ld_poll(b.count) < target) {
-            if (++polls > GRID_BAR_POLLS || ((polls & 1023u) == 0 && ld_poll(b.fail))) {
+        while ((int)(ld_poll(b.count) - target) < 0) {  // both may wrap
+            if (++polls > b.polls || ((polls & 1023u) == 0 && ld_poll(b.fail))) {
                 atomicExch(b.fail, 1u);
                 ok = false;
                 break;
@@ -44,17 +46,17 @@ __device__ __forceinline__ bool grid_sync(const GridBar &b, unsigned &arrivals) 
     return __syncthreads_and(ok) != 0;
 }
 
-// the end of the kernel, every thread of every CTA: counters back to zero for
-// the next launch on the same stream
-__device__ __forceinline__ void grid_leave(const GridBar &b) {
-    if (threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd(b.left, 1u) == gridDim.x - 1) {
-            *b.count = 0u;
-            *b.left = 0u;
-            __threadfence();
-        }
-    }
+// the end of the kernel, every thread of every CTA: true in one thread of the last
+// CTA, once every CTA has come here; counters back to zero for the next launch on
+// the same stream
+__device__ __forceinline__ bool grid_leave(const GridBar &b) {
+    if (threadIdx.x != 0) return false;
+    __threadfence();
+    if (atomicAdd(b.left, 1u) != gridDim.x - 1) return false;
+    *b.count = 0u;
+    *b.left = 0u;
+    __threadfence();
+    return true;
 }
 
 // CTA sums of NV FP32 values per thread into out[v * stride], v = 0..NV-1.

@@ -414,16 +414,15 @@ __global__ void __launch_bounds__(FT_N, 3) k_filt_solve(const FiltArgs A) {
         __syncthreads();
     }
     const int status = s_status;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (status == TOPO_OK && !R[0].hard && !R[1].hard) {
+        for (int r = 0; r < A.nr; r++) filt_out(A, r, A.u[r][ub]);
+    }
+    if (grid_leave(A.bar)) {
         A.out->status = status;
         A.out->hard = (R[0].hard ? 1 : 0) | (R[1].hard ? 2 : 0);
         A.out->cur = ub;
         __threadfence_system();
     }
-    if (status == TOPO_OK && !R[0].hard && !R[1].hard) {
-        for (int r = 0; r < A.nr; r++) filt_out(A, r, A.u[r][ub]);
-    }
-    grid_leave(A.bar);
 }
 
 // Jacobi CG in FP64 on right-hand side r, whose b = T x stands in A.b[r], from u = 0:
@@ -494,11 +493,10 @@ __global__ void __launch_bounds__(FT_N, 3) k_filt_cg(const FiltArgs A, int r) {
         for (long long n = t0; n < nn; n += ts) p[n] = prec(n, res[n]) + be * p[n];
         if (!grid_sync(A.bar, arrivals)) return;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (grid_leave(A.bar)) {
         A.out->status = cg.status;
         __threadfence_system();
     }
-    grid_leave(A.bar);
 }
 
 static __global__ void k_filt_out(const FiltArgs A, int r, const double *u) { filt_out(A, r, u); }

@@ -359,10 +359,11 @@ static __global__ void __launch_bounds__(MMA_NT, 4) k_mma_update(const MMAArgs A
         W->z = D.z;
         W->epsi = D.epsi;
         W->err = D.err;
+    }
+    if (grid_leave(A.bar)) {
         *A.status = bad ? TOPO_ERR_NAN : TOPO_OK;
         __threadfence_system();
     }
-    grid_leave(A.bar);
 }
 
 __global__ void k_mma_movelimit(long long n, double Xmin, double Xmax, double movlim, const double *__restrict__ x,
