@@ -1158,7 +1158,7 @@ static T *vcycle(TopoLE *le, int o, int l, const T *b, VFuse *fz = nullptr) {
     if constexpr (std::is_same<T, float>::value) {
         int ntx, nty;
         const int nt = tile_count(lv.g, ntx, nty);
-        if (l > 0 && l == le->nlev - 2 && le->coarse_dense && op.depth == le->nlev && nu <= VT_SMOOTH &&
+        if (l > 0 && l == le->nlev - 2 && le->coarse_dense && op.depth == le->nlev && nu >= 1 && nu <= VT_SMOOTH &&
             nt <= vtail_ctas()) {
             Level &lc = le->L[l + 1];
             VW<T> wc = vw<T>(le, o, l + 1);
