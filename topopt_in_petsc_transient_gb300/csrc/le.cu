@@ -1045,28 +1045,28 @@ static bool brick_order(const TopoLE *le) { return le->fp64_solves && le->basis3
 // up to VT_CTAS
 static int vtail_ctas() {
     static int n_dev[MAX_DEVICES] = {};
-    int &n = n_dev[device_slot()];
-    if (!n) {
-        const int sm = (int)TileSmem<float, PolCheb<float>>::bytes;
-        cudaFuncSetAttribute(k_vtail, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-        cudaFuncSetAttribute(k_vtail, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        cudaLaunchConfig_t c = {};
-        c.blockDim = TILE_THREADS;
-        c.dynamicSmemBytes = sm;
-        for (n = VT_CTAS; n > 1; n /= 2) {
-            cudaLaunchAttribute at = {};
-            at.id = cudaLaunchAttributeClusterDimension;
-            at.val.clusterDim = {(unsigned)n, 1, 1};
-            c.gridDim = (unsigned)n;
-            c.attrs = &at;
-            c.numAttrs = 1;
-            int clusters = 0;
-            const cudaError_t e = cudaOccupancyMaxActiveClusters(&clusters, k_vtail, &c);
-            if (e == cudaSuccess && clusters > 0) break;
-            if (e != cudaSuccess) cudaGetLastError();  // a size that the device refuses
-        }
+    int &known = n_dev[device_slot()];
+    if (known) return known;
+    const int sm = (int)TileSmem<float, PolCheb<float>>::bytes;
+    cudaFuncSetAttribute(k_vtail, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    cudaFuncSetAttribute(k_vtail, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaLaunchConfig_t c = {};
+    c.blockDim = TILE_THREADS;
+    c.dynamicSmemBytes = sm;
+    int n = VT_CTAS;
+    for (; n > 1; n /= 2) {
+        cudaLaunchAttribute at = {};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim = {(unsigned)n, 1, 1};
+        c.gridDim = (unsigned)n;
+        c.attrs = &at;
+        c.numAttrs = 1;
+        int clusters = 0;
+        const cudaError_t e = cudaOccupancyMaxActiveClusters(&clusters, k_vtail, &c);
+        if (e == cudaSuccess && clusters > 0) break;
+        if (e != cudaSuccess) cudaGetLastError();  // a size that the device refuses
     }
-    return n;
+    return known = n;  // set once it holds: another thread may read it at any time
 }
 static void launch_vtail(const VTail &V, const ElemConst<float> &C, int bricks, cudaStream_t s) {
     unsigned ctas = 1;
