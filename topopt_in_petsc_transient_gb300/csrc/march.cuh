@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(MARCH_THREADS, Pol::M_IN == 1 ? 2 : 1)
             if (v >= nst) continue;
             double t[NIN];
             pol.mval(r[q], t);
-            const bool fx = (f[q] >> (slot[q] % 3)) & 1;  // a clamped value is staged as zero
+            const bool fx = (f[q] >> ((unsigned)slot[q] % 3u)) & 1;  // a clamped value is staged as zero (f is 0 outside)
 #pragma unroll
             for (int n = 0; n < NIN; n++) lay[n * nst + v] = fx ? 0.0 : t[n];
         }
