@@ -505,7 +505,6 @@ struct TopoPDEFilt {
     GridDesc g;
     double rtol;
     int maxit;
-    double KF[64];
     FiltArgs args;   // operator, buffers and layout of the launches
     unsigned grid;   // CTAs of k_filt_solve: as many as are resident at once, at most one per run
     double *mnd;
@@ -547,32 +546,6 @@ int pdefilt_create(TopoPDEFilt **out, int nx, int ny, int nz, double hx, double 
     const double R = rmin / 2.0 / sqrt(3.0);  // PDEFilter.cc:32
     f->rtol = rtol;
     f->maxit = maxit;
-    // KF = R^2 * Laplacian + mass of the box: mode-basis diagonal, mapped back
-    // to the reference local node order (PDEFilter.cc:485-578 gives the same
-    // matrix in closed form); FiltOp holds the same operator for the solve
-    {
-        const double w[2] = {0.25, 1.0 / 12.0};
-        double V = hx * hy * hz, g2[3] = {4.0 / (hx * hx), 4.0 / (hy * hy), 4.0 / (hz * hz)};
-        double dm[8];
-        for (int m = 0; m < 8; m++) {
-            double Wm = V * w[m & 1] * w[(m >> 1) & 1] * w[(m >> 2) & 1];
-            double lap = 0.0;
-            for (int a = 0; a < 3; a++)
-                if (m & (1 << a)) {
-                    int ms = m & ~(1 << a);
-                    lap += g2[a] * V * w[ms & 1] * w[(ms >> 1) & 1] * w[(ms >> 2) & 1];
-                }
-            dm[m] = R * R * lap + Wm;
-        }
-        for (int col = 0; col < 8; col++) {
-            double v[8] = {0};
-            v[col] = 1.0;
-            mode_fwd(v);
-            for (int m = 0; m < 8; m++) v[m] *= dm[m];
-            mode_bwd(v);
-            for (int L = 0; L < 8; L++) f->KF[L * 8 + col] = v[L];
-        }
-    }
     const double hh[3] = {hx, hy, hz};
     filt_stencil(hh, R, f->args.Kd.c);
     for (int S = 0; S < 8; S++) f->args.Kf.c[S] = (float)f->args.Kd.c[S];
@@ -668,7 +641,6 @@ void pdefilt_destroy(TopoPDEFilt *f) {
 }
 
 long long pdefilt_nel(const TopoPDEFilt *f) { return f->g.nel(); }
-const double *pdefilt_matrix(const TopoPDEFilt *f) { return f->KF; }
 
 // results of up to FILT_RHS element fields, in place allowed (every input is
 // read before the first result is written)

@@ -8,7 +8,6 @@ int pdefilt_create(TopoPDEFilt **out, int nx, int ny, int nz, double hx, double 
                    int maxit);
 void pdefilt_destroy(TopoPDEFilt *f);
 long long pdefilt_nel(const TopoPDEFilt *f);
-const double *pdefilt_matrix(const TopoPDEFilt *f);
 int pdefilt_apply_dev(TopoPDEFilt *f, const double *x_dev, double *xout_dev);
 int filter_project_dev(TopoPDEFilt *f, const double *x_dev, double *xTilde_dev, double *xPhys_dev, int projection,
                        double beta, double eta);
