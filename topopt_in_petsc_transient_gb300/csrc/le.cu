@@ -294,7 +294,7 @@ static void launch_march(const GridDesc &g, const ElemConst<double> &C, const Po
 // FP64 bricks of another shape, for operators without reductions (one CTA a brick)
 template <class Pol, int TL, int TZ>
 static void launch_brick_of(const GridDesc &g, const ElemConst<double> &C, const Pol &pol, cudaStream_t s) {
-    constexpr size_t sm = tile_smem_bytes<double, Pol, TL, TZ>();
+    constexpr size_t sm = tile_smem_bytes<double, TL, TZ>();
     static bool attr_dev[MAX_DEVICES] = {};
     bool &attr = attr_dev[device_slot()];
     if (!attr) {
@@ -1460,7 +1460,7 @@ static void fwd_rhs(TopoLE *le) {
     const LEParams &p = le->p;
     Level &l0 = le->L[0];
     const double *a = le->a;
-    PolRhsFwd<double> pr;
+    PolRhsFwd pr;
     memset(&pr, 0, sizeof(pr));
     pr.fixed = l0.fixed;
     pr.w = fine_weights<double>(le, true, true, nullptr, 1.0, 1.0);

@@ -89,7 +89,7 @@ __device__ __forceinline__ void init_finish(SolveScalars *S, const double t[2], 
 // ---------------------------------------------------------------------------
 template <class T>
 struct PolInitResid {
-    static constexpr int NIN = 1, NRED = 2;
+    static constexpr int NRED = 2;
     static constexpr bool HAS_K = true, HAS_M = true;
     const uint8_t *fixed;
     Weights<T> w;
@@ -100,11 +100,11 @@ struct PolInitResid {
     cudaGraphConditionalHandle cond;
     int has_cond;
     Partials<2> part;
-    __device__ void load(long long n, T v[1][3]) const {
-        v[0][0] = T(x[3 * n]);
-        v[0][1] = T(x[3 * n + 1]);
-        v[0][2] = T(x[3 * n + 2]);
-        mask3(fixed[n], v[0]);
+    __device__ void load(long long n, T v[3]) const {
+        v[0] = T(x[3 * n]);
+        v[1] = T(x[3 * n + 1]);
+        v[2] = T(x[3 * n + 2]);
+        mask3(fixed[n], v);
     }
     // FP64 form (march.cuh)
     static constexpr int M_SRC = 1, M_IN = 1;
@@ -131,7 +131,7 @@ struct PolInitResid {
 // ---------------------------------------------------------------------------
 template <class T>
 struct PolPQ {
-    static constexpr int NIN = 1, NRED = 1;
+    static constexpr int NRED = 1;
     static constexpr bool HAS_K = true, HAS_M = true;
     const uint8_t *fixed;
     Weights<T> w;
@@ -139,11 +139,11 @@ struct PolPQ {
     T *q;
     SolveScalars *S;
     Partials<1> part;
-    __device__ void load(long long n, T v[1][3]) const {
-        v[0][0] = p[3 * n];
-        v[0][1] = p[3 * n + 1];
-        v[0][2] = p[3 * n + 2];
-        mask3(fixed[n], v[0]);
+    __device__ void load(long long n, T v[3]) const {
+        v[0] = p[3 * n];
+        v[1] = p[3 * n + 1];
+        v[2] = p[3 * n + 2];
+        mask3(fixed[n], v);
     }
     // FP64 form (march.cuh)
     static constexpr int M_SRC = 1, M_IN = 1;
@@ -185,7 +185,7 @@ struct PolPQ32 {
     // p = z + beta p_prev (k_mfcg_p) done while staging: p_prev is read from
     // pb[it & 1] and the new p written to pb[(it + 1) & 1], so no CTA
     // overwrites a halo value another CTA still stages
-    static constexpr int NIN = 1, NRED = 1;
+    static constexpr int NRED = 1;
     static constexpr bool HAS_K = true, HAS_M = true;
     const uint8_t *fixed;
     Weights<float> w;
@@ -205,9 +205,9 @@ struct PolPQ32 {
         const float *pp = odd ? pb[1] : pb[0];  // a select: no local copy of pb
         for (int c = 0; c < 3; c++) v[c] = (beta == 0.0f) ? z[3 * n + c] : z[3 * n + c] + beta * pp[3 * n + c];
     }
-    __device__ void load(long long n, float v[1][3]) const {
-        pnew(n, v[0]);
-        mask3(fixed[n], v[0]);
+    __device__ void load(long long n, float v[3]) const {
+        pnew(n, v);
+        mask3(fixed[n], v);
     }
     __device__ void coef(long long e, float &ck, float &cm) const { w.get(e, ck, cm); }
     struct Pre {
@@ -279,7 +279,7 @@ __device__ __forceinline__ void replace_finish(SolveScalars *S, double rr, cudaG
 // reduction whose last CTA clears it.
 template <class T>
 struct PolReplace {
-    static constexpr int NIN = 1, NRED = 1;
+    static constexpr int NRED = 1;
     static constexpr bool HAS_K = true, HAS_M = true;
     const uint8_t *fixed;
     Weights<T> w;
@@ -291,20 +291,20 @@ struct PolReplace {
     int has_cond;
     Partials<1> part;
     __device__ bool skip() const { return S->need_replace == 0; }
-    __device__ void load(long long n, T v[1][3]) const {
-        v[0][0] = T(x[3 * n]);
-        v[0][1] = T(x[3 * n + 1]);
-        v[0][2] = T(x[3 * n + 2]);
-        mask3(fixed[n], v[0]);
+    __device__ void load(long long n, T v[3]) const {
+        v[0] = T(x[3 * n]);
+        v[1] = T(x[3 * n + 1]);
+        v[2] = T(x[3 * n + 2]);
+        mask3(fixed[n], v);
     }
     // asynchronous staging (tile.cuh): x and the clamp mask
     using Src = double;
     static constexpr int NSRC = 1;
     static constexpr bool MASK = true;
     __device__ const double *src(int) const { return x; }
-    __device__ void xform(const double raw[][3], uint8_t f, T v[1][3]) const {
-        for (int c = 0; c < 3; c++) v[0][c] = T(raw[0][c]);
-        mask3(f, v[0]);
+    __device__ void xform(const double raw[][3], uint8_t f, T v[3]) const {
+        for (int c = 0; c < 3; c++) v[c] = T(raw[0][c]);
+        mask3(f, v);
     }
     __device__ void coef(long long e, T &ck, T &cm) const { w.get(e, ck, cm); }
     struct Pre {
@@ -355,7 +355,7 @@ __device__ __forceinline__ void cheb_coeffs(const double *lohi, int k, T &c1, T 
 
 template <class T>
 struct PolCheb {
-    static constexpr int NIN = 1, NRED = 0;
+    static constexpr int NRED = 0;
     static constexpr bool HAS_K = true, HAS_M = true;
     const uint8_t *fixed;
     Weights<T> w;
@@ -364,11 +364,11 @@ struct PolCheb {
     const T *ctab;  // Chebyshev table [k][2] = (c1, c2), built once per design
     int k;
     Partials<1> part;
-    __device__ void load(long long n, T v[1][3]) const {
-        v[0][0] = x_in[3 * n];
-        v[0][1] = x_in[3 * n + 1];
-        v[0][2] = x_in[3 * n + 2];
-        mask3(fixed[n], v[0]);
+    __device__ void load(long long n, T v[3]) const {
+        v[0] = x_in[3 * n];
+        v[1] = x_in[3 * n + 1];
+        v[2] = x_in[3 * n + 2];
+        mask3(fixed[n], v);
     }
     // FP64 form (march.cuh)
     static constexpr int M_SRC = 1, M_IN = 1;
@@ -408,7 +408,7 @@ struct PolCheb {
 // residual): z.r32 -> rho, z.q32 -> gamma, beta = -gamma / (p.q)  (k_mfcg_dot).
 // Here b is r32.
 struct PolChebDot {
-    static constexpr int NIN = 1, NRED = 2;
+    static constexpr int NRED = 2;
     static constexpr bool HAS_K = true, HAS_M = true;
     const uint8_t *fixed;
     Weights<float> w;
@@ -419,11 +419,11 @@ struct PolChebDot {
     const float *q32;
     SolveScalars *S;
     Partials<2> part;
-    __device__ void load(long long n, float v[1][3]) const {
-        v[0][0] = x_in[3 * n];
-        v[0][1] = x_in[3 * n + 1];
-        v[0][2] = x_in[3 * n + 2];
-        mask3(fixed[n], v[0]);
+    __device__ void load(long long n, float v[3]) const {
+        v[0] = x_in[3 * n];
+        v[1] = x_in[3 * n + 1];
+        v[2] = x_in[3 * n + 2];
+        mask3(fixed[n], v);
     }
     __device__ void coef(long long e, float &ck, float &cm) const { w.get(e, ck, cm); }
     struct Pre {
@@ -471,18 +471,18 @@ struct PolChebDot {
 // residual only: r = b - (N A N + I - N) x   (before restriction)
 template <class T>
 struct PolResid {
-    static constexpr int NIN = 1, NRED = 0;
+    static constexpr int NRED = 0;
     static constexpr bool HAS_K = true, HAS_M = true;
     const uint8_t *fixed;
     Weights<T> w;
     const T *x, *b;
     T *r;
     Partials<1> part;
-    __device__ void load(long long n, T v[1][3]) const {
-        v[0][0] = x[3 * n];
-        v[0][1] = x[3 * n + 1];
-        v[0][2] = x[3 * n + 2];
-        mask3(fixed[n], v[0]);
+    __device__ void load(long long n, T v[3]) const {
+        v[0] = x[3 * n];
+        v[1] = x[3 * n + 1];
+        v[2] = x[3 * n + 2];
+        mask3(fixed[n], v);
     }
     // FP64 form (march.cuh)
     static constexpr int M_SRC = 1, M_IN = 1;
@@ -503,24 +503,24 @@ struct PolResid {
 // plain weighted product y = sum_e (ck KE + cm ME) x_e, no masking
 template <class T, bool HK, bool HM>
 struct PolProduct {
-    static constexpr int NIN = 1, NRED = 0;
+    static constexpr int NRED = 0;
     static constexpr bool HAS_K = HK, HAS_M = HM;
     Weights<T> w;
     const double *x;
     double *y;
     Partials<1> part;
-    __device__ void load(long long n, T v[1][3]) const {
-        v[0][0] = T(x[3 * n]);
-        v[0][1] = T(x[3 * n + 1]);
-        v[0][2] = T(x[3 * n + 2]);
+    __device__ void load(long long n, T v[3]) const {
+        v[0] = T(x[3 * n]);
+        v[1] = T(x[3 * n + 1]);
+        v[2] = T(x[3 * n + 2]);
     }
     // asynchronous staging (tile.cuh): x, no mask
     using Src = double;
     static constexpr int NSRC = 1;
     static constexpr bool MASK = false;
     __device__ const double *src(int) const { return x; }
-    __device__ void xform(const double raw[][3], uint8_t, T v[1][3]) const {
-        for (int c = 0; c < 3; c++) v[0][c] = T(raw[0][c]);
+    __device__ void xform(const double raw[][3], uint8_t, T v[3]) const {
+        for (int c = 0; c < 3; c++) v[c] = T(raw[0][c]);
     }
     // FP64 form (march.cuh)
     static constexpr int M_SRC = 1, M_IN = 1;
@@ -580,12 +580,11 @@ static __global__ void k_load_table(int Ts, double dt, int which, double scale, 
 // element pass gives K vK + M vM.  Also writes the initial guess x0 (the
 // Newmark predictor, see fwd_prep_args).
 // ---------------------------------------------------------------------------
-template <class T>
 struct PolRhsFwd {
     static constexpr int M_SRC = 3, M_IN = 2, NRED = 0;
     static constexpr bool HAS_K = true, HAS_M = true;
     const uint8_t *fixed;
-    Weights<T> w;
+    Weights<double> w;
     const double *cp;                   // checkpoints: block start state (j == 0)
     const double *Uh, *DUh, *DDUh;      // block history [tsc][ndof]
     long long ndof;
@@ -622,7 +621,7 @@ struct PolRhsFwd {
         v[1] = cM[0] * r[0] + cM[1] * r[1] + cM[2] * r[2];
     }
     __device__ const uint8_t *mmask() const { return fixed; }
-    __device__ void epilogue(long long n, int, int, int, const T y[3], double *) const {
+    __device__ void epilogue(long long n, int, int, int, const double y[3], double *) const {
         const double *u, *du, *ddu;
         prev(u, du, ddu);
         // acceleration one step further back: history slot j-2, or the block
@@ -638,7 +637,7 @@ struct PolRhsFwd {
         for (int c = 0; c < 3; c++) {
             bool fx = (f >> c) & 1;
             const double f2 = (3 * n + c == load2_dof) ? sig2[t] : 0.0;
-            b[3 * n + c] = fx ? 0.0 : (rhs0[3 * n + c] * s + f2 + todbl(y[c]));
+            b[3 * n + c] = fx ? 0.0 : (rhs0[3 * n + c] * s + f2 + y[c]);
             double xv = pred[0] * u[3 * n + c] + pred[1] * du[3 * n + c];
             if (ddu2)
                 xv += pred2[0] * ddu[3 * n + c] + pred2[1] * ddu2[3 * n + c];

@@ -36,10 +36,9 @@ struct TileGeom {
     static_assert(E == 1 << LOG && STAGED <= 2 * THREADS, "staging in two passes");
 };
 
-template <class T, class Pol, int TL = TILE, int TZ = TILE>
+template <class T, int TL = TILE, int TZ = TILE>
 constexpr size_t tile_smem_bytes() {
-    return sizeof(T) *
-           ((size_t)Pol::NIN * TileGeom<TL, TZ>::STAGED * 3 + (size_t)TileGeom<TL, TZ>::THREADS * EL_STRIDE);
+    return sizeof(T) * ((size_t)TileGeom<TL, TZ>::STAGED * 3 + (size_t)TileGeom<TL, TZ>::THREADS * EL_STRIDE);
 }
 
 __host__ __device__ inline int tile_count(const GridDesc &g, int &ntx, int &nty, int tl = TILE, int tz = TILE) {
@@ -49,11 +48,9 @@ __host__ __device__ inline int tile_count(const GridDesc &g, int &ntx, int &nty,
 }
 
 // Policy interface:
-//   static constexpr int NIN;      staged 3-vectors per node (1: K and M act on
-//                                  input 0; 2: K on input 0, M on input 1)
 //   static constexpr bool HAS_K, HAS_M;
 //   static constexpr int NRED;     grid-reduced doubles (0..4)
-//   __device__ void load(long long n, T v[NIN][3]) const;
+//   __device__ void load(long long n, T v[3]) const;
 //   __device__ void coef(long long e, T &ck, T &cm) const;
 //   __device__ void epilogue(long long n, int i, int j, int k, const T y[3], double red[]) const;
 //   __device__ void finish(const double tot[]) const;   (thread 0 of last CTA)
@@ -145,7 +142,7 @@ __device__ __forceinline__ long long tile_index(int i, int j, int k, int nx, int
 
 // staged input nodes of a brick held by this thread (at most two)
 template <class T, int TL = TILE, int TZ = TILE, class Pol>
-__device__ __forceinline__ void tile_fetch(const Pol &pol, const GridDesc &g, TilePos at, T v[2][Pol::NIN][3]) {
+__device__ __forceinline__ void tile_fetch(const Pol &pol, const GridDesc &g, TilePos at, T v[2][3]) {
     using G = TileGeom<TL, TZ>;
     const int i0 = at.i * TL, j0 = at.j * TL, k0 = at.k * TZ;
 #pragma unroll
@@ -157,8 +154,7 @@ __device__ __forceinline__ void tile_fetch(const Pol &pol, const GridDesc &g, Ti
             const long long n = tile_index(gi, gj, gk, g.nx, g.ny);
             pol.load(n, v[it]);
         } else {
-#pragma unroll
-            for (int f = 0; f < Pol::NIN; f++) v[it][f][0] = v[it][f][1] = v[it][f][2] = T(0);
+            v[it][0] = v[it][1] = v[it][2] = T(0);
         }
     }
 }
@@ -190,42 +186,13 @@ __device__ __forceinline__ void tile_elements(const GridDesc &g, const ElemConst
 #pragma unroll
         for (int c = 0; c < 3; c++) mode_fwd(U[c]);
         T Y[3][8];
-        if (Pol::HAS_K && Pol::HAS_M && Pol::NIN == 1) {
-            mode_khat_mass(C, ck, cm, U, Y);
-        } else if (Pol::HAS_K && !Pol::HAS_M) {
-            mode_khat_mass<false>(C, ck, cm, U, Y);
+        if (Pol::HAS_K) {
+            mode_khat_mass<Pol::HAS_M>(C, ck, cm, U, Y);
         } else {
-            if (Pol::HAS_K) {
-                mode_khat(C, U, Y);
 #pragma unroll
-                for (int c = 0; c < 3; c++)
+            for (int b = 0; b < 3; b++)
 #pragma unroll
-                    for (int m = 0; m < 8; m++) Y[c][m] *= ck;
-            } else {
-#pragma unroll
-                for (int c = 0; c < 3; c++)
-#pragma unroll
-                    for (int m = 0; m < 8; m++) Y[c][m] = T(0);
-            }
-            if (Pol::HAS_M) {
-#pragma unroll
-                for (int b = 0; b < 3; b++) {
-                    T V[8];
-                    if (Pol::NIN == 2) {
-#pragma unroll
-                        for (int L = 0; L < 8; L++) {
-                            int s = (lx + (L & 1)) + G::N * ((ly + ((L >> 1) & 1)) + G::N * (lz + (L >> 2)));
-                            V[L] = sIn[((Pol::NIN - 1) * G::STAGED + s) * 3 + b];
-                        }
-                        mode_fwd(V);
-                    } else {
-#pragma unroll
-                        for (int m = 0; m < 8; m++) V[m] = U[b][m];
-                    }
-#pragma unroll
-                    for (int m = 0; m < 8; m++) Y[b][m] = tadd(Y[b][m], tmul(tmul(cm, C.W[m]), V[m]));
-                }
-            }
+                for (int m = 0; m < 8; m++) Y[b][m] = tadd(T(0), tmul(tmul(cm, C.W[m]), U[b][m]));
         }
 #pragma unroll
         for (int b = 0; b < 3; b++) {
@@ -280,7 +247,7 @@ constexpr bool tile_persistent() {
 // this brick is computed
 template <class T, int TL = TILE, int TZ = TILE, class Pol>
 __device__ __forceinline__ void tile_brick(const GridDesc &g, const ElemConst<T> &C, const Pol &pol, T *sIn, T *sEl,
-                                           TilePos at, TilePos next, bool more, T v[2][Pol::NIN][3],
+                                           TilePos at, TilePos next, bool more, T v[2][3],
                                            pol_red_t<Pol> *red) {
     using G = TileGeom<TL, TZ>;
     const int tid = threadIdx.x;
@@ -290,9 +257,7 @@ __device__ __forceinline__ void tile_brick(const GridDesc &g, const ElemConst<T>
         const int s = tid + it * G::THREADS;
         if (s < G::STAGED) {
 #pragma unroll
-            for (int f = 0; f < Pol::NIN; f++)
-#pragma unroll
-                for (int c = 0; c < 3; c++) sIn[(f * G::STAGED + s) * 3 + c] = v[it][f][c];
+            for (int c = 0; c < 3; c++) sIn[s * 3 + c] = v[it][c];
         }
     }
     // output node of this thread and its prefetched epilogue operands
@@ -318,7 +283,7 @@ __device__ __forceinline__ void tile_brick(const GridDesc &g, const ElemConst<T>
 //   static constexpr int NSRC;           raw arrays staged per node (1 or 2)
 //   static constexpr bool MASK;          read the clamp bitmask `fixed` too
 //   const Src *src(int k) const;         raw array k, 3 values per node
-//   void xform(const Src raw[NSRC][3], uint8_t f, T v[1][3]) const;
+//   void xform(const Src raw[NSRC][3], uint8_t f, T v[3]) const;
 //                                        staged value from the raw values
 // The kernel is then persistent: every thread issues `cp.async` copies of the
 // raw values of its own staged nodes of the next brick into its own slots of a
@@ -348,7 +313,7 @@ constexpr bool tile_async() {
 
 template <class T, class Pol, bool ASYNC = tile_async<T, Pol>()>
 struct TileSmem {
-    static constexpr size_t bytes = tile_smem_bytes<T, Pol>();
+    static constexpr size_t bytes = tile_smem_bytes<T>();
 };
 template <class T, class Pol>
 struct TileSmem<T, Pol, true> {
@@ -398,7 +363,6 @@ __device__ __forceinline__ void tile_run_async(const GridDesc &g, const ElemCons
                                                unsigned char *sm, int ntiles, int ntx, int nty, pol_red_t<Pol> *red) {
     using L = TileSmem<T, Pol>;
     using Src = typename Pol::Src;
-    static_assert(Pol::NIN == 1, "async staging stages one 3-vector per node");
     const int tid = threadIdx.x;
     Src *raw = reinterpret_cast<Src *>(sm + L::raw);
     T *sIn = reinterpret_cast<T *>(sm + L::in);
@@ -419,7 +383,7 @@ __device__ __forceinline__ void tile_run_async(const GridDesc &g, const ElemCons
             if (s < TILE_STAGED) {
                 const int lx = s % TILE_N, ly = (s / TILE_N) % TILE_N, lz = s / (TILE_N * TILE_N);
                 const int gi = i0 - 1 + lx, gj = j0 - 1 + ly, gk = k0 - 1 + lz;
-                T v[1][3] = {{T(0), T(0), T(0)}};
+                T v[3] = {T(0), T(0), T(0)};
                 if (tile_in(gi, gj, gk, g.nx, g.ny, g.nz)) {
                     Src rv[Pol::NSRC][3];
 #pragma unroll
@@ -429,7 +393,7 @@ __device__ __forceinline__ void tile_run_async(const GridDesc &g, const ElemCons
                     pol.xform(rv, f[it], v);
                 }
 #pragma unroll
-                for (int c = 0; c < 3; c++) sIn[s * 3 + c] = v[0][c];
+                for (int c = 0; c < 3; c++) sIn[s * 3 + c] = v[c];
             }
         }
         const int tx = tid % TILE, ty = (tid / TILE) % TILE, tz = tid / (TILE * TILE);
@@ -461,8 +425,8 @@ __global__ void __launch_bounds__(TileGeom<TL, TZ>::THREADS, sizeof(T) == 4 ? 2 
         tile_run_async<T>(g, C, pol, smem_raw, ntiles, ntx, nty, red);
     } else {
         T *sIn = reinterpret_cast<T *>(smem_raw);
-        T *sEl = sIn + Pol::NIN * TileGeom<TL, TZ>::STAGED * 3;
-        T v[2][Pol::NIN][3];
+        T *sEl = sIn + TileGeom<TL, TZ>::STAGED * 3;
+        T v[2][3];
         TilePos at = tile_pos(blockIdx.x, ntx, nty);
         if constexpr (tile_persistent<T>()) {
             const TilePos step = tile_pos(gridDim.x, ntx, nty);

@@ -31,7 +31,6 @@ struct VTail {
     int nu, n;  // smoothing steps, coarse DOFs
 };
 struct VTElem {  // weights of the thread's element, loaded once
-    static constexpr int NIN = 1;
     static constexpr bool HAS_K = true, HAS_M = true;
     float k, m;
     __device__ void coef(long long, float &ck, float &cm) const {
