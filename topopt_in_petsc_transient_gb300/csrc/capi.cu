@@ -345,14 +345,10 @@ void topo_box_element_matrices(double hx, double hy, double hz, double nu, doubl
 }
 
 // ---------------------------------------------------------------------------
-int topo_pdefilt_create(topo_pdefilt **out, int nx, int ny, int nz, double hx, double hy, double hz, double rmin,
-                        double rtol, int maxit) {
-    if (!out) return TOPO_ERR_ARG;
-    *out = nullptr;
-    int rc = device_ok();
-    if (rc) return rc;
+static int pdefilt_try(topo_pdefilt **out, int nx, int ny, int nz, double hx, double hy, double hz, double rmin,
+                       double rtol, int maxit, int nrhs) {
     TopoPDEFilt *impl = nullptr;
-    rc = pdefilt_create(&impl, nx, ny, nz, hx, hy, hz, rmin, rtol, maxit);
+    int rc = pdefilt_create(&impl, nx, ny, nz, hx, hy, hz, rmin, rtol, maxit, nrhs);
     if (rc) return rc;
     topo_pdefilt *h = new topo_pdefilt();
     h->impl = impl;
@@ -370,6 +366,20 @@ int topo_pdefilt_create(topo_pdefilt **out, int nx, int ny, int nz, double hx, d
     }
     *out = h;
     return TOPO_OK;
+}
+
+int topo_pdefilt_create(topo_pdefilt **out, int nx, int ny, int nz, double hx, double hy, double hz, double rmin,
+                        double rtol, int maxit) {
+    if (!out) return TOPO_ERR_ARG;
+    *out = nullptr;
+    int rc = device_ok();
+    if (rc) return rc;
+    // fields are solved in pairs where the memory is there for it, else one by one
+    for (int nrhs = FILT_RHS; nrhs >= 1; nrhs--) {
+        rc = pdefilt_try(out, nx, ny, nz, hx, hy, hz, rmin, rtol, maxit, nrhs);
+        if (rc != TOPO_ERR_OOM) break;
+    }
+    return rc;
 }
 
 void topo_pdefilt_destroy(topo_pdefilt *f) {

@@ -31,7 +31,6 @@ namespace topo {
         }                                                                    \
     } while (0)
 
-constexpr int FILT_RHS = 2;        // right-hand sides solved at once
 constexpr int FT_N = 256;          // threads: node columns of a CTA, tx x ty of them
 constexpr int FT_PLANE = 2 * FT_N;  // most values of a staged plane: the columns and one node around
 constexpr int FT_RING = 4;          // planes whose raw values are in flight or in use
@@ -503,8 +502,7 @@ static __global__ void k_filt_out(const FiltArgs A, int r, const double *u) { fi
 
 struct TopoPDEFilt {
     GridDesc g;
-    double rtol;
-    int maxit;
+    int nrhs;        // right-hand sides that the workspace is for
     FiltArgs args;   // operator, buffers and layout of the launches
     unsigned grid;   // CTAs of k_filt_solve: as many as are resident at once, at most one per run
     double *mnd;
@@ -535,7 +533,7 @@ __global__ void k_mnd(long long n, const double *__restrict__ x, Partials<1> par
 
 // ---------------------------------------------------------------------------
 int pdefilt_create(TopoPDEFilt **out, int nx, int ny, int nz, double hx, double hy, double hz, double rmin, double rtol,
-                   int maxit) {
+                   int maxit, int nrhs) {
     *out = nullptr;
     if (nx < 2 || ny < 2 || nz < 2 || hx <= 0 || hy <= 0 || hz <= 0 || rmin <= 0) {
         set_error("invalid PDE filter parameters");
@@ -544,8 +542,7 @@ int pdefilt_create(TopoPDEFilt **out, int nx, int ny, int nz, double hx, double 
     TopoPDEFilt *f = new TopoPDEFilt();
     f->g = GridDesc{nx, ny, nz, nx - 1, ny - 1, nz - 1};
     const double R = rmin / 2.0 / sqrt(3.0);  // PDEFilter.cc:32
-    f->rtol = rtol;
-    f->maxit = maxit;
+    f->nrhs = nrhs;
     const double hh[3] = {hx, hy, hz};
     filt_stencil(hh, R, f->args.Kd.c);
     for (int S = 0; S < 8; S++) f->args.Kf.c[S] = (float)f->args.Kd.c[S];
@@ -562,7 +559,7 @@ int pdefilt_create(TopoPDEFilt **out, int nx, int ny, int nz, double hx, double 
     A.g = f->g;
     std::vector<std::pair<void **, size_t>> want;
     auto get = [&](auto **p, size_t n) { want.emplace_back((void **)p, sizeof(**p) * n); };
-    for (int r = 0; r < FILT_RHS; r++) {
+    for (int r = 0; r < nrhs; r++) {
         for (int k = 0; k < 2; k++) {
             get(&A.u[r][k], nn);
             for (float **q : {&A.s32[r][k], &A.w32[r][k]}) get(q, nn);
@@ -587,7 +584,7 @@ int pdefilt_create(TopoPDEFilt **out, int nx, int ny, int nz, double hx, double 
             *w.first = mem;
             mem += (w.second + 255) / 256 * 256;
         }
-        for (int r = 0; r < FILT_RHS; r++) {
+        for (int r = 0; r < nrhs; r++) {
             A.r32[r][0] = (float *)A.q[r];
             A.r32[r][1] = A.r32[r][0] + nn;
         }
@@ -707,10 +704,10 @@ int filter_gradients_dev(TopoPDEFilt *f, const double *xTilde_dev, double *dfdx_
                                                          make_projection(1, beta, eta));
     }
     // PDEFilt::Gradients == FilterProject (PDEFilter.cc:224), dfdx and the m columns of dgdx
-    for (int j = 0; j <= m; j += FILT_RHS) {
+    for (int j = 0; j <= m; j += f->nrhs) {
         double *v[FILT_RHS];
         int nr = 0;
-        for (; nr < FILT_RHS && j + nr <= m; nr++) v[nr] = j + nr == 0 ? dfdx_dev : dgdx_dev + (size_t)(j + nr - 1) * nel;
+        for (; nr < f->nrhs && j + nr <= m; nr++) v[nr] = j + nr == 0 ? dfdx_dev : dgdx_dev + (size_t)(j + nr - 1) * nel;
         const int rc = filt_solve(f, nr, v, v, nullptr, 0, 0, 0.0, 0.0);
         if (rc) return rc;
     }

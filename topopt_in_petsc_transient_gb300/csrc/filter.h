@@ -4,8 +4,10 @@
 
 namespace topo {
 struct TopoPDEFilt;
+constexpr int FILT_RHS = 2;  // right-hand sides solved at once, at most
+// nrhs: those that the workspace is for (64 bytes a node each)
 int pdefilt_create(TopoPDEFilt **out, int nx, int ny, int nz, double hx, double hy, double hz, double rmin, double rtol,
-                   int maxit);
+                   int maxit, int nrhs);
 void pdefilt_destroy(TopoPDEFilt *f);
 long long pdefilt_nel(const TopoPDEFilt *f);
 int pdefilt_apply_dev(TopoPDEFilt *f, const double *x_dev, double *xout_dev);
