@@ -919,9 +919,11 @@ static int setup_operator(TopoLE *le, int o) {
                                       std::max(kron_yz_smem(l0.g, 2, 8), kron_yz_smem(l0.g, 2, 4, true)));
         op.kron = stage <= KRON_SMEM_MAX && op.sM > 0.0 && op.sK >= 0.0 &&
                   (le->p.mass_precond == 1 || (le->p.mass_precond == 2 && op.share <= le->p.mass_precond_share));
-        if (op.kron) {  // its node scaling, in the precision of the solves
+        // its node scaling, in the precision of the solves: FP32 on the mixed path but for
+        // operator 2, the basis solves' (sommg_basis), whose sM < 0 rules it out anyway
+        if (op.kron) {
             count_launch();
-            if (le->p.mixed)
+            if (le->p.mixed && o != 2)
                 k_kron_scale<float><<<ew_blocks(l0.g.nn()), EW, 0, s>>>(l0.g, l0.fixed, l0.mfd, op.sM, op.kscale_f);
             else
                 k_kron_scale<double><<<ew_blocks(l0.g.nn()), EW, 0, s>>>(l0.g, l0.fixed, l0.mfd, op.sM, op.kscale_d);
