@@ -43,9 +43,12 @@ inline void count_launch(long long n = 1) { launch_counter() += n; }
 // Letting the next kernel in from this one's start was slower (FP64 solves of
 // 48x24x24 123 instead of 101 ms, 104 without): its CTAs fill the SMs in the order
 // in which these become free, and the load is uneven.
-// Up to this many nodes of a grid: 96x48x48 (233 thousand) takes 190.9 instead of
-// 193.6 ms, 192x96x96 (1.8 million) 215 instead of 211: the launch is short beside
-// kernels of 100 us, and early CTAs disturb the persistent ones.
+// Up to this many nodes of a grid, past which the gain falls under 1% and then turns:
+// an evaluation with the Kronecker preconditioner takes 0.975 of the time of plain
+// launches at 233 thousand nodes, 0.978 at 367, 0.992 at 450, 0.995 at 545, 1.004 at
+// 773, 0.995 at 1056 and 1.019 at 1816 (with multigrid 0.990, 0.993 at 367, 0.991 at
+// 545, 0.997 at 1056): the launch is short beside kernels of 100 us, and early CTAs
+// disturb the persistent ones.
 constexpr long long DEP_NODES = 400000;
 __device__ __forceinline__ void grid_dep_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
