@@ -391,7 +391,7 @@ struct OpLevel {
     double *dinvd = nullptr;
     float *dinvf = nullptr;
     double *lohi = nullptr;  // device [5]: smoothing interval, full-spectrum interval, raw lower bound
-    double *cheb = nullptr;   // device [kmax][2] Chebyshev step coefficients (smoothing)
+    double *cheb = nullptr;   // device [CHEB_MAX][2] Chebyshev step coefficients (smoothing), then the same in FP32 (cheb_tab)
     double *chebf = nullptr;  // same over the full spectrum (smoother-as-solver level)
     double hlohi[5] = {0, 0, 0, 0, 0};
 };
@@ -891,8 +891,11 @@ void le_destroy(TopoLE *le) {
 // ---------------------------------------------------------------------------
 static int cheb_kmax(const TopoLE *le) {
     int k = le->p.smooth > le->p.coarse_smooth ? le->p.smooth : le->p.coarse_smooth;
-    return k < 1 ? 1 : (k > 64 ? 64 : k);
+    return k < 1 ? 1 : (k > CHEB_MAX ? CHEB_MAX : k);
 }
+
+// table row of step k: later steps than it has rows go on with the last
+static int cheb_row(int k) { return std::min(k, CHEB_MAX - 1); }
 
 static int setup_operator(TopoLE *le, int o) {
     Operator &op = le->ops[o];
@@ -1120,14 +1123,14 @@ static T *vcycle(TopoLE *le, int o, int l, const T *b, VFuse *fz = nullptr) {
         bool done = false;
         if constexpr (std::is_same<T, float>::value) {
             if (fuse && last) {
-                PolChebDot pc{lv.fixed, wt, x, b, w.dinv, xo, w.d, tab, k, fz->q32, fz->S, fz->part};
+                PolChebDot pc{lv.fixed, wt, x, b, w.dinv, xo, w.d, tab, cheb_row(k), fz->q32, fz->S, fz->part};
                 launch_tile<float>(lv.g, *w.C, pc, s);
                 fz->dotted = true;
                 done = true;
             }
         }
         if (!done) {
-            PolCheb<T> pc{lv.fixed, wt, x, b, w.dinv, xo, w.d, tab, k, {}};
+            PolCheb<T> pc{lv.fixed, wt, x, b, w.dinv, xo, w.d, tab, cheb_row(k), {}};
             launch_solve_tile<T>(brick_order(le), lv.g, *w.C, pc, s);
         }
         T *t = x;
@@ -1248,14 +1251,14 @@ static T *kron_smooth(TopoLE *le, int o, const T *r, T *z0, VFuse *fz) {
         bool done = false;
         if constexpr (std::is_same<T, float>::value) {
             if (fz && k == ns - 1) {
-                PolChebDot pc{l0.fixed, wt, x, r, w.dinv, xo, w.d, tab, k, fz->q32, fz->S, fz->part};
+                PolChebDot pc{l0.fixed, wt, x, r, w.dinv, xo, w.d, tab, cheb_row(k), fz->q32, fz->S, fz->part};
                 launch_tile<float>(l0.g, *w.C, pc, s);
                 fz->dotted = true;
                 done = true;
             }
         }
         if (!done) {
-            PolCheb<T> pc{l0.fixed, wt, x, r, w.dinv, xo, w.d, tab, k, {}};
+            PolCheb<T> pc{l0.fixed, wt, x, r, w.dinv, xo, w.d, tab, cheb_row(k), {}};
             launch_solve_tile<T>(brick_order(le), l0.g, *w.C, pc, s);
         }
         T *t = x;
