@@ -385,7 +385,8 @@ static __global__ void k_coarse_assemble(GridDesc g, const uint8_t *__restrict__
 // product.  In panels of CH columns: every entry takes the same operations in
 // the same order as column by column (a -= (c_i / c_k) c_j for k ascending, c
 // the updated, unscaled column k), with two launches a panel where a column
-// took two: 8 ms of launches for n = 675 become 0.6.
+// took two: the set-up of a design at 64x32x32 (n = 675, two operators) takes 6.0
+// instead of 17.7 ms, 0.7 of them without the coarse inverse.
 constexpr int CH = 32;
 // panel k0: rows k0 + 32 b .. of block b, one row a lane, the diagonal block
 // factored by every CTA for itself.  Uc, Qc [n][CH]: unscaled columns and c_i / c_k

@@ -172,8 +172,8 @@ __device__ double mma_residual(const MMADual<M> &D, const MMAScalars *S) {
 // one at a bound adds ga or gb to the gradient.  About 40 FP64 instructions an
 // element against about 200 with a quotient for every term in two passes a
 // step, at GB300's 2 lanes a clock and SM the whole time of a pass: an update
-// of 1,769,472 elements takes 1.8 ms instead of 6.2, one of 27,648 (launches and
-// host polls before) 0.15 instead of 0.53.
+// of 1,769,472 elements takes 1.85 ms instead of 6.3, one of 27,648 (launches and
+// host polls before) 0.21 instead of 0.59.
 template <int M>
 __device__ __forceinline__ void mma_sums(const MMAArgs &A, const double *lam, double *acc) {
     const long long n = A.n;
