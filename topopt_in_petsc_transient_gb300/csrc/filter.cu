@@ -6,7 +6,8 @@
 // PDEFilter.cc:485-578); T (0.125 per element node, :580-588) and T^t are
 // gathers.  The assembled operator is a sum of tensor products of the 1-D
 // stiffness and mass, applied without the matrix; the solve is one cooperative
-// kernel (k_filt_solve).
+// kernel (k_filt_solve), with a second one for what FP32 corrections cannot solve
+// (k_filt_cg).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -653,20 +654,22 @@ static int filt_solve(TopoPDEFilt *f, int nr, const double *const *xin, double *
     A.xphys = xphys;
     A.clamp = clamp;
     A.proj = make_projection(projection, beta, eta);
-    auto launch = [&](const void *kernel, void **args) -> int {
+    auto launch = [&](const void *kernel, void **args) {
         f->status->status = TOPO_ERR_CUDA;
         count_launch();
-        FCK(cudaLaunchCooperativeKernel(kernel, dim3(f->grid), dim3(FT_N), args, 0, s));
-        FCK(cudaStreamSynchronize(s));
-        return *(volatile int *)&f->status->status;
+        const cudaError_t e = cudaLaunchCooperativeKernel(kernel, dim3(f->grid), dim3(FT_N), args, 0, s);
+        return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
     };
     void *args[] = {&A};
-    int st = launch((const void *)k_filt_solve, args);
+    FCK(launch((const void *)k_filt_solve, args));
+    int st = *(volatile int *)&f->status->status;
     const int hard = f->status->hard, cur = f->status->cur;
     if (st == TOPO_OK && hard) {
         for (int r = 0; r < nr && st == TOPO_OK; r++) {
+            if (!((hard >> r) & 1)) continue;
             void *cargs[] = {&A, &r};
-            if ((hard >> r) & 1) st = launch((const void *)k_filt_cg, cargs);
+            FCK(launch((const void *)k_filt_cg, cargs));
+            st = *(volatile int *)&f->status->status;
         }
         for (int r = 0; r < nr && st == TOPO_OK; r++) {  // no result before all are solved
             count_launch();
